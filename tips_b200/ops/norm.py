@@ -63,9 +63,7 @@ class _BatchNormFn(torch.autograd.Function):
                 xc.data_ptr(), base.ptr(res), y.data_ptr(), weight.data_ptr(), bias.data_ptr(),
                 running_mean.data_ptr(), running_var.data_ptr(), m, c, eps, int(relu), base.code(xc), base.stream()),
                 "bn_fwd_eval")
-            ctx.mask_mode = "y" if relu else "none"
-            ctx.save_for_backward(xc, y if relu else None, weight,
-                                  running_mean.clone(), torch.rsqrt(running_var + eps), None, None)
+            # nothing is saved: the backward pass is refused in eval mode
         ctx.relu = bool(relu)
         ctx.has_res = residual is not None
         ctx.training_mode = bool(training)
@@ -73,9 +71,9 @@ class _BatchNormFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, y, weight, save_mean, save_invstd, bias, bits = ctx.saved_tensors
         if not ctx.training_mode:
             raise RuntimeError("backward through batch norm in eval mode is not supported by the fused kernel")
+        x, y, weight, save_mean, save_invstd, bias, bits = ctx.saved_tensors
         c = x.shape[1]
         m = x.numel() // c
         dyc = dy.contiguous(memory_format=torch.channels_last) if dy.dim() == 4 else dy.contiguous()
