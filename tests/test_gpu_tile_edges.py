@@ -1,0 +1,50 @@
+"""Kernels at the edges of their tiles and of the rules that choose them, against plain PyTorch in fp32 or fp64.
+
+Tolerances: a bf16 result of an fp32 accumulation is off by at most half a unit in the last place, 2^-8 of its value, plus
+the accumulation's own error; `_close` allows 2^-12 of the largest value for the latter."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+BF16 = torch.bfloat16
+
+
+def _close(got, ref, slack=2.0 ** -12, rel=2.0 ** -8):
+    got, ref = got.double(), ref.double()
+    assert got.shape == ref.shape
+    bad = (got - ref).abs() > ref.abs() * rel + float(ref.abs().max()) * slack
+    assert not bool(bad.any()), float((got - ref).abs().max())
+
+
+def _rand(*shape, scale=0.5, dtype=BF16, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed + sum(shape))
+    return (torch.randn(*shape, generator=g, device=DEV) * scale).to(dtype)
+
+
+@pytest.mark.parametrize("src,flat", [(BF16, BF16), (torch.float32, BF16), (torch.float16, torch.float32)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_pack_many_tensors(src, flat, accumulate):
+    from tips_b200.ops import base
+    numels = [1, 3, 8191, 8192, 8193, 0, 40001] + [5 + i for i in range(120)]  # more than one launch takes
+    offs, at = [], 0
+    for i, n in enumerate(numels):
+        offs.append(at)
+        at += n + i % 3  # some of them not aligned to a vector
+    tensors = [_rand(n, dtype=src, seed=i) for i, n in enumerate(numels)]
+    buf = _rand(at, dtype=flat, seed=7)
+    want = buf.float().clone()
+    for t, o in zip(tensors, offs):
+        v = t.float() * 0.5
+        want[o:o + t.numel()] = want[o:o + t.numel()] + v if accumulate else v
+    base.check(base.K().tipsk_pack(base.ptr_array(tensors), base.i64_array(offs), base.i64_array(numels), len(tensors),
+                                   base.code(src), buf.data_ptr(), base.code(flat), 0.5, int(accumulate), base.stream()),
+               "pack")
+    assert torch.equal(buf, want.to(flat))
+    back = [torch.empty_like(t) for t in tensors]
+    base.check(base.K().tipsk_unpack(buf.data_ptr(), base.code(flat), base.ptr_array(back), base.i64_array(offs),
+                                     base.i64_array(numels), len(back), base.code(src), 2.0, base.stream()), "unpack")
+    for t, o in zip(back, offs):
+        assert torch.equal(t, (buf[o:o + t.numel()].float() * 2.0).to(src))
