@@ -24,6 +24,20 @@ def _rand(*shape, scale=0.5, dtype=BF16, seed=0):
     return (torch.randn(*shape, generator=g, device=DEV) * scale).to(dtype)
 
 
+@pytest.mark.parametrize("n,c,h,w", [(1, 8, 1, 1), (2, 8, 2, 3), (3, 72, 5, 8), (2, 64, 31, 33), (1, 2056, 4, 4)])
+def test_maxpool_edges(n, c, h, w):
+    from tips_b200.ops.pool import max_pool_3x3_s2
+    x = _rand(n, c, h, w).contiguous(memory_format=torch.channels_last).requires_grad_()
+    y = max_pool_3x3_s2(x)
+    xr = x.detach().float().requires_grad_()
+    yr = F.max_pool2d(xr, 3, stride=2, padding=1)
+    assert torch.equal(y.float(), yr)
+    dy = _rand(*y.shape, seed=1).contiguous(memory_format=torch.channels_last)
+    y.backward(dy)
+    yr.backward(dy.float())
+    _close(x.grad, xr.grad)
+
+
 @pytest.mark.parametrize("src,flat", [(BF16, BF16), (torch.float32, BF16), (torch.float16, torch.float32)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_pack_many_tensors(src, flat, accumulate):

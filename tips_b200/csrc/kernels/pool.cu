@@ -2,8 +2,8 @@
 //
 // Forward: one thread per (output pixel, 8 channels): nine 16-byte loads, a running maximum that keeps the
 // FIRST maximum in scan order (rows, then columns), one 16-byte store of the result and 8 bytes of argmax
-// codes (0..8).  Backward: one thread per (input pixel, 8 channels) gathers from the at most four windows
-// that contain the pixel the gradients whose argmax code points at it: no atomics, deterministic, and the
+// codes (0..8).  Backward: one thread per (2 x 2 input pixels, 8 channels) gathers from the at most four windows
+// that contain them the gradients whose argmax code points at each: no atomics, deterministic, and the
 // input activation is not read again.
 //
 // The reference has no pooling (model math is TensorFlow's); this serves the ResNet-50 benchmark model.
@@ -15,100 +15,132 @@
 namespace tipsk {
 namespace {
 
+// Two 16-bit floats in a register: minus infinity twice, and a mask of the halves in which a > b (NaN: not greater).
 template <typename T>
-__global__ void __launch_bounds__(256)
-MaxPoolFwdKernel(const T* __restrict__ x, T* __restrict__ y, uint8_t* __restrict__ idx, int n, int h, int w, int c,
+__device__ __forceinline__ uint32_t NegInf2();
+template <>
+__device__ __forceinline__ uint32_t NegInf2<__nv_bfloat16>() { return 0xff80ff80u; }
+template <>
+__device__ __forceinline__ uint32_t NegInf2<__half>() { return 0xfc00fc00u; }
+template <typename T>
+__device__ __forceinline__ uint32_t Greater2(uint32_t a, uint32_t b);
+template <>
+__device__ __forceinline__ uint32_t Greater2<__nv_bfloat16>(uint32_t a, uint32_t b) {
+  return __hgt2_mask(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+}
+template <>
+__device__ __forceinline__ uint32_t Greater2<__half>(uint32_t a, uint32_t b) {
+  return __hgt2_mask(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
+}
+
+// Both directions are bound by HBM.  A block works on one row (of outputs, or of 2 x 2 input quads), so a thread needs a
+// single 32-bit division to find its pixel, and all its loads are issued before the first comparison.
+template <typename T>
+__global__ void __launch_bounds__(256, 4)
+MaxPoolFwdKernel(const T* __restrict__ x, T* __restrict__ y, uint8_t* __restrict__ idx, int64_t rows, int h, int w, int c,
                  int ho, int wo) {
   constexpr int V = 8;
   const int cv = c / V;
-  const int64_t total = static_cast<int64_t>(n) * ho * wo * cv;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int cg = static_cast<int>(i % cv);
-    int64_t pix  = i / cv;
-    const int ow = static_cast<int>(pix % wo); pix /= wo;
-    const int oh = static_cast<int>(pix % ho);
-    const int in = static_cast<int>(pix / ho);
-    float best[V];
-    uint8_t arg[V];
-#pragma unroll
-    for (int j = 0; j < V; ++j) { best[j] = -INFINITY; arg[j] = 0; }
+  const int i  = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= wo * cv) return;
+  const int ow = i / cv, cg = i - ow * cv;
+  for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {  // row = image * ho + oh
+    const int64_t in = row / ho;
+    const int oh     = static_cast<int>(row - in * ho);
+    const T* base    = x + in * h * w * c + cg * V;
+    Vec16<T> v[9];
+    bool have[9];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       const int ih = oh * 2 - 1 + r;
-      if (ih < 0 || ih >= h) continue;
 #pragma unroll
       for (int s = 0; s < 3; ++s) {
         const int iw = ow * 2 - 1 + s;
-        if (iw < 0 || iw >= w) continue;
-        const Vec16<T> v = LoadVec(x + ((static_cast<int64_t>(in) * h + ih) * w + iw) * c + cg * V);
-#pragma unroll
-        for (int j = 0; j < V; ++j) {
-          const float f = ToFloat(v.v[j]);
-          if (f > best[j]) { best[j] = f; arg[j] = static_cast<uint8_t>(r * 3 + s); }
-        }
+        have[r * 3 + s] = ih >= 0 && ih < h && iw >= 0 && iw < w;
+        if (have[r * 3 + s]) v[r * 3 + s] = LoadVec(base + (static_cast<int64_t>(ih) * w + iw) * c);
       }
     }
-    Vec16<T> o;
+    // two channels per register: the comparison yields a mask that selects value and position of both
+    uint32_t best[4], arg[4];
 #pragma unroll
-    for (int j = 0; j < V; ++j) o.v[j] = FromFloat<T>(best[j]);
-    const int64_t opix = (static_cast<int64_t>(in) * ho + oh) * wo + ow;
-    StoreVec(y + opix * c + cg * V, o);
-    uint2 packed;
-    packed.x = arg[0] | (arg[1] << 8) | (arg[2] << 16) | (arg[3] << 24);
-    packed.y = arg[4] | (arg[5] << 8) | (arg[6] << 16) | (arg[7] << 24);
-    *reinterpret_cast<uint2*>(idx + opix * c + cg * V) = packed;
+    for (int i = 0; i < 4; ++i) { best[i] = NegInf2<T>(); arg[i] = 0; }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      if (!have[k]) continue;
+      const uint32_t* q = reinterpret_cast<const uint32_t*>(&v[k]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t gt = Greater2<T>(q[i], best[i]);
+        best[i] = (q[i] & gt) | (best[i] & ~gt);
+        arg[i]  = (k * 0x10001u & gt) | (arg[i] & ~gt);
+      }
+    }
+    const int64_t at = (row * wo + ow) * c + cg * V;
+    *reinterpret_cast<uint4*>(y + at) = make_uint4(best[0], best[1], best[2], best[3]);
+    // bytes 0 and 2 of each: the positions of eight channels
+    *reinterpret_cast<uint2*>(idx + at) = make_uint2(__byte_perm(arg[0], arg[1], 0x6420), __byte_perm(arg[2], arg[3], 0x6420));
   }
 }
 
+// One thread per 2 x 2 input quad (2a..2a+1, 2b..2b+1) and 8 channels: exactly the windows (a..a+1, b..b+1) reach the
+// quad, so four gradients and four code words serve four outputs (a thread per pixel read nine of each).
 template <typename T>
 __global__ void __launch_bounds__(256)
-MaxPoolBwdKernel(const T* __restrict__ dy, const uint8_t* __restrict__ idx, T* __restrict__ dx, int n, int h, int w,
+MaxPoolBwdKernel(const T* __restrict__ dy, const uint8_t* __restrict__ idx, T* __restrict__ dx, int64_t rows, int h, int w,
                  int c, int ho, int wo) {
   constexpr int V = 8;
   const int cv = c / V;
-  const int64_t total = static_cast<int64_t>(n) * h * w * cv;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int cg = static_cast<int>(i % cv);
-    int64_t pix  = i / cv;
-    const int iw = static_cast<int>(pix % w); pix /= w;
-    const int ih = static_cast<int>(pix % h);
-    const int in = static_cast<int>(pix / h);
-    float acc[V];
+  const int hq = (h + 1) / 2, wq = (w + 1) / 2;
+  const int i  = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= wq * cv) return;
+  const int b = i / cv, cg = i - b * cv;
+  for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {  // row = image * hq + a
+    const int64_t in = row / hq;
+    const int a      = static_cast<int>(row - in * hq);
+    Vec16<T> g[4];
+    uint2 code[4];
 #pragma unroll
-    for (int j = 0; j < V; ++j) acc[j] = 0.f;
-    // windows oh with 2*oh - 1 <= ih <= 2*oh + 1
-    const int oh_lo = ih / 2, oh_hi = (ih + 1) / 2;
-    const int ow_lo = iw / 2, ow_hi = (iw + 1) / 2;
-    for (int oh = oh_lo; oh <= oh_hi; ++oh) {
-      if (oh >= ho) continue;
-      const int r = ih - (oh * 2 - 1);
-      for (int ow = ow_lo; ow <= ow_hi; ++ow) {
-        if (ow >= wo) continue;
-        const int s = iw - (ow * 2 - 1);
-        const uint32_t code = static_cast<uint32_t>(r * 3 + s);
-        const int64_t opix  = (static_cast<int64_t>(in) * ho + oh) * wo + ow;
-        const uint2 packed  = *reinterpret_cast<const uint2*>(idx + opix * c + cg * V);
-        const Vec16<T> g    = LoadVec(dy + opix * c + cg * V);
-#pragma unroll
-        for (int j = 0; j < V; ++j) {
-          const uint32_t a = ((j < 4 ? packed.x : packed.y) >> ((j & 3) * 8)) & 0xffu;
-          if (a == code) acc[j] += ToFloat(g.v[j]);
-        }
+    for (int k = 0; k < 4; ++k) {
+      const int oh = a + (k >> 1), ow = b + (k & 1);
+      if (oh < ho && ow < wo) {
+        const int64_t at = ((in * ho + oh) * wo + ow) * c + cg * V;
+        g[k]    = LoadVec(dy + at);
+        code[k] = *reinterpret_cast<const uint2*>(idx + at);
+      } else {
+        code[k] = make_uint2(0xffffffffu, 0xffffffffu);  // matches no position
       }
     }
-    Vec16<T> o;
 #pragma unroll
-    for (int j = 0; j < V; ++j) o.v[j] = FromFloat<T>(acc[j]);
-    StoreVec(dx + ((static_cast<int64_t>(in) * h + ih) * w + iw) * c + cg * V, o);
+    for (int q = 0; q < 4; ++q) {
+      const int dh = q >> 1, dw = q & 1;
+      const int ih = 2 * a + dh, iw = 2 * b + dw;
+      if (ih >= h || iw >= w) continue;
+      float acc[V];
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[j] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        // window (a + kh, b + kw) covers input rows 2(a + kh) - 1 .. 2(a + kh) + 1
+        const int r = dh + 1 - 2 * (k >> 1), s = dw + 1 - 2 * (k & 1);
+        if (r < 0 || s < 0) continue;
+        const uint32_t want = static_cast<uint32_t>(r * 3 + s);
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+          const uint32_t got = ((j < 4 ? code[k].x : code[k].y) >> ((j & 3) * 8)) & 0xffu;
+          if (got == want) acc[j] += ToFloat(g[k].v[j]);
+        }
+      }
+      Vec16<T> o;
+#pragma unroll
+      for (int j = 0; j < V; ++j) o.v[j] = FromFloat<T>(acc[j]);
+      StoreVec(dx + ((in * h + ih) * w + iw) * c + cg * V, o);
+    }
   }
 }
 
-int GridFor(int64_t total) {
-  const int64_t blocks = (total + 255) / 256;
-  const int64_t cap    = static_cast<int64_t>(NumSMs()) * 16;
-  return static_cast<int>(blocks < cap ? blocks : cap);
+// Grid of the pooling kernels: x covers the columns of a row, y the rows.
+dim3 RowGrid(int64_t per_row, int64_t rows) {
+  return dim3(static_cast<unsigned>((per_row + 255) / 256), static_cast<unsigned>(std::min<int64_t>(rows, 65535)));
 }
 
 // Global average pooling of an NHWC activation: y[n, c] = mean over the hw pixels; one thread per (image, 8
@@ -172,16 +204,18 @@ int tipsk_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int n, int h, int 
   TIPSK_REQUIRE(c % 8 == 0, "maxpool: channel count must be a multiple of 8");
   TIPSK_REQUIRE(dtype == kBF16 || dtype == kF16, "maxpool: bf16 or fp16 only");
   const int ho = (h + 2 - 3) / 2 + 1, wo = (w + 2 - 3) / 2 + 1;
-  const int64_t total = static_cast<int64_t>(n) * ho * wo * (c / 8);
-  if (total == 0) return 0;
+  const int64_t per_row = static_cast<int64_t>(wo) * (c / 8), rows = static_cast<int64_t>(n) * ho;
+  if (per_row <= 0 || rows <= 0) return 0;
+  TIPSK_REQUIRE(per_row < (int64_t{1} << 30), "maxpool: a row has too many elements");
+  const dim3 grid = RowGrid(per_row, rows);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == kBF16)
-    MaxPoolFwdKernel<__nv_bfloat16><<<GridFor(total), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x),
+    MaxPoolFwdKernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x),
                                                                   static_cast<__nv_bfloat16*>(y),
-                                                                  static_cast<uint8_t*>(idx), n, h, w, c, ho, wo);
+                                                                  static_cast<uint8_t*>(idx), rows, h, w, c, ho, wo);
   else
-    MaxPoolFwdKernel<__half><<<GridFor(total), 256, 0, s>>>(static_cast<const __half*>(x), static_cast<__half*>(y),
-                                                            static_cast<uint8_t*>(idx), n, h, w, c, ho, wo);
+    MaxPoolFwdKernel<__half><<<grid, 256, 0, s>>>(static_cast<const __half*>(x), static_cast<__half*>(y),
+                                                            static_cast<uint8_t*>(idx), rows, h, w, c, ho, wo);
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
@@ -191,17 +225,19 @@ int tipsk_maxpool3x3s2_bwd(const void* dy, const void* idx, void* dx, int n, int
   TIPSK_REQUIRE(c % 8 == 0, "maxpool: channel count must be a multiple of 8");
   TIPSK_REQUIRE(dtype == kBF16 || dtype == kF16, "maxpool: bf16 or fp16 only");
   const int ho = (h + 2 - 3) / 2 + 1, wo = (w + 2 - 3) / 2 + 1;
-  const int64_t total = static_cast<int64_t>(n) * h * w * (c / 8);
-  if (total == 0) return 0;
+  const int64_t per_row = static_cast<int64_t>((w + 1) / 2) * (c / 8), rows = static_cast<int64_t>(n) * ((h + 1) / 2);
+  if (per_row <= 0 || rows <= 0) return 0;
+  TIPSK_REQUIRE(per_row < (int64_t{1} << 30), "maxpool: a row has too many elements");
+  const dim3 grid = RowGrid(per_row, rows);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == kBF16)
-    MaxPoolBwdKernel<__nv_bfloat16><<<GridFor(total), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dy),
+    MaxPoolBwdKernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dy),
                                                                   static_cast<const uint8_t*>(idx),
-                                                                  static_cast<__nv_bfloat16*>(dx), n, h, w, c, ho, wo);
+                                                                  static_cast<__nv_bfloat16*>(dx), rows, h, w, c, ho, wo);
   else
-    MaxPoolBwdKernel<__half><<<GridFor(total), 256, 0, s>>>(static_cast<const __half*>(dy),
+    MaxPoolBwdKernel<__half><<<grid, 256, 0, s>>>(static_cast<const __half*>(dy),
                                                             static_cast<const uint8_t*>(idx), static_cast<__half*>(dx),
-                                                            n, h, w, c, ho, wo);
+                                                            rows, h, w, c, ho, wo);
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
