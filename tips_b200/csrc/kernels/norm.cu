@@ -8,6 +8,8 @@
 //
 // Layout: activations are a row-major [M, C] matrix (M = N*H*W for NHWC batch
 // norm, rows x cols for layer norm), 16-byte vectors along C.
+#include <algorithm>
+
 #include "kernels/common.cuh"
 #include "kernels/tips_kernels.h"
 
@@ -38,7 +40,8 @@ __device__ __forceinline__ void StoreV(T* p, const float (&in)[V]) {
 struct BnGeom {
   int tx, ty;      // block = tx * ty threads; tx vector-columns, ty rows
   int col_tiles;   // grid.x
-  int partials;    // grid.y of the reduction kernels and of the backward apply kernel (3 blocks per SM, 2 waves)
+  int partials;    // grid.y of the reduction kernels (3 blocks per SM, one wave: a second one pays the tree again)
+  int bwd_rows;    // grid.y of the backward apply kernel (3 blocks per SM, 2 waves)
   int fwd_rows;    // grid.y of the forward apply kernel (4 blocks per SM, 2 waves)
 };
 
@@ -51,11 +54,12 @@ BnGeom BnGeometry(int64_t m, int c, int v) {
   g.col_tiles = vec_cols / g.tx;
   // Whole waves: the kernels are grid-stride loops over the rows, and a last partial wave costs a full one.
   int64_t maxp = (m + g.ty * 4 - 1) / (g.ty * 4);
-  int64_t want = (static_cast<int64_t>(NumSMs()) * 6 + g.col_tiles - 1) / g.col_tiles;
-  if (want > maxp) want = maxp;
-  if (want < 1) want = 1;
-  if (want > 1024) want = 1024;
-  g.partials = static_cast<int>(want);
+  auto rows_for = [&](int blocks_per_sm) {
+    const int64_t want = (static_cast<int64_t>(NumSMs()) * blocks_per_sm + g.col_tiles - 1) / g.col_tiles;
+    return static_cast<int>(std::min<int64_t>(std::max<int64_t>(std::min(want, maxp), 1), 1024));
+  };
+  g.partials = rows_for(3);
+  g.bwd_rows = rows_for(6);
   int64_t fwd = (static_cast<int64_t>(NumSMs()) * 8 + g.col_tiles - 1) / g.col_tiles;
   if (fwd > maxp) fwd = maxp;
   if (fwd < 1) fwd = 1;
@@ -354,7 +358,7 @@ int tipsk_bn_partials(int64_t m, int c) {
   int best = 1;
   for (int v = 1; v <= 8; v *= 2)
     if (c % v == 0) {
-      int p = BnGeometry(m, c, v).partials;
+      int p = BnGeometry(m, c, v).bwd_rows;  // at least the rows the reduction writes; callers size workspaces with it
       if (p > best) best = p;
     }
   return best + 1;  // one more row: the column sums of the partial rows
@@ -432,7 +436,7 @@ int tipsk_bn_bwd(const void* dy, const void* x, const void* y, const float* gamm
                                                          static_cast<const T*>(y), save_mean, save_invstd, workspace, m,
                                                          c, relu);
     BnFinalizeKernel<<<CeilDiv(2 * c, 32), dim3(32, kFinalizeRows), 0, s>>>(workspace, g.partials, c);
-    BnBwdApplyKernel<T, V><<<grid, block, smem, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x),
+    BnBwdApplyKernel<T, V><<<dim3(g.col_tiles, g.bwd_rows), block, smem, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x),
                                                   static_cast<const T*>(y), gamma, save_mean, save_invstd,
                                                   static_cast<T*>(dx), static_cast<T*>(dresidual), dgamma, dbeta,
                                                   workspace, g.partials, m, c, relu);
@@ -484,7 +488,7 @@ int tipsk_bn_bwd_bitmask(const void* dy, const void* x, const void* relu_mask, c
                                                             save_mean, save_invstd, workspace, m, c, 1, nullptr, nullptr,
                                                             static_cast<const uint8_t*>(relu_mask));
     BnFinalizeKernel<<<CeilDiv(2 * c, 32), dim3(32, kFinalizeRows), 0, s>>>(workspace, g.partials, c);
-    BnBwdApplyKernel<T, V, 2><<<grid, block, smem, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x), nullptr, gamma,
+    BnBwdApplyKernel<T, V, 2><<<dim3(g.col_tiles, g.bwd_rows), block, smem, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x), nullptr, gamma,
                                                      save_mean, save_invstd, static_cast<T*>(dx),
                                                      static_cast<T*>(dresidual), dgamma, dbeta, workspace, g.partials, m,
                                                      c, 1, nullptr, static_cast<const uint8_t*>(relu_mask));
@@ -509,7 +513,7 @@ int tipsk_bn_bwd_relu_recompute(const void* dy, const void* x, const float* gamm
                                                                nullptr, save_mean, save_invstd, workspace, m, c, 1,
                                                                gamma, beta);
     BnFinalizeKernel<<<CeilDiv(2 * c, 32), dim3(32, kFinalizeRows), 0, s>>>(workspace, g.partials, c);
-    BnBwdApplyKernel<T, V, 1><<<grid, block, smem, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x), nullptr,
+    BnBwdApplyKernel<T, V, 1><<<dim3(g.col_tiles, g.bwd_rows), block, smem, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x), nullptr,
                                                         gamma, save_mean, save_invstd, static_cast<T*>(dx), nullptr,
                                                         dgamma, dbeta, workspace, g.partials, m, c, 1, beta);
   });
