@@ -24,6 +24,60 @@ def _rand(*shape, scale=0.5, dtype=BF16, seed=0):
     return (torch.randn(*shape, generator=g, device=DEV) * scale).to(dtype)
 
 
+# one CTA pair, a ragged last tile in each direction, several tiles per pair, a K of one block and with a remainder
+GEMM = [(256, 256, 64), (257, 512, 72), (300, 1000, 200), (512, 264, 1024), (4100, 1032, 136), (20000, 1024, 264)]
+
+
+@pytest.mark.parametrize("m,n,k", GEMM)
+@pytest.mark.parametrize("act", [None, "relu", "gelu"])
+def test_linear_products(m, n, k, act):
+    from tips_b200.ops.linear import gemm_nn, gemm_status, gemm_tn
+    a, b, bias = _rand(m, k), _rand(n, k, seed=1), _rand(n, seed=2)
+    ref_pre = a.double() @ b.double().t() + bias.double()
+    ref = {None: lambda t: t, "relu": F.relu, "gelu": F.gelu}[act](ref_pre)
+    y, pre = gemm_tn(a, b, bias, act, want_pre=True)
+    _close(pre, ref_pre)
+    _close(y, ref)
+    _close(gemm_tn(a, b, bias, act), ref)
+    if act is None:
+        nn = ref_pre - bias.double()
+        bt = b.t().contiguous()
+        _close(gemm_nn(a, bt), nn)
+        into = _rand(m, n, seed=3)
+        want = into.double() + nn
+        # the product is rounded to bf16 before the addition, and the sum once more
+        _close(gemm_nn(a, bt, into=into), want, slack=2.0 ** -8)
+    assert gemm_status() == 0
+
+
+@pytest.mark.parametrize("rows,n,k", [(16, 64, 64), (77, 256, 128), (1232, 320, 1024), (4096, 1024, 1024), (8200, 4096, 192)])
+def test_weight_gradient_in_bf16(rows, n, k):
+    from tips_b200.ops.linear import _weight_grad, gemm_status
+    dz, x = _rand(rows, n), _rand(rows, k, seed=1)
+    ref = dz.double().t() @ x.double()
+    _close(_weight_grad(dz, x, BF16), ref)
+    _close(_weight_grad(dz, x), ref)
+    assert gemm_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 64, 4096), (1232, 1024, 30528), (256, 2048, 4104), (300, 72, 8200)])
+def test_split_contraction(m, n, k):
+    from tips_b200.ops import base
+    from tips_b200.ops.linear import gemm_nn, gemm_status, gemm_tn
+    assert base.K().tipsk_gemm_splits(m, n, k) > 1
+    a, b, bias = _rand(m, k, scale=0.1), _rand(n, k, scale=0.1, seed=1), _rand(n, seed=2)
+    ref = a.double() @ b.double().t()
+    y, pre = gemm_tn(a, b, bias, "gelu", want_pre=True)
+    _close(pre, ref + bias.double())
+    _close(y, F.gelu(ref + bias.double()))
+    bt = b.t().contiguous()
+    _close(gemm_nn(a, bt), ref)
+    into = _rand(m, n, seed=3)
+    want = into.double() + ref
+    _close(gemm_nn(a, bt, into=into), want)
+    assert gemm_status() == 0
+
+
 @pytest.mark.parametrize("n,c,h,w", [(1, 8, 1, 1), (2, 8, 2, 3), (3, 72, 5, 8), (2, 64, 31, 33), (1, 2056, 4, 4)])
 def test_maxpool_edges(n, c, h, w):
     from tips_b200.ops.pool import max_pool_3x3_s2

@@ -20,6 +20,8 @@
 // the BERT-shaped encoder's linear layers.
 #include <cuda.h>
 
+#include <algorithm>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -42,6 +44,8 @@ struct GemmParams {
   int tma_store;               // 1: the output goes through shared memory and the TMA store unit
   int accumulate;              // 1 (TMA store path only): add to what C holds, with a reduce-add store
   int bias_vec;                // 1: bias is 16-byte aligned, so eight values can be read with one load
+  float* partial;              // pair kernel, K split over several tiles: [splits][m][n] fp32 partial products
+  int splits;
 };
 
 // Eight consecutive bias values as floats (zeros without a bias): one 16-byte load when the bias is 16-byte aligned
@@ -61,6 +65,14 @@ __device__ __forceinline__ void LoadBias8(const GemmParams& p, int col, float (&
       if (col + j < p.n) bv[j] = __bfloat162float(p.bias[col + j]);
   }
 }
+
+// The activation of a value that is rounded to bf16 next, and of a pair of them.
+__device__ __forceinline__ float2 GemmAct2(float x, float y, int act) {
+  if (act == 1) return make_float2(fmaxf(x, 0.f), fmaxf(y, 0.f));
+  if (act == 2) return SplitF2(Gelu2(MakeF2(x, y)));
+  return make_float2(x, y);
+}
+__device__ __forceinline__ float GemmAct(float x, int act) { return GemmAct2(x, x, act).x; }
 
 // Hands a staged 64-column box to the TMA store unit: a plain store, or a bf16 reduce-add into global memory.
 __device__ __forceinline__ void TmaStoreOrAdd2D(const CUtensorMap* tmap, int x, int y, const void* smem_src, int add) {
@@ -94,7 +106,7 @@ struct GemmCfg {
 template <int BN, bool kBMn = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-             const __grid_constant__ CUtensorMap tmap_c, GemmParams p) {
+             const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_pre, GemmParams p) {
   using Cfg = GemmCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -129,7 +141,7 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ElectOne()) {
       for (int kt = 0; kt < num_k; ++kt) {
         const int s = kt % Cfg::kStages;
         const uint32_t parity = ((kt / Cfg::kStages) & 1) ^ 1;
@@ -150,15 +162,15 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {  // the whole warp walks the loop, one lane issues
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (kBMn ? (1u << 16) : 0u) |
                                  (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
       bool ok = true;
       for (int kt = 0; kt < num_k && ok; ++kt) {
         const int s = kt % Cfg::kStages;
         const uint32_t parity = (kt / Cfg::kStages) & 1;
-        if (!MbarWait(&full_bar[s], parity)) {
-          atomicExch(p.error, 2);
+        if (!MbarWaitWarp(&full_bar[s], parity)) {
+          if (lane == 0) atomicExch(p.error, 2);
           ok = false;
           break;
         }
@@ -167,15 +179,17 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         const uint32_t b_addr = a_addr + Cfg::kABytes;
         const uint64_t adesc  = SmemDescSw128(a_addr);
         const uint64_t bdesc  = kBMn ? SmemDescMnSw128(b_addr, 8192) : SmemDescSw128(b_addr);
+        if (ElectOne()) {
 #pragma unroll
-        for (int k = 0; k < kBK / 16; ++k) {
-          // advancing 16 elements (32 bytes) along K inside the swizzle row = +2 in the address field;
-          // for the MN-major B sixteen K rows = 2048 bytes = +128
-          UmmaBf16(tmem_base, adesc + 2 * k, bdesc + (kBMn ? 128 : 2) * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < kBK / 16; ++k) {
+            // advancing 16 elements (32 bytes) along K inside the swizzle row = +2 in the address field;
+            // for the MN-major B sixteen K rows = 2048 bytes = +128
+            UmmaBf16(tmem_base, adesc + 2 * k, bdesc + (kBMn ? 128 : 2) * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+          }
+          UmmaCommit(&empty_bar[s]);
         }
-        UmmaCommit(&empty_bar[s]);
       }
-      UmmaCommit(tmem_full);  // arrives when every MMA issued so far has completed
+      if (ElectOne()) UmmaCommit(tmem_full);  // arrives when every MMA issued so far has completed
     }
   } else {
     const int q = warp & 3;  // TMEM lane quarter this warp may access
@@ -196,21 +210,23 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         TmemLoad32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(c * 32), acc);
         const int col0 = n0 + c * 32;
         uint8_t* box   = smem + (c >> 1) * (kBM * 128);
+        uint8_t* pbox  = box + (BN / 64) * (kBM * 128);  // the second output's boxes follow
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           alignas(16) __nv_bfloat16 o[8];
-#pragma unroll
+          alignas(16) __nv_bfloat16 pr[8];
           float bv[8];
           LoadBias8(p, col0 + g * 8, bv);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float x = __uint_as_float(acc[g * 8 + j]) + bv[j];
-            if (p.act == 1) x = fmaxf(x, 0.f);
-            else if (p.act == 2) x = 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-            o[j] = __float2bfloat16_rn(x);
+          for (int j = 0; j < 8; j += 2) {
+            const float x = __uint_as_float(acc[g * 8 + j]) + bv[j], y = __uint_as_float(acc[g * 8 + j + 1]) + bv[j + 1];
+            const float2 z = GemmAct2(x, y, p.act);
+            *reinterpret_cast<__nv_bfloat162*>(&pr[j]) = __floats2bfloat162_rn(x, y);
+            *reinterpret_cast<__nv_bfloat162*>(&o[j])  = __floats2bfloat162_rn(z.x, z.y);
           }
-          const int chunk = (c & 1) * 4 + g;  // 16-byte chunk inside the 128-byte row
-          *reinterpret_cast<uint4*>(box + r * 128 + ((chunk ^ (r & 7)) << 4)) = *reinterpret_cast<uint4*>(o);
+          const int off = r * 128 + ((((c & 1) * 4 + g) ^ (r & 7)) << 4);  // 16-byte chunk inside the swizzled row
+          *reinterpret_cast<uint4*>(box + off) = *reinterpret_cast<uint4*>(o);
+          if (p.pre) *reinterpret_cast<uint4*>(pbox + off) = *reinterpret_cast<uint4*>(pr);
         }
       }
       }
@@ -222,6 +238,7 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         for (int b = 0; b < BN / 64; ++b) {
           if (n0 + b * 64 < p.n) {
             TmaStoreOrAdd2D(&tmap_c, n0 + b * 64, m0, smem + b * (kBM * 128), p.accumulate);
+            if (p.pre) TmaStoreOrAdd2D(&tmap_pre, n0 + b * 64, m0, smem + (BN / 64 + b) * (kBM * 128), 0);
           }
         }
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -258,9 +275,7 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 float x = v[g * 8 + j];
-                if (p.act == 1) x = fmaxf(x, 0.f);
-                else if (p.act == 2) x = 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-                o[j] = __float2bfloat16_rn(x);
+                o[j] = __float2bfloat16_rn(GemmAct(x, p.act));
               }
               *reinterpret_cast<uint4*>(crow + g * 8) = *reinterpret_cast<uint4*>(o);
             }
@@ -268,9 +283,7 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             for (int j = 0; j < 32 && col0 + j < p.n && j < BN; ++j) {
               float x = v[j];
               if (prow) prow[j] = __float2bfloat16_rn(x);
-              if (p.act == 1) x = fmaxf(x, 0.f);
-              else if (p.act == 2) x = 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-              crow[j] = __float2bfloat16_rn(x);
+              crow[j] = __float2bfloat16_rn(GemmAct(x, p.act));
             }
           }
         }
@@ -346,7 +359,7 @@ GemmTnPersistentKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ElectOne()) {
       uint32_t it = 0;  // running k-stage counter over all tiles
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -372,7 +385,7 @@ GemmTnPersistentKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {  // the whole warp walks the loop, one lane issues
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (kBMn ? (1u << 16) : 0u) |
                                  (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
       uint32_t it = 0;
@@ -380,16 +393,16 @@ GemmTnPersistentKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
         const int buf = local & 1;
-        if (!MbarWait(&tmem_empty[buf], ((local >> 1) & 1) ^ 1)) {  // the epilogue has drained this accumulator
-          atomicExch(p.error, 4);
+        if (!MbarWaitWarp(&tmem_empty[buf], ((local >> 1) & 1) ^ 1)) {  // the epilogue has drained this accumulator
+          if (lane == 0) atomicExch(p.error, 4);
           break;
         }
         TcFenceAfter();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * BN);
         for (int kt = 0; kt < num_k; ++kt, ++it) {
           const int s = it % Cfg::kStages;
-          if (!MbarWait(&full_bar[s], (it / Cfg::kStages) & 1)) {
-            atomicExch(p.error, 2);
+          if (!MbarWaitWarp(&full_bar[s], (it / Cfg::kStages) & 1)) {
+            if (lane == 0) atomicExch(p.error, 2);
             ok = false;
             break;
           }
@@ -397,12 +410,14 @@ GemmTnPersistentKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           const uint32_t a_addr = SmemAddr(smem + s * Cfg::kStageBytes);
           const uint64_t adesc  = SmemDescSw128(a_addr);
           const uint64_t bdesc  = kBMn ? SmemDescMnSw128(a_addr + Cfg::kABytes, 8192) : SmemDescSw128(a_addr + Cfg::kABytes);
+          if (ElectOne()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            UmmaBf16(tmem_d, adesc + 2 * k, bdesc + (kBMn ? 128 : 2) * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
-          UmmaCommit(&empty_bar[s]);
+            for (int k = 0; k < kBK / 16; ++k)
+              UmmaBf16(tmem_d, adesc + 2 * k, bdesc + (kBMn ? 128 : 2) * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            UmmaCommit(&empty_bar[s]);
+          }
         }
-        if (ok) UmmaCommit(&tmem_full[buf]);
+        if (ok && ElectOne()) UmmaCommit(&tmem_full[buf]);
       }
     }
   } else {
@@ -434,9 +449,7 @@ GemmTnPersistentKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               float x = __uint_as_float(acc[g * 8 + j]) + bv[j];
-              if (p.act == 1) x = fmaxf(x, 0.f);
-              else if (p.act == 2) x = 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-              o[j] = __float2bfloat16_rn(x);
+              o[j] = __float2bfloat16_rn(GemmAct(x, p.act));
             }
             const int chunk = (c & 1) * 4 + g;
             *reinterpret_cast<uint4*>(box + r * 128 + ((chunk ^ (r & 7)) << 4)) = *reinterpret_cast<uint4*>(o);
@@ -473,72 +486,96 @@ GemmTnPersistentKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   }
 }
 
-// ---------------------------------------------------------------- 256 x 256 tiles
-// A 128 x 256 tile streams 48 KB per K block from L2 for 512 tensor-core clocks of work, and an SM takes 64 bytes per
-// clock from L2: the main loop is load-bound at two thirds of the tensor peak.  Here one CTA owns a 256 x 256 tile: two
-// A blocks share one B block, 64 KB per 1024 clocks of work, so loads and MMAs balance.  The two accumulators fill all
-// 512 TMEM columns, so the epilogue of a tile cannot overlap the MMAs of the next (only its loads); the variant is
-// chosen for long K and grids that fill whole waves.  Persistent, one CTA per SM.
-struct Big256Cfg {
-  static constexpr int kBN         = 256;
-  static constexpr int kStages     = 3;
-  static constexpr int kABytes     = kBM * kBK * 2;          // one 128-row half
-  static constexpr int kBBytes     = kBN * kBK * 2;
-  static constexpr int kStageBytes = 2 * kABytes + kBBytes;  // 64 KB
-  static constexpr int kStagingBytes = 2 * kBM * 128;        // two 64-column boxes, used alternately
-  static constexpr int kTmemCols   = 512;
-  static constexpr int kSmemBytes  = kStages * kStageBytes + kStagingBytes + 1024 + 256;
+// ---------------------------------------------------------------- CTA pairs, 256 x 256 tiles
+// A pair of CTAs computes a 256 x 256 tile: per K block each SM takes 128 rows of A and 128 columns of B from L2
+// (32 KB) for 512 tensor-core clocks, 64 bytes per clock, where a single CTA's 128 x 256 tile needs 96; and the
+// accumulators take 256 TMEM columns per CTA, so two tiles fit and the epilogue of one overlaps the MMAs of the next.
+// Eight epilogue warps: the GELU of 128 x 256 values per CTA costs about as many issue slots as the 8192 clocks of MMAs of
+// a K = 1024 tile, so it needs two warps per scheduler, and two values per instruction (with erff, one at a time, the
+// same product took 183 us).  A second output
+// (the value before the activation, which the backward pass of GELU reads) leaves through the same staging boxes.
+// Bound by the tensor cores.  Measured against the single-CTA kernels it took over from (us, M x N x K): 16384 x 4096 x
+// 1024 with bias 100 : 114 (1377 TFLOP/s), the same with GELU and the second output 159 : 307, 1232 x 30528 x 1024 71 : 105;
+// A and B MN-major (a weight gradient) 4096 x 1024 x 16384 92 : 114, 30528 x 1024 x 1232 57 : 128.
+struct PairCfg {
+  static constexpr int kBN            = 256;
+  static constexpr int kStages        = 5;
+  static constexpr int kABytes        = kBM * kBK * 2;
+  static constexpr int kBBytes        = (kBN / 2) * kBK * 2;
+  static constexpr int kStageBytes    = kABytes + kBBytes;      // 32 KB per CTA
+  static constexpr int kBoxBytes      = kBM * 128;              // 128 rows x 64 columns
+  static constexpr int kStagingBytes  = 4 * kBoxBytes;          // two boxes per epilogue group
+  static constexpr int kTmemCols      = 512;
+  static constexpr int kThreads       = 320;                    // TMA warp, MMA warp, eight epilogue warps
+  static constexpr int kSmemBytes     = kStages * kStageBytes + kStagingBytes + 1024 + 256;
 };
 
-template <bool kBMn>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-GemmTn256Kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                const __grid_constant__ CUtensorMap tmap_c, GemmParams p) {
-  using Cfg = Big256Cfg;
+// What the epilogue of the pair kernel writes: the bf16 result, also the value before the activation, or fp32 partials.
+constexpr int kOutPlain = 0, kOutPre = 1, kOutPartial = 2;
+
+__host__ __device__ __forceinline__ int SplitBegin(int k_blocks, int split, int splits) {
+  return static_cast<int>(static_cast<int64_t>(k_blocks) * split / splits);
+}
+
+template <bool kAMn, bool kBMn, int kOut>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg::kThreads, 1)
+GemmPairKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+               const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_pre, GemmParams p) {
+  using Cfg = PairCfg;
   constexpr int BN = Cfg::kBN;
+  constexpr bool kPre = kOut == kOutPre, kSplit = kOut == kOutPartial;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem    = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + Cfg::kStages * Cfg::kStageBytes;
-  uint64_t* full_bar   = reinterpret_cast<uint64_t*>(staging + Cfg::kStagingBytes);
-  uint64_t* empty_bar  = full_bar + Cfg::kStages;
-  uint64_t* tmem_full  = empty_bar + Cfg::kStages;
-  uint64_t* tmem_empty = tmem_full + 1;
-  uint32_t* tmem_slot  = reinterpret_cast<uint32_t*>(tmem_empty + 1);
+  uint64_t* full_bar   = reinterpret_cast<uint64_t*>(staging + Cfg::kStagingBytes);  // the leader's copy is used
+  uint64_t* empty_bar  = full_bar + Cfg::kStages;   // each CTA's own
+  uint64_t* tmem_full  = empty_bar + Cfg::kStages;  // [2], each CTA's own
+  uint64_t* tmem_empty = tmem_full + 2;             // [2], the leader's copy is used
+  uint32_t* tmem_slot  = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_k   = (p.k + kBK - 1) / kBK;
+  const int cta  = static_cast<int>(ClusterCtaRank());
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int all_k   = (p.k + kBK - 1) / kBK;
   const int tiles_n = (p.n + BN - 1) / BN;
   const int tiles_m = (p.m + 2 * kBM - 1) / (2 * kBM);
-  const int num_tiles = tiles_m * tiles_n;
+  const int plane     = tiles_m * tiles_n;
+  const int num_tiles = kSplit ? plane * p.splits : plane;  // a tile of split s covers its share of the K blocks
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::kStages; ++s) {
       MbarInit(&full_bar[s], 1);
       MbarInit(&empty_bar[s], 1);
     }
-    MbarInit(tmem_full, 1);
-    MbarInit(tmem_empty, 4);  // one arrival per epilogue warp
+    for (int b = 0; b < 2; ++b) {
+      MbarInit(&tmem_full[b], 1);
+      MbarInit(&tmem_empty[b], 16);  // eight epilogue warps of each CTA
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(tmem_slot)),
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(tmem_slot)),
                  "r"(static_cast<uint32_t>(Cfg::kTmemCols))
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   TcFenceBefore();
   __syncthreads();
+  ClusterSync();  // both CTAs' barriers exist before any remote arrival
   TcFenceAfter();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ElectOne()) {
       uint32_t it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int m0 = (tile / tiles_n) * 2 * kBM, n0 = (tile % tiles_n) * BN;
-        for (int kt = 0; kt < num_k; ++kt, ++it) {
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
+        const int mn = kSplit ? tile % plane : tile, sp = kSplit ? tile / plane : 0;
+        const int k_lo = kSplit ? SplitBegin(all_k, sp, p.splits) : 0;
+        const int k_hi = kSplit ? SplitBegin(all_k, sp + 1, p.splits) : all_k;
+        const int m0 = (mn / tiles_n) * 2 * kBM + cta * kBM, n0 = (mn % tiles_n) * BN + cta * (BN / 2);
+        for (int kt = k_lo; kt < k_hi; ++kt, ++it) {
           const int s = it % Cfg::kStages;
           if (!MbarWait(&empty_bar[s], ((it / Cfg::kStages) & 1) ^ 1)) {
             atomicExch(p.error, 1);
@@ -546,135 +583,222 @@ GemmTn256Kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             break;
           }
           uint8_t* a_dst = smem + s * Cfg::kStageBytes;
-          uint8_t* b_dst = a_dst + 2 * Cfg::kABytes;
-          MbarExpectTx(&full_bar[s], Cfg::kStageBytes);
-          TmaLoad2D(a_dst, &tmap_a, kt * kBK, m0, &full_bar[s]);
-          TmaLoad2D(a_dst + Cfg::kABytes, &tmap_a, kt * kBK, m0 + kBM, &full_bar[s]);
-          if (kBMn) {
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j) TmaLoad2D(b_dst + j * 8192, &tmap_b, n0 + j * 64, kt * kBK, &full_bar[s]);
+          uint8_t* b_dst = a_dst + Cfg::kABytes;
+          if (cta == 0) MbarExpectTx(&full_bar[s], 2 * Cfg::kStageBytes);  // both CTAs' bytes
+          if (kAMn) {
+            TmaLoad2DPair(a_dst, &tmap_a, m0, kt * kBK, &full_bar[s]);
+            TmaLoad2DPair(a_dst + 8192, &tmap_a, m0 + 64, kt * kBK, &full_bar[s]);
           } else {
-            TmaLoad2D(b_dst, &tmap_b, kt * kBK, n0, &full_bar[s]);
+            TmaLoad2DPair(a_dst, &tmap_a, kt * kBK, m0, &full_bar[s]);
+          }
+          if (kBMn) {
+            TmaLoad2DPair(b_dst, &tmap_b, n0, kt * kBK, &full_bar[s]);
+            TmaLoad2DPair(b_dst + 8192, &tmap_b, n0 + 64, kt * kBK, &full_bar[s]);
+          } else {
+            TmaLoad2DPair(b_dst, &tmap_b, kt * kBK, n0, &full_bar[s]);
           }
         }
       }
+      // The leader's commits arrive on this CTA's barriers: wait for the last of every stage before leaving.
+      for (uint32_t i = it > Cfg::kStages ? it - Cfg::kStages : 0; i < it && ok; ++i)
+        if (!MbarWait(&empty_bar[i % Cfg::kStages], (i / Cfg::kStages) & 1)) {
+          atomicExch(p.error, 1);
+          ok = false;
+        }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (kBMn ? (1u << 16) : 0u) |
-                                 (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
+    if (cta == 0) {  // the whole warp walks the loop, one lane issues
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (kAMn ? (1u << 15) : 0u) | (kBMn ? (1u << 16) : 0u) |
+                                 (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>((2 * kBM) >> 4) << 24);
       uint32_t it = 0;
       int local = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
-        if (!MbarWait(tmem_empty, (local & 1) ^ 1)) {  // the epilogue has drained both accumulators
-          atomicExch(p.error, 4);
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++local) {
+        const int buf = local & 1;
+        if (!MbarWaitWarp(&tmem_empty[buf], ((local >> 1) & 1) ^ 1)) {
+          if (lane == 0) atomicExch(p.error, 4);
           break;
         }
         TcFenceAfter();
+        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * BN);
+        const int sp    = kSplit ? tile / plane : 0;
+        const int num_k = kSplit ? SplitBegin(all_k, sp + 1, p.splits) - SplitBegin(all_k, sp, p.splits) : all_k;
         for (int kt = 0; kt < num_k; ++kt, ++it) {
           const int s = it % Cfg::kStages;
-          if (!MbarWait(&full_bar[s], (it / Cfg::kStages) & 1)) {
-            atomicExch(p.error, 2);
+          if (!MbarWaitWarp(&full_bar[s], (it / Cfg::kStages) & 1)) {
+            if (lane == 0) atomicExch(p.error, 2);
             ok = false;
             break;
           }
           TcFenceAfter();
           const uint32_t a_addr = SmemAddr(smem + s * Cfg::kStageBytes);
-          const uint32_t b_addr = a_addr + 2 * Cfg::kABytes;
-          const uint64_t bdesc  = kBMn ? SmemDescMnSw128(b_addr, 8192) : SmemDescSw128(b_addr);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint64_t adesc = SmemDescSw128(a_addr + h * Cfg::kABytes);
+          const uint64_t adesc  = kAMn ? SmemDescMnSw128(a_addr, 8192) : SmemDescSw128(a_addr);
+          const uint64_t bdesc  = kBMn ? SmemDescMnSw128(a_addr + Cfg::kABytes, 8192) : SmemDescSw128(a_addr + Cfg::kABytes);
+          if (ElectOne()) {
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k)
-              UmmaBf16(tmem_base + static_cast<uint32_t>(h * BN), adesc + 2 * k, bdesc + (kBMn ? 128 : 2) * k, idesc,
-                       (kt > 0 || k > 0) ? 1u : 0u);
+              UmmaBf16Pair(tmem_d, adesc + (kAMn ? 128 : 2) * k, bdesc + (kBMn ? 128 : 2) * k, idesc,
+                           (kt > 0 || k > 0) ? 1u : 0u);
+            UmmaCommitPair(&empty_bar[s]);
           }
-          UmmaCommit(&empty_bar[s]);
         }
-        if (ok) UmmaCommit(tmem_full);
+        if (ok && ElectOne()) UmmaCommitPair(&tmem_full[buf]);
       }
     }
   } else {
-    const int q = warp & 3;
-    const int r = q * 32 + lane;
-    constexpr int kBoxes = BN / 64;
+    // Two groups of four warps: group g drains columns [128 g, 128 g + 128) as two boxes of 64.
+    const int q = warp & 3;                // TMEM lane quarter
+    const int g = (warp - 2) >> 2;
+    const int r = q * 32 + lane;           // row of this CTA's half tile
+    const bool issuer = (warp == 2 || warp == 6) && lane == 0;
+    uint8_t* boxes = staging + g * 2 * Cfg::kBoxBytes;
     int local = 0;
-    uint32_t boxes_done = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
-      const int m0 = (tile / tiles_n) * 2 * kBM, n0 = (tile % tiles_n) * BN;
-      if (ok && !MbarWait(tmem_full, local & 1)) {
+    for (int tile = pair; tile < num_tiles; tile += pairs, ++local) {
+      const int mn = kSplit ? tile % plane : tile;
+      const int m0 = (mn / tiles_n) * 2 * kBM + cta * kBM, n0 = (mn % tiles_n) * BN + g * (BN / 2);
+      const int buf = local & 1;
+      if (ok && !MbarWait(&tmem_full[buf], (local >> 1) & 1)) {
         if (lane == 0) atomicExch(p.error, 3);
         ok = false;
       }
       TcFenceAfter();
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t tsrc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(h * BN);
-        uint32_t acc[2][32];
-        if (ok) TmemLoad32Async(tsrc, acc[0]);
+      const uint32_t tsrc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN + g * (BN / 2));
+      uint32_t acc[2][32];
+      if (ok) TmemLoad32Async(tsrc, acc[0]);
+      if constexpr (kSplit) {  // fp32 partial rows, straight from the registers: 128 bytes per lane and chunk
+        float* row = p.partial + (static_cast<int64_t>(tile / plane) * p.m + m0 + r) * p.n;
 #pragma unroll
-        for (int b = 0; b < kBoxes; ++b, ++boxes_done) {
-          uint8_t* box = staging + (boxes_done & 1) * (kBM * 128);
-          // the store that read this staging box two boxes ago must have finished reading it
-          if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          NamedBarSync(1, 128);
+        for (int c = 0; c < 4; ++c) {
+          if (!ok) continue;
+          TmemLoadWait(acc[c & 1]);
+          if (c + 1 < 4) TmemLoad32Async(tsrc + static_cast<uint32_t>((c + 1) * 32), acc[(c + 1) & 1]);
+          const int col0 = n0 + c * 32;
+          if (m0 + r < p.m) {
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int c = 2 * b + half;
-            if (ok) {
-              // the 32 bias values of this chunk as four 16-byte loads, in flight while the TMEM load completes
-              // (N is a multiple of 256 here, so the chunk is never ragged)
-              const int col0 = n0 + c * 32;
-              uint4 bq[4] = {};
-              if (p.bias) {
+            for (int u = 0; u < 8; ++u)  // n is a multiple of 8, so a vector is inside or outside as a whole
+              if (col0 + u * 4 < p.n)
+                *reinterpret_cast<uint4*>(row + col0 + u * 4) = make_uint4(acc[c & 1][u * 4], acc[c & 1][u * 4 + 1],
+                                                                           acc[c & 1][u * 4 + 2], acc[c & 1][u * 4 + 3]);
+          }
+        }
+        if (ok) {
+          TcFenceBefore();
+          __syncwarp();
+          if (lane == 0) MbarArriveLeader(&tmem_empty[buf]);
+        }
+        continue;
+      }
 #pragma unroll
-                for (int g = 0; g < 4; ++g) bq[g] = *reinterpret_cast<const uint4*>(p.bias + col0 + g * 8);
+      for (int b = 0; b < 2; ++b) {
+        uint8_t* box  = boxes + (kPre ? 0 : b) * Cfg::kBoxBytes;
+        uint8_t* pbox = boxes + Cfg::kBoxBytes;
+        // without a second output the boxes alternate, so the one written two boxes ago must have been read
+        if (issuer) {
+          if constexpr (kPre) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        }
+        NamedBarSync(1 + g, 128);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int c = 2 * b + half;
+          if (ok) {
+            const int col0 = n0 + c * 32;
+            TmemLoadWait(acc[c & 1]);
+            if (c + 1 < 4) TmemLoad32Async(tsrc + static_cast<uint32_t>((c + 1) * 32), acc[(c + 1) & 1]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              float bv[8];
+              LoadBias8(p, col0 + u * 8, bv);
+              alignas(16) __nv_bfloat16 o[8];
+              alignas(16) __nv_bfloat16 pr[8];
+#pragma unroll
+              for (int j = 0; j < 8; j += 2) {
+                const float x = __uint_as_float(acc[c & 1][u * 8 + j]) + bv[j];
+                const float y = __uint_as_float(acc[c & 1][u * 8 + j + 1]) + bv[j + 1];
+                const float2 z = GemmAct2(x, y, p.act);
+                if (kPre) *reinterpret_cast<__nv_bfloat162*>(&pr[j]) = __floats2bfloat162_rn(x, y);
+                *reinterpret_cast<__nv_bfloat162*>(&o[j]) = __floats2bfloat162_rn(z.x, z.y);
               }
-              TmemLoadWait(acc[c & 1]);
-              if (c + 1 < BN / 32) TmemLoad32Async(tsrc + static_cast<uint32_t>((c + 1) * 32), acc[(c + 1) & 1]);
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                alignas(16) __nv_bfloat16 o[8];
-                const __nv_bfloat16* bb = reinterpret_cast<const __nv_bfloat16*>(&bq[g]);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  float x = __uint_as_float(acc[c & 1][g * 8 + j]);
-                  if (p.bias) x += __bfloat162float(bb[j]);
-                  if (p.act == 1) x = fmaxf(x, 0.f);
-                  else if (p.act == 2) x = 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-                  o[j] = __float2bfloat16_rn(x);
-                }
-                const int chunk = half * 4 + g;
-                *reinterpret_cast<uint4*>(box + r * 128 + ((chunk ^ (r & 7)) << 4)) = *reinterpret_cast<uint4*>(o);
-              }
+              const int off = r * 128 + (((half * 4 + u) ^ (r & 7)) << 4);
+              *reinterpret_cast<uint4*>(box + off) = *reinterpret_cast<uint4*>(o);
+              if (kPre) *reinterpret_cast<uint4*>(pbox + off) = *reinterpret_cast<uint4*>(pr);
             }
           }
-          if (h == 1 && b == kBoxes - 1 && ok) {  // both accumulators are drained
-            TcFenceBefore();
-            __syncwarp();
-            if (lane == 0) MbarArrive(tmem_empty);
+        }
+        if (b == 1 && ok) {  // this warp's share of the accumulator is drained
+          TcFenceBefore();
+          __syncwarp();
+          if (lane == 0) MbarArriveLeader(&tmem_empty[buf]);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        NamedBarSync(1 + g, 128);
+        if (issuer) {
+          if (ok && n0 + b * 64 < p.n && m0 < p.m) {
+            TmaStoreOrAdd2D(&tmap_c, n0 + b * 64, m0, box, p.accumulate);
+            if (kPre) TmaStoreOrAdd2D(&tmap_pre, n0 + b * 64, m0, pbox, 0);
           }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          NamedBarSync(1, 128);
-          if (warp == 2 && lane == 0) {
-            if (ok && n0 + b * 64 < p.n && m0 + h * kBM < p.m)
-              TmaStoreOrAdd2D(&tmap_c, n0 + b * 64, m0 + h * kBM, box, p.accumulate);
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          }
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
     }
-    if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (!kSplit && issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   TcFenceBefore();
   __syncthreads();
+  ClusterSync();  // no CTA leaves while its peer may still signal its barriers or use its TMEM
+  TcFenceAfter();
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(static_cast<uint32_t>(Cfg::kTmemCols))
                  : "memory");
+  }
+}
+
+// Sum of the partial products, then bias and activation as in the other epilogues: eight columns per `lanes` threads,
+// which take every lanes-th split each and add up by shuffles (with few outputs a thread per output leaves most SMs
+// idle: 512 x 128 from 37 splits took 11 us).  With `accumulate` the sum is added to what C holds.
+__global__ void __launch_bounds__(256)
+GemmSplitSumKernel(GemmParams p, int lanes) {
+  const int vecs      = p.n / 8;
+  const int64_t total = static_cast<int64_t>(p.m) * vecs, plane = static_cast<int64_t>(p.m) * p.n;
+  const int64_t step  = static_cast<int64_t>(gridDim.x) * 256 / lanes;
+  const int64_t first = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) / lanes;
+  const int part      = threadIdx.x % lanes;
+  // whole warps run the same number of rounds, so that the shuffles below meet
+  for (int64_t i0 = first - (threadIdx.x & 31) / lanes; i0 < total; i0 += step) {
+    const int64_t i = i0 + (threadIdx.x & 31) / lanes;
+    const int64_t at  = i < total ? i : total - 1;
+    const int64_t row = at / vecs;
+    const int col     = static_cast<int>(at - row * vecs) * 8;
+    const float* src  = p.partial + row * p.n + col;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+#pragma unroll 4
+    for (int s = part; s < p.splits; s += lanes) {
+      const float4 a = *reinterpret_cast<const float4*>(src + s * plane), b = *reinterpret_cast<const float4*>(src + s * plane + 4);
+      v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+      v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+    }
+    for (int o = 1; o < lanes; o <<= 1)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+    if (i >= total || part != 0) continue;
+    float bv[8];
+    LoadBias8(p, col, bv);
+    __nv_bfloat16* dst = p.c + row * p.ldc + col;
+    Vec16<__nv_bfloat16> o, pr;
+    if (p.accumulate) o = LoadVec(dst);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float x = v[j] + bv[j];
+      pr.v[j] = __float2bfloat16_rn(x);
+      x       = GemmAct(x, p.act);
+      o.v[j]  = __float2bfloat16_rn(p.accumulate ? __bfloat162float(o.v[j]) + x : x);
+    }
+    if (p.pre) StoreVec(p.pre + row * p.ldc + col, pr);
+    StoreVec(dst, o);
   }
 }
 
@@ -707,8 +831,8 @@ int32_t* GemmErrorWord() {
 }
 
 template <int BN, bool kBMn = false>
-int LaunchGemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
-               cudaStream_t s) {
+int LaunchGemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tp,
+               const GemmParams& p, cudaStream_t s) {
   using Cfg = GemmCfg<BN>;
   static bool configured = false;
   if (!configured) {
@@ -718,7 +842,7 @@ int LaunchGemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& 
     configured = true;
   }
   dim3 grid((p.n + BN - 1) / BN, (p.m + kBM - 1) / kBM);
-  GemmTnKernel<BN, kBMn><<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(ta, tb, tc, p);
+  GemmTnKernel<BN, kBMn><<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(ta, tb, tc, tp, p);
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
@@ -740,32 +864,58 @@ int LaunchGemmPersistent(const CUtensorMap& ta, const CUtensorMap& tb, const CUt
   return 0;
 }
 
-template <bool kBMn>
-int LaunchGemm256(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
-                  cudaStream_t s) {
-  using Cfg = Big256Cfg;
-  static bool configured = false;
-  if (!configured) {
-    TIPSK_CUDA(cudaFuncSetAttribute(GemmTn256Kernel<kBMn>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    configured = true;
+// Pairs of SMs that can run a cluster of the pair kernel at the same time (an odd SM of a GPC stays without a partner).
+template <bool kAMn, bool kBMn, int kOut>
+int LaunchPair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tp,
+               const GemmParams& p, cudaStream_t s) {
+  using Cfg = PairCfg;
+  static std::atomic<int> resident{0};
+  int pairs = resident.load(std::memory_order_acquire);
+  if (pairs == 0) {
+    TIPSK_CUDA(cudaFuncSetAttribute(GemmPairKernel<kAMn, kBMn, kOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = dim3(NumSMs() & ~1);
+    cfg.blockDim         = dim3(Cfg::kThreads);
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cudaLaunchAttribute at{};
+    at.id               = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs    = &at;
+    cfg.numAttrs = 1;
+    TIPSK_CUDA(cudaOccupancyMaxActiveClusters(&pairs, GemmPairKernel<kAMn, kBMn, kOut>, &cfg));
+    TIPSK_REQUIRE(pairs > 0, "gemm: no CTA pair fits on this device");
+    resident.store(pairs, std::memory_order_release);
   }
-  const int tiles = ((p.n + 255) / 256) * ((p.m + 255) / 256);
-  const int grid  = tiles < NumSMs() ? tiles : NumSMs();
-  GemmTn256Kernel<kBMn><<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(ta, tb, tc, p);
+  const int64_t tiles = static_cast<int64_t>(CeilDiv(p.n, Cfg::kBN)) * CeilDiv(p.m, 2 * kBM) * (kOut == kOutPartial ? p.splits : 1);
+  const int grid = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
+  GemmPairKernel<kAMn, kBMn, kOut><<<grid, Cfg::kThreads, Cfg::kSmemBytes, s>>>(ta, tb, tc, tp, p);
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
 
-// Whether the 256 x 256 tile variant should take the problem: long enough K for the exposed epilogue to be a small
-// share of a tile, and a tile count that fills its waves.
-bool Prefer256(int m, int n, int k) {
-  static const bool off = getenv("TIPS_GEMM_NO_BM256") != nullptr;
-  if (off || n % 256 != 0 || m < 512 || k < 2048) return false;  // measured: no gain at K = 1024, +17..19 % at K = 4096
-  const int64_t tiles = static_cast<int64_t>((m + 255) / 256) * (n / 256);
-  const int64_t sms   = NumSMs();
-  const int64_t waves = (tiles + sms - 1) / sms;
-  const double fill   = static_cast<double>(tiles) / static_cast<double>(waves * sms);
-  return fill >= 0.80;
+// Both halves of a product whose K is split: the partial products, then their sum.
+template <bool kAMn, bool kBMn>
+int LaunchPairSplit(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t s) {
+  int rc = LaunchPair<kAMn, kBMn, kOutPartial>(ta, tb, ta, ta, p, s);
+  if (rc) return rc;
+  const int64_t vecs = static_cast<int64_t>(p.m) * (p.n / 8);
+  int lanes = 1;
+  while (lanes < 8 && lanes * 2 <= p.splits && vecs * lanes < static_cast<int64_t>(NumSMs()) * 1024) lanes *= 2;
+  const int64_t grid = std::min<int64_t>((vecs * lanes + 255) / 256, NumSMs() * 8);
+  GemmSplitSumKernel<<<static_cast<int>(grid), 256, 0, s>>>(p, lanes);
+  TIPSK_LAUNCH_CHECK();
+  return 0;
+}
+
+// Whether the CTA-pair kernel should take the problem: from about 1.25 tiles per pair of SMs on.  Measured against the
+// single-CTA kernels (us, M x N x K): 192 tiles 4096 x 3072 x 1024 32 : 45, 128 tiles 8192 x 1024 x 1024 27 : 32, 96
+// tiles 2048 x 3072 x 1024 26 : 31; below, a pair's single 256 x 256 tile and its exposed epilogue take longer than
+// two small CTAs per SM: 64 tiles 4096 x 1024 x 1024 21 : 17, 8192 x 512 x 1728 25 : 21.
+bool PreferPair(int m, int n, int k) {
+  (void)k;
+  const int64_t tiles = static_cast<int64_t>(CeilDiv(m, 2 * kBM)) * CeilDiv(n, PairCfg::kBN);
+  return n > 128 && tiles * 4 >= (NumSMs() / 2) * 5;
 }
 
 }  // namespace
@@ -790,12 +940,7 @@ int tipsk_gemm_bf16(const void* a, const void* b, void* c, const void* bias, voi
   else if (n <= 32) bn = 32;
   else if (n <= 64) bn = 64;
   else if (n % 256 == 0 && (static_cast<int64_t>(m) / kBM) * (n / 256) >= NumSMs()) bn = 256;
-  CUtensorMap ta, tb;
-  int rc = MakeTmap(&ta, a, m, k, lda, kBM);
-  if (rc) return rc;
-  rc = MakeTmap(&tb, b, n, k, ldb, bn);
-  if (rc) return rc;
-  GemmParams p;
+  GemmParams p{};
   p.c     = static_cast<__nv_bfloat16*>(c);
   p.pre   = static_cast<__nv_bfloat16*>(pre);
   p.bias  = static_cast<const __nv_bfloat16*>(bias);
@@ -803,33 +948,40 @@ int tipsk_gemm_bf16(const void* a, const void* b, void* c, const void* bias, voi
   TIPSK_REQUIRE(p.error != nullptr, "gemm: cannot allocate the error word");
   p.m = m; p.n = n; p.k = k; p.ldc = ldc; p.act = act; p.accumulate = 0;
   p.bias_vec = (bias != nullptr && reinterpret_cast<uintptr_t>(bias) % 16 == 0) ? 1 : 0;
-  // The coalesced store path needs 64-column boxes and a 16-byte aligned, 16-byte strided output.
-  p.tma_store = (bn >= 64 && pre == nullptr && ldc % 8 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0) ? 1 : 0;
-  CUtensorMap tc = ta;
+  // The coalesced store path needs 64-column boxes and 16-byte aligned, 16-byte strided outputs.
+  p.tma_store = (bn >= 64 && ldc % 8 == 0 && reinterpret_cast<uintptr_t>(c) % 16 == 0 &&
+                 reinterpret_cast<uintptr_t>(pre) % 16 == 0) ? 1 : 0;
+  const bool pair = p.tma_store && PreferPair(m, n, k);
+  CUtensorMap ta, tb;
+  int rc = MakeTmap(&ta, a, m, k, lda, kBM);
+  if (rc) return rc;
+  rc = MakeTmap(&tb, b, n, k, ldb, pair ? PairCfg::kBN / 2 : bn);
+  if (rc) return rc;
+  CUtensorMap tc = ta, tp = ta;
   if (p.tma_store) {
     rc = MakeTmap(&tc, c, m, n, ldc, kBM);
     if (rc) return rc;
+    if (pre) rc = MakeTmap(&tp, pre, m, n, ldc, kBM);
+    if (rc) return rc;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (p.tma_store && bn == 256 && Prefer256(m, n, k) && reinterpret_cast<uintptr_t>(bias) % 16 == 0)
-    return LaunchGemm256<false>(ta, tb, tc, p, s);
+  if (pair)
+    return pre ? LaunchPair<false, false, kOutPre>(ta, tb, tc, tp, p, s) : LaunchPair<false, false, kOutPlain>(ta, tb, tc, tp, p, s);
   // More tiles than SMs and a TMA-storable output: the persistent kernel overlaps epilogue and main loop.
-  static const bool no_persist = getenv("TIPS_GEMM_NO_PERSISTENT") != nullptr;
-  if (!no_persist && p.tma_store && (bn == 128 || bn == 256)) {
+  if (p.tma_store && pre == nullptr && bn == 128) {
     const int64_t tiles = static_cast<int64_t>((n + bn - 1) / bn) * ((m + kBM - 1) / kBM);
     // Measured on B200: the overlap pays when the epilogue is a visible share of a tile (K <= 2048) and
     // there are enough tiles to fill several waves; otherwise two independent CTAs per SM do better.
     if (tiles >= 3 * NumSMs() && k <= 2048) {
-      if (bn == 256) return LaunchGemmPersistent<256>(ta, tb, tc, p, s);
       return LaunchGemmPersistent<128>(ta, tb, tc, p, s);
     }
   }
   switch (bn) {
-    case 16: return LaunchGemm<16>(ta, tb, tc, p, s);
-    case 32: return LaunchGemm<32>(ta, tb, tc, p, s);
-    case 64: return LaunchGemm<64>(ta, tb, tc, p, s);
-    case 256: return LaunchGemm<256>(ta, tb, tc, p, s);
-    default: return LaunchGemm<128>(ta, tb, tc, p, s);
+    case 16: return LaunchGemm<16>(ta, tb, tc, tp, p, s);
+    case 32: return LaunchGemm<32>(ta, tb, tc, tp, p, s);
+    case 64: return LaunchGemm<64>(ta, tb, tc, tp, p, s);
+    case 256: return LaunchGemm<256>(ta, tb, tc, tp, p, s);
+    default: return LaunchGemm<128>(ta, tb, tc, tp, p, s);
   }
 }
 
@@ -851,7 +1003,7 @@ int tipsk_gemm_bf16_nn(const void* a, const void* b, void* c, int m, int n, int 
   if (rc) return rc;
   rc = MakeTmap(&tc, c, m, n, ldc, kBM);
   if (rc) return rc;
-  GemmParams p;
+  GemmParams p{};
   p.c = static_cast<__nv_bfloat16*>(c);
   p.pre = nullptr;
   p.bias = nullptr;
@@ -860,19 +1012,95 @@ int tipsk_gemm_bf16_nn(const void* a, const void* b, void* c, int m, int n, int 
   p.m = m; p.n = n; p.k = k; p.ldc = ldc; p.act = 0; p.tma_store = 1; p.accumulate = accumulate ? 1 : 0;
   p.bias_vec = 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (bn == 256 && Prefer256(m, n, k)) return LaunchGemm256<true>(ta, tb, tc, p, s);
-  if (bn != 64) {
+  if (PreferPair(m, n, k)) return LaunchPair<false, true, kOutPlain>(ta, tb, tc, tc, p, s);
+  if (bn == 128) {
     const int64_t tiles = static_cast<int64_t>((n + bn - 1) / bn) * ((m + kBM - 1) / kBM);
     if (tiles >= 3 * NumSMs() && k <= 2048) {
-      if (bn == 256) return LaunchGemmPersistent<256, true>(ta, tb, tc, p, s);
       return LaunchGemmPersistent<128, true>(ta, tb, tc, p, s);
     }
   }
   switch (bn) {
-    case 64: return LaunchGemm<64, true>(ta, tb, tc, p, s);
-    case 256: return LaunchGemm<256, true>(ta, tb, tc, p, s);
-    default: return LaunchGemm<128, true>(ta, tb, tc, p, s);
+    case 64: return LaunchGemm<64, true>(ta, tb, tc, tc, p, s);
+    case 256: return LaunchGemm<256, true>(ta, tb, tc, tc, p, s);
+    default: return LaunchGemm<128, true>(ta, tb, tc, tc, p, s);
   }
+}
+
+/* Whether the pair kernel is the one to run a product of this kind (the kinds of tipsk_gemm_bf16_split). */
+int tipsk_gemm_prefers_pair(int kind, int m, int n, int k) {
+  if (m < 64 || n < 64 || n % 8 != 0 || k <= 0) return 0;
+  return (kind == 2 || PreferPair(m, n, k)) ? 1 : 0;
+}
+
+/* Number of K splits with which tipsk_gemm_bf16_split should run the product (1: use the unsplit entry points). */
+int tipsk_gemm_splits(int m, int n, int k) {
+  if (m <= 0 || n < 64 || n % 8 != 0 || k <= 0) return 1;
+  const int64_t tiles = static_cast<int64_t>(CeilDiv(m, 2 * kBM)) * CeilDiv(n, PairCfg::kBN);
+  const int64_t pairs = NumSMs() / 2, blocks = CeilDiv(k, kBK);
+  if (2 * tiles > pairs) return 1;
+  const int64_t s = std::min<int64_t>(pairs / tiles, blocks / 8);  // at least eight K blocks per share
+  // A second launch and the partial products cost about 8 us: from K = 4096 on the shorter chain is worth them (us, split
+  // against not: 1024 x 1024 x 4096 25 : 28, 512 x 1024 x 4096 23 : 28, 1024 x 1024 x 30528 63 : 150; 2048 x 1024 x 4096
+  // with two shares 31 : 31, 1024 x 1024 x 2048 23 : 20).
+  if (k < 4096 || (k < 8192 && s < 4)) return 1;
+  return s < 2 ? 1 : static_cast<int>(s);
+}
+
+/* The three products of a linear layer with the contraction split over `splits` shares (few output tiles, long K):
+ *   kind 0  C[m,n] = act(A[m,k] * B[n,k]^T + bias), `pre` as in tipsk_gemm_bf16
+ *   kind 1  C[m,n] = A[m,k] * B[k,n], with `accumulate` added to C
+ *   kind 2  C[m,n] = A[k,m]^T * B[k,n]
+ * `partial`: fp32 workspace of splits * m * n elements.  n a multiple of 8, 16-byte aligned rows throughout. */
+int tipsk_gemm_bf16_split(int kind, const void* a, const void* b, void* c, const void* bias, void* pre, float* partial,
+                          int splits, int m, int n, int k, int lda, int ldb, int ldc, int act, int accumulate,
+                          void* stream) {
+  TIPSK_REQUIRE(kind >= 0 && kind <= 2 && m > 0 && n >= 64 && n % 8 == 0 && k > 0, "gemm_split: unsupported shape");
+  TIPSK_REQUIRE(lda % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0, "gemm_split: leading dimensions must be multiples of 8");
+  TIPSK_REQUIRE(partial != nullptr && splits >= 1 && splits <= CeilDiv(k, kBK), "gemm_split: workspace or split count");
+  TIPSK_REQUIRE(reinterpret_cast<uintptr_t>(c) % 16 == 0 && reinterpret_cast<uintptr_t>(pre) % 16 == 0 &&
+                    reinterpret_cast<uintptr_t>(partial) % 16 == 0,
+                "gemm_split: outputs must be 16-byte aligned");
+  CUtensorMap ta, tb;
+  int rc = kind == 2 ? MakeTmap(&ta, a, k, m, lda, kBK) : MakeTmap(&ta, a, m, k, lda, kBM);
+  if (rc) return rc;
+  rc = kind == 0 ? MakeTmap(&tb, b, n, k, ldb, PairCfg::kBN / 2) : MakeTmap(&tb, b, k, n, ldb, kBK);
+  if (rc) return rc;
+  GemmParams p{};
+  p.c     = static_cast<__nv_bfloat16*>(c);
+  p.pre   = static_cast<__nv_bfloat16*>(pre);
+  p.bias  = static_cast<const __nv_bfloat16*>(bias);
+  p.error = GemmErrorWord();
+  TIPSK_REQUIRE(p.error != nullptr, "gemm: cannot allocate the error word");
+  p.m = m; p.n = n; p.k = k; p.ldc = ldc; p.act = act; p.accumulate = accumulate ? 1 : 0;
+  p.bias_vec = (bias != nullptr && reinterpret_cast<uintptr_t>(bias) % 16 == 0) ? 1 : 0;
+  p.partial  = partial;
+  p.splits   = splits;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (kind == 0) return LaunchPairSplit<false, false>(ta, tb, p, s);
+  if (kind == 1) return LaunchPairSplit<false, true>(ta, tb, p, s);
+  return LaunchPairSplit<true, true>(ta, tb, p, s);
+}
+
+/* C[m,n] = A[k,m]^T * B[k,n], both operands row-major with the contraction over their rows (MN-major for the MMA, no
+ * transposed copies): the weight gradient dW = dz^T x of a linear layer, written in bf16 once.  m, n >= 64. */
+int tipsk_gemm_bf16_tt(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc,
+                       void* stream) {
+  TIPSK_REQUIRE(m >= 64 && n >= 64 && k > 0 && lda % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0,
+                "gemm_tt: leading dimensions must be multiples of 8 elements, m and n >= 64");
+  TIPSK_REQUIRE(reinterpret_cast<uintptr_t>(c) % 16 == 0, "gemm_tt: output must be 16-byte aligned");
+  CUtensorMap ta, tb, tc;
+  int rc = MakeTmap(&ta, a, k, m, lda, kBK);  // boxes of 64 contraction rows x 64 columns
+  if (rc) return rc;
+  rc = MakeTmap(&tb, b, k, n, ldb, kBK);
+  if (rc) return rc;
+  rc = MakeTmap(&tc, c, m, n, ldc, kBM);
+  if (rc) return rc;
+  GemmParams p{};
+  p.c = static_cast<__nv_bfloat16*>(c);
+  p.error = GemmErrorWord();
+  TIPSK_REQUIRE(p.error != nullptr, "gemm: cannot allocate the error word");
+  p.m = m; p.n = n; p.k = k; p.ldc = ldc; p.tma_store = 1;
+  return LaunchPair<true, true, kOutPlain>(ta, tb, tc, tc, p, static_cast<cudaStream_t>(stream));
 }
 
 /* Reads and clears the GEMM error word (0 ok; 1/2/3 = producer / MMA / epilogue wait ran out). Synchronises. */

@@ -49,6 +49,24 @@ __device__ __forceinline__ bool MbarWait(uint64_t* bar, uint32_t parity) {
   }
   return false;
 }
+// The same for a whole warp: every lane waits, and all of them get one answer, so that the warp stays converged.
+__device__ __forceinline__ bool MbarWaitWarp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, MbarWait(bar, parity));
+}
+// True in one lane of a converged warp, always the same one.  The instructions that a single thread issues (tcgen05.mma,
+// commits, TMA) take their operands from uniform registers: behind this predicate, in a loop that the whole warp walks,
+// the compiler knows that one lane is active and keeps descriptors and counters uniform.  Behind `lane == 0` the issue of
+// narrow MMAs was the bound: with nothing else changed, the 64-column kernels went from 139 to 111 us (3x3, 64 -> 64, 256
+// images of 56 x 56), 134 to 124 us (7x7 stem, 64 images of 224 x 224) and 140 to 117 us (its weight gradient).
+__device__ __forceinline__ bool ElectOne() {
+  uint32_t leader;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(leader));
+  return leader != 0;
+}
 __device__ __forceinline__ void TmaLoad2D(void* smem_dst, const CUtensorMap* tmap, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -128,6 +146,52 @@ __device__ __forceinline__ void TmemLoadWait(uint32_t (&r)[32]) {
                  "+r"(r[30]), "+r"(r[31])
                :
                : "memory");
+}
+// ---- CTA pairs (cta_group::2): two CTAs of a cluster on the two SMs of a TPC share one MMA of 256 rows.  Each CTA
+// stages its 128 rows of A and its half of the columns of B; the even CTA (the leader) issues the MMAs for both, and
+// each CTA's TMEM receives the accumulator of its own 128 rows.
+__device__ __forceinline__ uint32_t ClusterCtaRank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void ClusterSync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Tile load into this CTA's shared memory whose bytes are counted on the leader's copy of the barrier: clearing bit 24
+// of a shared::cluster address selects the even CTA of the pair.
+__device__ __forceinline__ void TmaLoad2DPair(void* smem_dst, const CUtensorMap* tmap, int x, int y, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(SmemAddr(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y),
+      "r"(SmemAddr(bar) & 0xFEFFFFFFu)
+      : "memory");
+}
+__device__ __forceinline__ void UmmaBf16Pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+      : "memory");
+}
+// Arrives on the barrier at this offset in both CTAs once the pair's MMAs issued so far have completed.
+__device__ __forceinline__ void UmmaCommitPair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          SmemAddr(bar)),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+// Arrival on the leader's copy of a barrier, from either CTA of the pair.
+__device__ __forceinline__ void MbarArriveLeader(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(SmemAddr(bar))
+      : "memory");
 }
 __device__ __forceinline__ void NamedBarSync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");

@@ -214,6 +214,13 @@ int tipsk_gemm_bf16(const void* a, const void* b, void* c, const void* bias, voi
 /* C[m,n] = A[m,k] * B[k,n] with B row-major [k, n] (contraction over its rows), n >= 64. */
 int tipsk_gemm_bf16_nn(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc,
                        int accumulate, void* stream);
+int tipsk_gemm_prefers_pair(int kind, int m, int n, int k);
+int tipsk_gemm_splits(int m, int n, int k);
+int tipsk_gemm_bf16_split(int kind, const void* a, const void* b, void* c, const void* bias, void* pre, float* partial,
+                          int splits, int m, int n, int k, int lda, int ldb, int ldc, int act, int accumulate,
+                          void* stream);
+int tipsk_gemm_bf16_tt(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc,
+                       void* stream);
 int tipsk_gemm_status(void);
 
 /* ---- 3x3 / stride 2 / pad 1 max pooling on NHWC (pool.cu); idx holds the argmax position 0..8 per output ---- */

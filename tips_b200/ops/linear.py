@@ -6,9 +6,9 @@ and activation fused into the epilogue.  ``Linear`` builds forward and backward 
     y  = act(x W^T + b)                      gemm_tn(x, W)
     dz = dy * act'(.) ; db = colsum(dz)      one pass (bias_act_bwd kernel)
     dx = dz W                                gemm_nn(dz, W): W is read in place as an MN-major operand
-    dW = dz^T x                              the split-K weight-gradient kernel of conv_tcgen05.cu, which reads dz and x
-                                             as they are (both operands MN-major); transposed copies of the
-                                             activations only for feature counts that are not multiples of 64
+    dW = dz^T x                              the same GEMM with both operands MN-major (dz and x as they are); transposed
+                                             copies only for feature counts that are not multiples of 64; fp32
+                                             gradients come from the weight-gradient kernel of conv_tcgen05.cu
 
 The reference has no GEMM or linear layer; this serves the CTR MLP and the BERT-shaped encoder.
 CPU tensors (host-only tests) and shapes the kernel does not take (row strides that are not a
@@ -33,6 +33,21 @@ def _supported(a: torch.Tensor, b: torch.Tensor) -> bool:
             and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0)
 
 
+def _split(kind, a, b, c, bias, pre, m, n, k, act, accumulate) -> bool:
+    """Run the product with its contraction split over idle SMs when it has few output tiles and a long K; False when
+    the unsplit kernels are to take it.  The fp32 partial products live in a workspace of this call."""
+    lib = base.K()
+    splits = lib.tipsk_gemm_splits(m, n, k)
+    if splits <= 1:
+        return False
+    partial = torch.empty(splits * m * n, dtype=torch.float32, device=c.device)
+    base.check(lib.tipsk_gemm_bf16_split(kind, a.data_ptr(), b.data_ptr(), c.data_ptr(), base.ptr(bias), base.ptr(pre),
+                                         partial.data_ptr(), splits, m, n, k, a.stride(0), b.stride(0), n, act,
+                                         int(accumulate), base.stream()), "gemm_bf16_split")
+    base.count_launches(1)
+    return True
+
+
 def gemm_tn(a, b, bias=None, act=None, want_pre=False):
     """act(a @ b.T + bias). Returns y, or (y, pre_activation) when want_pre."""
     code = _ACT[act]
@@ -49,6 +64,8 @@ def gemm_tn(a, b, bias=None, act=None, want_pre=False):
     c = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     pre = torch.empty_like(c) if want_pre else None
     bb = None if bias is None else bias.to(torch.bfloat16).contiguous()
+    if _split(0, a, b, c, bb, pre, m, n, k, code, False):
+        return (c, pre) if want_pre else c
     base.check(base.K().tipsk_gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), base.ptr(bb), base.ptr(pre), m, n, k,
                                         a.stride(0), b.stride(0), n, code, base.stream()), "gemm_bf16")
     return (c, pre) if want_pre else c
@@ -68,19 +85,28 @@ def gemm_nn(a: torch.Tensor, b: torch.Tensor, into: torch.Tensor | None = None) 
         c = into
     else:
         c = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
+    if _split(1, a, b, c, None, None, m, n, k, 0, into is not None):
+        return c
     base.check(base.K().tipsk_gemm_bf16_nn(a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, a.stride(0), b.stride(0),
                                            n, 0 if into is None else 1, base.stream()), "gemm_bf16_nn")
     return c
 
 
-def _weight_grad(dz: torch.Tensor, x2: torch.Tensor) -> torch.Tensor:
-    """dz^T @ x2 as [N, K].  A linear layer is a 1x1 convolution over "pixels" = rows, so the convolution's
-    weight-gradient kernel applies: it contracts over the rows with both operands read in place."""
+def _weight_grad(dz: torch.Tensor, x2: torch.Tensor, dtype: torch.dtype | None = None) -> torch.Tensor:
+    """dz^T @ x2 as [N, K], in fp32 or, with dtype=torch.bfloat16, rounded once from the fp32 accumulators.  Both
+    operands are read in place (MN-major)."""
     m, n = dz.shape
     k = x2.shape[1]
     if (dz.is_cuda and dz.dtype == torch.bfloat16 and x2.dtype == torch.bfloat16 and n % 64 == 0 and k % 64 == 0
             and m >= 16 and dz.is_contiguous() and x2.is_contiguous()
             and dz.data_ptr() % 16 == 0 and x2.data_ptr() % 16 == 0):
+        if dtype == torch.bfloat16 and base.K().tipsk_gemm_prefers_pair(2, n, k, m):
+            dw = torch.empty(n, k, dtype=torch.bfloat16, device=dz.device)
+            if not _split(2, dz, x2, dw, None, None, n, k, m, 0, False):
+                base.check(base.K().tipsk_gemm_bf16_tt(dz.data_ptr(), x2.data_ptr(), dw.data_ptr(), n, k, m, n, k, k,
+                                                       base.stream()), "gemm_bf16_tt")
+            return dw
+        # the convolution's weight-gradient kernel (a linear layer is a 1x1 convolution over "pixels" = rows)
         dw = torch.empty(n, k, dtype=torch.float32, device=dz.device)
         base.check(base.K().tipsk_conv2d_wgrad(x2.data_ptr(), dz.data_ptr(), dw.data_ptr(), 1, 1, m, k, n, 1, 1, 1, 0,
                                                base.stream()), "linear_wgrad")
@@ -157,7 +183,7 @@ def _linear_backward(ctx, dy, d_alias):
                 into = into.contiguous()
         dx = gemm_nn(dz, weight, into=into).view(ctx.in_shape)
     if ctx.needs_input_grad[1]:
-        dw = _weight_grad(dz, x2).to(weight.dtype)
+        dw = _weight_grad(dz, x2, weight.dtype).to(weight.dtype)
     return dx, dw, dbias, None
 
 
