@@ -116,3 +116,46 @@ def test_pack_many_tensors(src, flat, accumulate):
                                      base.i64_array(numels), len(back), base.code(src), 2.0, base.stream()), "unpack")
     for t, o in zip(back, offs):
         assert torch.equal(t, (buf[o:o + t.numel()].float() * 2.0).to(src))
+
+
+@pytest.mark.parametrize("dtype", [BF16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 4096), (5, 4104), (700, 1000), (4, 30522), (3, 32768), (3, 32776)])
+def test_softmax_cross_entropy_rows(dtype, rows, cols):
+    from tips_b200.ops.pointwise import softmax_cross_entropy
+    z = _rand(rows, cols, scale=3.0, dtype=dtype).requires_grad_()
+    labels = torch.randint(0, cols, (rows,), device=DEV, generator=torch.Generator(device=DEV).manual_seed(1))
+    if rows > 2:
+        labels[1] = -100
+    labels[0] = cols - 1
+    loss = softmax_cross_entropy(z, labels)
+    (loss * 3.0).backward()
+    zr = z.detach().double().requires_grad_()
+    ref = F.cross_entropy(zr, labels, ignore_index=-100)
+    (ref * 3.0).backward()
+    assert torch.allclose(loss.double(), ref.detach(), rtol=1e-5)
+    # rounded once as the gradient of the mean, once after the factor 3: twice 2^-8, their product, and fp32 terms
+    _close(z.grad, zr.grad, slack=2.0 ** -18, rel=2.0 ** -7 + 2.0 ** -13)
+
+
+def test_softmax_cross_entropy_without_counted_rows():
+    from tips_b200.ops.pointwise import softmax_cross_entropy
+    z = _rand(4, 64).requires_grad_()
+    loss = softmax_cross_entropy(z, torch.full((4,), -100, device=DEV))
+    loss.backward()
+    assert float(loss.detach()) == 0.0 and not bool(z.grad.any())
+
+
+@pytest.mark.parametrize("dtype", [BF16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (31, 264), (33, 1000), (4097, 72)])
+@pytest.mark.parametrize("act", [None, "relu", "gelu"])
+def test_bias_act_backward_rows(dtype, rows, cols, act):
+    from tips_b200.ops.pointwise import bias_act
+    x, b = _rand(rows, cols, dtype=dtype, scale=2.0).requires_grad_(), _rand(cols, dtype=dtype, seed=1).requires_grad_()
+    dy = _rand(rows, cols, dtype=dtype, seed=2)
+    bias_act(x, b, act).backward(dy)
+    xr, br = x.detach().double().requires_grad_(), b.detach().double().requires_grad_()
+    y = xr + br
+    y = F.relu(y) if act == "relu" else F.gelu(y) if act == "gelu" else y
+    y.backward(dy.double())
+    _close(x.grad, xr.grad)
+    _close(b.grad, br.grad)

@@ -19,8 +19,9 @@ __device__ __forceinline__ float ActGrad(float v, int act) {
   if (act == 1) return v > 0.f ? 1.f : 0.f;
   if (act == 2) {
     // d/dv [v * Phi(v)] = Phi(v) + v * phi(v).  Phi through erf(z), z = v / sqrt(2), with the rational approximation
-    // erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z) (absolute error < 1.5e-7): exp(-z^2) is the
-    // same exponential the density phi(v) needs, so the whole derivative costs one exp and one reciprocal.
+    // (Abramowitz and Stegun, 7.1.26) erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z) (absolute error
+    // < 1.5e-7): exp(-z^2) is the same exponential the density phi(v) needs, so the whole derivative costs one exp and
+    // one reciprocal.
     const float e  = __expf(-0.5f * v * v);
     const float z  = fabsf(v) * 0.70710678118654752f;
     const float t  = __frcp_rn(1.f + 0.3275911f * z);
@@ -55,11 +56,13 @@ BiasActFwdKernel(const T* __restrict__ x, const T* __restrict__ bias, T* __restr
   }
 }
 
-// block (32, 8): tx -> vector column, ty -> row lane; grid (col tiles, row partitions)
-template <typename T>
-__global__ void __launch_bounds__(256)
+// block (32, 8): tx -> vector column, ty -> row lane; grid (col tiles, row partitions).  Bound by HBM, and with GELU by the
+// instructions of its derivative, hence two values per instruction there; three or four rows in flight per thread.
+// 16384 x 4096 bf16: GELU (400 MB) 135 -> 85 us; bias gradient alone, 1232 x 30528 (75 MB) 39 -> 19 us.
+template <typename T, int kAct>
+__global__ void __launch_bounds__(256, kAct == 2 ? 2 : 3)
 BiasActBwdKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ bias, T* __restrict__ dx,
-                 float* __restrict__ dbias, int64_t rows, int cols, int act) {
+                 float* __restrict__ dbias, int64_t rows, int cols) {
   constexpr int N = 16 / sizeof(T);
   __shared__ float red[8][32][N + 1];
   const int vec_cols = cols / N;
@@ -78,27 +81,38 @@ BiasActBwdKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __r
       for (int k = 0; k < N; ++k) bv[k] = 0.f;
     }
     const int64_t step = static_cast<int64_t>(gridDim.y) * 8;
-    for (int64_t r = static_cast<int64_t>(blockIdx.y) * 8 + threadIdx.y; r < rows; r += 2 * step) {
-      // two rows in flight per thread
-      const int64_t off[2] = {r * cols + static_cast<int64_t>(vc) * N, (r + step) * cols + static_cast<int64_t>(vc) * N};
-      const bool have[2]   = {true, r + step < rows};
-      Vec16<T> d[2], q[2];
+    constexpr int U = kAct == 0 ? 4 : 3;  // rows in flight per thread
+    for (int64_t r = static_cast<int64_t>(blockIdx.y) * 8 + threadIdx.y; r < rows; r += U * step) {
+      Vec16<T> d[U], q[U];
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
-        if (have[u]) {
-          d[u] = LoadVec(dy + off[u]);
-          if (act != 0) q[u] = LoadVec(x + off[u]);
+      for (int u = 0; u < U; ++u)
+        if (r + u * step < rows) {
+          const int64_t off = (r + u * step) * cols + static_cast<int64_t>(vc) * N;
+          d[u] = LoadVec(dy + off);
+          if (kAct != 0) q[u] = LoadVec(x + off);
         }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (!have[u]) continue;
+      for (int u = 0; u < U; ++u) {
+        if (r + u * step >= rows) continue;
         Vec16<T> o;
-        if (act != 0) {
+        if (kAct != 0) {
+          if constexpr (kAct == 2 && sizeof(T) == 2) {  // two values per instruction
 #pragma unroll
-          for (int k = 0; k < N; ++k) {
-            const float g = ToFloat<T>(d[u].v[k]) * ActGrad(ToFloat<T>(q[u].v[k]) + bv[k], act);
-            acc[k] += g;
-            o.v[k] = FromFloat<T>(g);
+            for (int k = 0; k < N; k += 2) {
+              const F2 v = MakeF2(ToFloat<T>(q[u].v[k]) + bv[k], ToFloat<T>(q[u].v[k + 1]) + bv[k + 1]);
+              const float2 g = SplitF2(Mul2(MakeF2(ToFloat<T>(d[u].v[k]), ToFloat<T>(d[u].v[k + 1])), GeluGrad2(v)));
+              acc[k] += g.x;
+              acc[k + 1] += g.y;
+              o.v[k]     = FromFloat<T>(g.x);
+              o.v[k + 1] = FromFloat<T>(g.y);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+              const float g = ToFloat<T>(d[u].v[k]) * ActGrad(ToFloat<T>(q[u].v[k]) + bv[k], kAct);
+              acc[k] += g;
+              o.v[k] = FromFloat<T>(g);
+            }
           }
         } else {
 #pragma unroll
@@ -107,7 +121,7 @@ BiasActBwdKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __r
             o.v[k] = d[u].v[k];
           }
         }
-        if (dx) StoreVec(dx + off[u], o);
+        if (dx) StoreVec(dx + (r + u * step) * cols + static_cast<int64_t>(vc) * N, o);
       }
     }
   }
@@ -350,12 +364,33 @@ __device__ __forceinline__ float BlockReduce(float v, bool is_max, float* scratc
   return r;
 }
 
+// What a row's loss and gradient are multiplied with: `scale`, or with `mean` one over the rows that count (every block
+// counts the labels itself, a few kilobytes from L2, so that the gradient is written finished in the same pass).
+__device__ __forceinline__ float XentScale(const int64_t* __restrict__ labels, int64_t rows, int cols,
+                                           int64_t ignore_index, float scale, int mean) {
+  if (!mean) return scale;
+  __shared__ int total;
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
+  int mine = 0;
+  for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) {
+    const int64_t l = labels[r];
+    mine += !(l == ignore_index || l < 0 || l >= cols);
+  }
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&total, mine);
+  __syncthreads();
+  return 1.f / static_cast<float>(total > 1 ? total : 1);
+}
+
+// General form: any row length and alignment.
 template <typename T>
 __global__ void __launch_bounds__(256)
 SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ loss_sum,
                   float* __restrict__ count, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index,
-                  float scale) {
+                  float grad_scale, int mean) {
   __shared__ float scratch[8];
+  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean);
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const T* row        = logits + r * cols;
     const int64_t label = labels[r];
@@ -373,7 +408,8 @@ SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labe
     se = BlockReduce(se, false, scratch);
     const float lse = mx + logf(se);
     if (threadIdx.x == 0) {
-      atomicAdd(loss_sum, lse - ToFloat<T>(row[label]));
+      const float loss = lse - ToFloat<T>(row[label]);
+      atomicAdd(loss_sum, mean ? loss * scale : loss);
       if (count) atomicAdd(count, 1.f);
     }
     if (dlogits) {
@@ -385,6 +421,132 @@ SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labe
       }
     }
   }
+}
+
+// Rows of whole 16-byte vectors, up to 512 * VPT of them: one block of 512 threads per row, which it reads from HBM once
+// into VPT vectors per thread and keeps for all three sweeps (maximum, sum of exponentials, gradient).  Bound by HBM
+// (one read, one write) and, close behind, by two exponentials per logit.  1232 x 30528 bf16 (150 MB): 46 us; the general
+// form, which reads scalars from L2 in each sweep, 221 us.
+constexpr int kXentThreads = 512;
+
+__device__ __forceinline__ float XentReduce(float v, bool is_max, float* scratch) {
+  v = is_max ? WarpMax(v) : WarpSum(v);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float o = scratch[0];
+#pragma unroll
+  for (int w = 1; w < kXentThreads / 32; ++w) o = is_max ? fmaxf(o, scratch[w]) : o + scratch[w];
+  return o;  // the caller alternates between two scratch arrays, so no second barrier is needed
+}
+
+// Makes the compiler forget what it knows about the vectors, so that it keeps them packed between the sweeps instead of
+// as twice as many fp32 registers (which spill at 64 registers per thread).
+template <typename T, int VPT>
+__device__ __forceinline__ void KeepPacked(Vec16<T> (&v)[VPT]) {
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    uint4& q = *reinterpret_cast<uint4*>(&v[k]);
+    asm volatile("" : "+r"(q.x), "+r"(q.y), "+r"(q.z), "+r"(q.w));
+  }
+}
+
+template <typename T, int VPT>
+__global__ void __launch_bounds__(kXentThreads, 2)
+SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ loss_sum,
+                     float* __restrict__ count, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index,
+                     float grad_scale, int mean) {
+  constexpr int N = 16 / sizeof(T);
+  __shared__ float smax[kXentThreads / 32], ssum[kXentThreads / 32];
+  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean);
+  const int nvec    = cols / N;
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+    const T* row        = logits + r * cols;
+    T* drow             = dlogits ? dlogits + r * cols : nullptr;
+    const int64_t label = labels[r];
+    if (label == ignore_index || label < 0 || label >= cols) {
+      if (drow) {
+        Vec16<T> z;
+#pragma unroll
+        for (int j = 0; j < N; ++j) z.v[j] = FromFloat<T>(0.f);
+        for (int i = threadIdx.x; i < nvec; i += kXentThreads) StoreVec(drow + i * N, z);
+      }
+      continue;
+    }
+    Vec16<T> v[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = k * kXentThreads + threadIdx.x;
+      if (i < nvec) v[k] = LoadVec(row + i * N);
+      else *reinterpret_cast<uint4*>(&v[k]) = make_uint4(0, 0, 0, 0);
+    }
+    float mx = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (k * kXentThreads + threadIdx.x < nvec) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) mx = fmaxf(mx, ToFloat<T>(v[k].v[j]));
+      }
+    mx = XentReduce(mx, true, smax);
+    KeepPacked(v);
+    float se = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (k * kXentThreads + threadIdx.x < nvec) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) se += __expf(ToFloat<T>(v[k].v[j]) - mx);
+      }
+    se = XentReduce(se, false, ssum);
+    KeepPacked(v);
+    if (threadIdx.x == 0) {
+      const float loss = mx + logf(se) - ToFloat<T>(row[label]);
+      atomicAdd(loss_sum, mean ? loss * scale : loss);
+      if (count) atomicAdd(count, 1.f);
+    }
+    if (drow) {
+      const float inv = 1.f / se;
+      const int lvec = static_cast<int>(label) / N, lj = static_cast<int>(label) % N;
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const int i = k * kXentThreads + threadIdx.x;
+        if (i < nvec) {
+          Vec16<T> o;
+#pragma unroll
+          for (int j = 0; j < N; ++j) {
+            float p = __expf(ToFloat<T>(v[k].v[j]) - mx) * inv;
+            if (i == lvec && j == lj) p -= 1.f;
+            o.v[j] = FromFloat<T>(p * scale);
+          }
+          StoreVec(drow + i * N, o);
+        }
+      }
+    }
+    // a thread may only reach the next row's first write of smax after every thread has read it: the barrier inside
+    // the sum's reduction lies between
+  }
+}
+
+// y = x * s for a scalar s on the device: 37.6 M bf16 values (150 MB) 25 us, 6 TB/s.
+template <typename T>
+__global__ void __launch_bounds__(256)
+ScaleByKernel(const T* __restrict__ x, const float* __restrict__ s, T* __restrict__ y, int64_t n) {
+  constexpr int N = 16 / sizeof(T), U = 4;
+  const float f = *s;
+  const int64_t vecs = n / N, stride = static_cast<int64_t>(gridDim.x) * 256;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < vecs; i += U * stride) {
+    Vec16<T> v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * stride < vecs) v[u] = LoadVec(x + (i + u * stride) * N);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * stride < vecs) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[u].v[j] = FromFloat<T>(ToFloat<T>(v[u].v[j]) * f);
+        StoreVec(y + (i + u * stride) * N, v[u]);
+      }
+  }
+  if (blockIdx.x == 0)
+    for (int64_t i = vecs * N + threadIdx.x; i < n; i += 256) y[i] = FromFloat<T>(ToFloat<T>(x[i]) * f);
 }
 
 }  // namespace
@@ -433,8 +595,9 @@ int tipsk_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx
   if (parts < 1) parts = 1;
   dim3 grid(col_tiles, parts), block(32, 8);
   EPI_DISPATCH(dtype, {
-    BiasActBwdKernel<T><<<grid, block, 0, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x),
-                                               static_cast<const T*>(bias), static_cast<T*>(dx), dbias, rows, cols, act);
+    auto* kernel = act == 0 ? BiasActBwdKernel<T, 0> : act == 1 ? BiasActBwdKernel<T, 1> : BiasActBwdKernel<T, 2>;
+    kernel<<<grid, block, 0, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x), static_cast<const T*>(bias),
+                                  static_cast<T*>(dx), dbias, rows, cols);
   });
   TIPSK_LAUNCH_CHECK();
   return 0;
@@ -537,14 +700,62 @@ int tipsk_embed_sum_bwd(const int64_t* ids, const void* dx, void* dtok, void* dp
   return 0;
 }
 
-int tipsk_softmax_xent(const void* logits, const int64_t* labels, float* loss_sum, float* count, void* dlogits,
-                       int64_t rows, int cols, int64_t ignore_index, float grad_scale, int dtype, void* stream) {
+static int SoftmaxXentImpl(const void* logits, const int64_t* labels, float* loss_sum, float* count, void* dlogits,
+                           int64_t rows, int cols, int64_t ignore_index, float grad_scale, int mean, int dtype,
+                           void* stream) {
   if (rows <= 0 || cols <= 0) return 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int grid = rows < NumSMs() * 8 ? static_cast<int>(rows) : NumSMs() * 8;
+  // The row kernel needs whole, aligned 16-byte vectors and at most eight of them per thread (it is the faster one
+  // wherever it applies: see the kernel).
+  const int n        = 16 / static_cast<int>(DTypeSize(dtype));
+  const bool aligned = cols % n == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0 &&
+                       reinterpret_cast<uintptr_t>(dlogits) % 16 == 0;
+  const int per_thread = CeilDiv(cols / n, kXentThreads);
+  if (aligned && per_thread <= 8) {
+    const int grid = static_cast<int>(rows < NumSMs() * 2 ? rows : NumSMs() * 2);
+    EPI_DISPATCH(dtype, {
+      auto* kernel = per_thread <= 1   ? SoftmaxXentRowKernel<T, 1>
+                     : per_thread <= 2 ? SoftmaxXentRowKernel<T, 2>
+                     : per_thread <= 4 ? SoftmaxXentRowKernel<T, 4>
+                                       : SoftmaxXentRowKernel<T, 8>;
+      kernel<<<grid, kXentThreads, 0, s>>>(static_cast<const T*>(logits), labels, loss_sum, count,
+                                           static_cast<T*>(dlogits), rows, cols, ignore_index, grad_scale, mean);
+    });
+    TIPSK_LAUNCH_CHECK();
+    return 0;
+  }
+  const int grid = static_cast<int>(rows < NumSMs() * 8 ? rows : NumSMs() * 8);
   EPI_DISPATCH(dtype, {
     SoftmaxXentKernel<T><<<grid, 256, 0, s>>>(static_cast<const T*>(logits), labels, loss_sum, count,
-                                              static_cast<T*>(dlogits), rows, cols, ignore_index, grad_scale);
+                                              static_cast<T*>(dlogits), rows, cols, ignore_index, grad_scale, mean);
+  });
+  TIPSK_LAUNCH_CHECK();
+  return 0;
+}
+
+int tipsk_softmax_xent(const void* logits, const int64_t* labels, float* loss_sum, float* count, void* dlogits,
+                       int64_t rows, int cols, int64_t ignore_index, float grad_scale, int dtype, void* stream) {
+  return SoftmaxXentImpl(logits, labels, loss_sum, count, dlogits, rows, cols, ignore_index, grad_scale, 0, dtype, stream);
+}
+
+/* Mean over the rows whose label counts: *loss (zeroed by the caller) receives the mean loss, dlogits its gradient. */
+int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, void* dlogits, int64_t rows, int cols,
+                            int64_t ignore_index, int dtype, void* stream) {
+  return SoftmaxXentImpl(logits, labels, loss, nullptr, dlogits, rows, cols, ignore_index, 1.f, 1, dtype, stream);
+}
+
+/* y = x * s, s one fp32 value on the device. */
+int tipsk_scale_by(const void* x, const float* s, void* y, int64_t n, int dtype, void* stream) {
+  if (n <= 0) return 0;
+  TIPSK_REQUIRE(reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0,
+                "scale_by: 16-byte aligned buffers are required");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int64_t vecs = n / (16 / static_cast<int64_t>(DTypeSize(dtype)));
+  int64_t grid = (vecs + 256 * 4 - 1) / (256 * 4);
+  if (grid > NumSMs() * 8) grid = NumSMs() * 8;
+  if (grid < 1) grid = 1;
+  EPI_DISPATCH(dtype, {
+    ScaleByKernel<T><<<static_cast<int>(grid), 256, 0, st>>>(static_cast<const T*>(x), s, static_cast<T*>(y), n);
   });
   TIPSK_LAUNCH_CHECK();
   return 0;

@@ -181,19 +181,23 @@ class _SoftmaxXentFn(torch.autograd.Function):
         z = logits.contiguous()
         rows = z.numel() // cols
         lab = labels.contiguous().view(-1)
-        acc = torch.zeros(2, dtype=torch.float32, device=z.device)
+        loss = torch.zeros((), dtype=torch.float32, device=z.device)
         dz = torch.empty_like(z)
-        base.check(base.K().tipsk_softmax_xent(z.data_ptr(), lab.data_ptr(), acc.data_ptr(),
-                                               acc.data_ptr() + 4, dz.data_ptr(), rows, cols, ignore_index, 1.0,
-                                               base.code(z), base.stream()), "softmax_xent")
-        inv = 1.0 / torch.clamp(acc[1], min=1.0)
-        ctx.save_for_backward(dz, inv)
-        return acc[0] * inv
+        base.check(base.K().tipsk_softmax_xent_mean(z.data_ptr(), lab.data_ptr(), loss.data_ptr(), dz.data_ptr(), rows,
+                                                    cols, ignore_index, base.code(z), base.stream()), "softmax_xent")
+        ctx.save_for_backward(dz)  # the gradient of the mean loss
+        return loss
 
     @staticmethod
     def backward(ctx, dloss):
-        dz, inv = ctx.saved_tensors
-        return dz * (dloss * inv).to(dz.dtype), None, None
+        (dz,) = ctx.saved_tensors
+        if torch.is_grad_enabled() or not base.plain(dloss):  # create_graph, or gradients batched by vmap
+            return dz * dloss.to(dz.dtype), None, None
+        up = dloss.to(torch.float32)
+        out = torch.empty_like(dz)
+        base.check(base.K().tipsk_scale_by(dz.data_ptr(), up.data_ptr(), out.data_ptr(), dz.numel(), base.code(dz),
+                                           base.stream()), "scale_by")
+        return out, None, None
 
 
 def softmax_cross_entropy(logits, labels, ignore_index=-100):
