@@ -159,3 +159,16 @@ def test_bias_act_backward_rows(dtype, rows, cols, act):
     y.backward(dy.double())
     _close(x.grad, xr.grad)
     _close(b.grad, br.grad)
+
+
+@pytest.mark.parametrize("dtype", [BF16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(1, 256), (14, 256), (2221, 256), (8, 1024), (1185, 1024), (1200, 768), (301, 2048)])
+def test_layer_norm_backward_groups(dtype, rows, cols):
+    from tips_b200.ops.norm import layer_norm
+    x, dy = _rand(rows, cols, dtype=dtype).requires_grad_(), _rand(rows, cols, dtype=dtype, seed=1)
+    w, b = (1 + _rand(cols, dtype=dtype, scale=0.1, seed=2)).requires_grad_(), _rand(cols, dtype=dtype, seed=3).requires_grad_()
+    layer_norm(x, w, b).backward(dy)
+    xr, wr, br = (t.detach().double().requires_grad_() for t in (x, w, b))
+    F.layer_norm(xr, (cols,), wr, br).backward(dy.double())
+    for got, ref in ((x.grad, xr.grad), (w.grad, wr.grad), (b.grad, br.grad)):
+        _close(got, ref)

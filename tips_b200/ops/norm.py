@@ -188,16 +188,17 @@ class _LayerNormFn(torch.autograd.Function):
         dyc = dy.contiguous()
         dx = torch.empty_like(x)
         lib = base.K()
-        parts = lib.tipsk_ln_bwd_partials(rows, cols)
+        parts = lib.tipsk_ln_bwd_partial_rows(rows, cols, base.code(x))
         pg = torch.empty(parts, cols, dtype=torch.float32, device=x.device)
         pb = torch.empty(parts, cols, dtype=torch.float32, device=x.device)
         base.check(lib.tipsk_ln_bwd(dyc.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                                     dx.data_ptr(), pg.data_ptr(), pb.data_ptr(), parts, rows, cols, base.code(x),
                                     base.stream()), "ln_bwd")
-        dgamma = torch.empty(cols, dtype=torch.float32, device=x.device)
-        dbeta = torch.empty(cols, dtype=torch.float32, device=x.device)
+        out_dtype = ctx.wdtype if ctx.wdtype in (torch.bfloat16, torch.float16) else torch.float32
+        dgamma = torch.empty(cols, dtype=out_dtype, device=x.device)
+        dbeta = torch.empty(cols, dtype=out_dtype, device=x.device)
         base.check(lib.tipsk_ln_reduce_partials(pg.data_ptr(), pb.data_ptr(), parts, cols, dgamma.data_ptr(),
-                                                dbeta.data_ptr(), 0, base.stream()), "ln_reduce")
+                                                dbeta.data_ptr(), base.code(dgamma), base.stream()), "ln_reduce")
         return dx, dgamma.to(ctx.wdtype), dbeta.to(ctx.wdtype), None, (dx if ctx.has_res else None)
 
 
