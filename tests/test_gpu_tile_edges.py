@@ -78,6 +78,40 @@ def test_split_contraction(m, n, k):
     assert gemm_status() == 0
 
 
+# n, h, w, cin, cout: widths at both ends of the halo kernel's range, image heights that leave a short last unit, an odd
+# number of units, weights resident (64 -> 64) and streamed
+HALO = [(300, 2, 62, 64, 64), (43, 56, 56, 64, 64), (149, 28, 28, 128, 128), (75, 17, 28, 64, 192), (40, 31, 33, 128, 64),
+        (297, 9, 9, 64, 128), (601, 5, 24, 192, 64)]
+
+
+@pytest.mark.parametrize("n,h,w,cin,cout", HALO)
+def test_conv3x3(n, h, w, cin, cout):
+    from tips_b200.ops.conv import conv2d_dgrad, conv2d_forward, conv2d_wgrad
+    from tips_b200.ops import base
+    x = _rand(n, cin, h, w).contiguous(memory_format=torch.channels_last)
+    wgt = _rand(cout, 3, 3, cin, scale=1.0 / (3 * cin ** 0.5), seed=1)
+    dy = _rand(n, cout, h, w, seed=2).contiguous(memory_format=torch.channels_last)
+    stats = torch.zeros(2, cout, device=DEV)
+    _, y = conv2d_forward(x, wgt, 1, 1, stats)
+    xr, wr = x.float().requires_grad_(), wgt.float().permute(0, 3, 1, 2).contiguous().requires_grad_()
+    torch.backends.cudnn.allow_tf32, before = False, torch.backends.cudnn.allow_tf32
+    try:
+        ref = F.conv2d(xr, wr, padding=1)
+        ref.backward(dy.float())
+    finally:
+        torch.backends.cudnn.allow_tf32 = before
+    _close(y, ref.detach())
+    yf = y.double()
+    assert torch.allclose(stats[0].double(), yf.sum((0, 2, 3)), rtol=1e-4, atol=1e-3 * float(yf.abs().sum((0, 2, 3)).max()))
+    assert torch.allclose(stats[1].double(), (yf * yf).sum((0, 2, 3)), rtol=1e-4)
+    _close(conv2d_dgrad(dy, wgt, tuple(x.shape), 1, 1), xr.grad)
+    into = _rand(n, cin, h, w, seed=4).contiguous(memory_format=torch.channels_last)
+    want = into.double() + xr.grad.double()
+    _close(conv2d_dgrad(dy, wgt, tuple(x.shape), 1, 1, into=into), want, slack=2.0 ** -8)
+    _close(conv2d_wgrad(x, dy, (cout, 3, 3, cin), 1, 1), wr.grad.permute(0, 2, 3, 1))
+    assert base.K().tipsk_conv_status() == 0
+
+
 @pytest.mark.parametrize("n,c,h,w", [(1, 8, 1, 1), (2, 8, 2, 3), (3, 72, 5, 8), (2, 64, 31, 33), (1, 2056, 4, 4)])
 def test_maxpool_edges(n, c, h, w):
     from tips_b200.ops.pool import max_pool_3x3_s2

@@ -152,7 +152,7 @@ ConvTapsKernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ElectOne()) {
       uint32_t it = 0;
       bool ok = true;
       if (b_res) {
@@ -197,7 +197,7 @@ ConvTapsKernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {  // the whole warp walks the loop, one lane issues
       // bit 16: B is MN-major (the weights in the layout the forward pass uses, contracted over their rows)
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (p.b_mn ? (1u << 16) : 0u) |
                              (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
@@ -205,22 +205,22 @@ ConvTapsKernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
       uint32_t it = 0;
       int local = 0;
       bool ok = true;
-      if (b_res && !MbarWait(b_full, 0)) {
-        atomicExch(p.error, 5);
+      if (b_res && !MbarWaitWarp(b_full, 0)) {
+        if (lane == 0) atomicExch(p.error, 5);
         ok = false;
       }
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
         const int buf = local & 1;
-        if (!MbarWait(&tmem_empty[buf], ((local >> 1) & 1) ^ 1)) {
-          atomicExch(p.error, 4);
+        if (!MbarWaitWarp(&tmem_empty[buf], ((local >> 1) & 1) ^ 1)) {
+          if (lane == 0) atomicExch(p.error, 4);
           break;
         }
         TcFenceAfter();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * BN);
         for (int kt = 0; kt < num_k; ++kt, ++it) {
           const int s = it % Cfg::kStages;
-          if (!MbarWait(&full_bar[s], (it / Cfg::kStages) & 1)) {
-            atomicExch(p.error, 2);
+          if (!MbarWaitWarp(&full_bar[s], (it / Cfg::kStages) & 1)) {
+            if (lane == 0) atomicExch(p.error, 2);
             ok = false;
             break;
           }
@@ -229,12 +229,14 @@ ConvTapsKernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
           const uint64_t adesc  = SmemDescSw128(a_addr);
           const uint32_t b_addr = b_res ? SmemAddr(resident) + kt * Cfg::kBBytes : a_addr + Cfg::kABytes;
           const uint64_t bdesc  = p.b_mn ? SmemDescMnSw128(b_addr, 8192) : SmemDescSw128(b_addr);
+          if (ElectOne()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            UmmaBf16(tmem_d, adesc + 2 * k, bdesc + b_kstep * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
-          UmmaCommit(&empty_bar[s]);
+            for (int k = 0; k < kBK / 16; ++k)
+              UmmaBf16(tmem_d, adesc + 2 * k, bdesc + b_kstep * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            UmmaCommit(&empty_bar[s]);
+          }
         }
-        if (ok) UmmaCommit(&tmem_full[buf]);
+        if (ok && ElectOne()) UmmaCommit(&tmem_full[buf]);
       }
     }
   } else if (warp < 6) {
@@ -381,6 +383,323 @@ ConvTapsKernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   }
 }
 
+// ------------------------------------------------------------------ 3x3, stride 1: one halo box for all nine taps
+// With few channels the tap kernel above is bound by its loads: it fetches the same box of pixels nine times, 16 KB for
+// 128 x 64 x 64 products.  Here a unit of `th` full image rows is loaded once per 64-channel block together with its
+// border, [th + 2] rows x [w + 2] pixels (zero fill outside the image), and the nine taps read it at nine offsets: pixel
+// (h, w) of the unit is row h * pitch + w of the box, pitch = w + 2, so a tap is a shift by whole 128-byte rows and the
+// MMA's A operand starts (dh + 1) * pitch + dw + 1 rows further.  The swizzle is a function of the shared-memory address,
+// so a shifted start needs no other descriptor.  Rows w .. pitch - 1 of every image row are computed and dropped
+// (112 of 128 rows are real pixels at 56 x 56 and 28 x 28).  A tile is two units that share every weight block.  Bound by
+// the rate of 64-column MMAs.  64 -> 64 channels, 256 images of 56 x 56: 111 us forward and data gradient, 157 with a box per
+// tap (59 GFLOP).
+struct HaloParams {
+  int32_t* error;
+  float* stat_sum;
+  float* stat_sq;
+  int cblocks, accumulate, b_mn;
+  int b_slots, b_resident;       // weight blocks in shared memory; 1: all 9 * cblocks of them stay for the whole kernel
+  int pitch, th, w, ho;          // box pitch in pixels, image rows of a unit, image width and height
+  int units_h, units;            // units per image, units in all
+  int half_bytes;                // shared memory of one halo box, a multiple of 1024
+  uint32_t box_tx;               // bytes that the TMA unit delivers for it
+  int cout, n_tiles;
+  int row_shift[kMaxTaps];       // first A row of the tap
+  int32_t kofs[kMaxTaps];        // first column of the tap in the weight matrix
+};
+
+struct HaloMaps {
+  CUtensorMap a, b, c;
+};
+
+constexpr int kHaloStages   = 2;    // halo boxes in flight, two halves each
+constexpr int kHaloMaxSlots = 12;
+constexpr int kHaloFixed    = 2 * kBM * 128 + 1024 /*alignment*/ + 512 /*barriers*/ + 4096 /*statistics*/;
+
+template <int BN>
+__global__ void __launch_bounds__(kConvThreads, 1)
+ConvHaloKernel(const __grid_constant__ HaloMaps maps, const __grid_constant__ HaloParams p) {
+  constexpr int kBBytes   = BN * kBK * 2;
+  constexpr int kTmemCols = 4 * BN;  // two tiles of two halves
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem    = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* b_smem  = smem + kHaloStages * 2 * p.half_bytes;
+  uint8_t* staging = b_smem + p.b_slots * kBBytes;
+  uint64_t* a_full     = reinterpret_cast<uint64_t*>(staging + 2 * kBM * 128);
+  uint64_t* a_empty    = a_full + kHaloStages;
+  uint64_t* b_full     = a_empty + kHaloStages;
+  uint64_t* b_empty    = b_full + kHaloMaxSlots;
+  uint64_t* tmem_full  = b_empty + kHaloMaxSlots;  // [2]
+  uint64_t* tmem_empty = tmem_full + 2;            // [2]
+  uint32_t* tmem_slot  = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int m_tiles   = (p.units + 1) / 2;
+  const int num_tiles = m_tiles * p.n_tiles;
+  const int num_k     = 9 * p.cblocks;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kHaloStages; ++s) {
+      MbarInit(&a_full[s], 1);
+      MbarInit(&a_empty[s], 1);
+    }
+    for (int s = 0; s < p.b_slots; ++s) {
+      MbarInit(&b_full[s], 1);
+      MbarInit(&b_empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      MbarInit(&tmem_full[b], 1);
+      MbarInit(&tmem_empty[b], 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(tmem_slot)),
+                 "r"(static_cast<uint32_t>(kTmemCols))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  TcFenceBefore();
+  __syncthreads();
+  TcFenceAfter();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+
+  if (warp == 0) {
+    if (ElectOne()) {
+      uint32_t ia = 0, ib = 0;
+      bool ok = true;
+      auto load_b = [&](int slot, int t, int cb, int nt) {
+        uint8_t* dst = b_smem + slot * kBBytes;
+        MbarExpectTx(&b_full[slot], kBBytes);
+        if (p.b_mn) {
+          for (int j = 0; j < BN / 64; ++j)
+            TmaLoad2D(dst + j * 8192, &maps.b, p.kofs[t] + nt * BN + j * 64, cb * kBK, &b_full[slot]);
+        } else {
+          TmaLoad2D(dst, &maps.b, p.kofs[t] + cb * kBK, nt * BN, &b_full[slot]);
+        }
+      };
+      if (p.b_resident)
+        for (int k = 0; k < num_k; ++k) load_b(k, k % 9, k / 9, 0);
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        const int mt = tile / p.n_tiles, nt = tile % p.n_tiles;
+        const int halves = p.units - 2 * mt < 2 ? 1 : 2;
+        for (int cb = 0; cb < p.cblocks && ok; ++cb, ++ia) {
+          const int s = ia % kHaloStages;
+          if (!MbarWait(&a_empty[s], ((ia / kHaloStages) & 1) ^ 1)) {
+            atomicExch(p.error, 1);
+            ok = false;
+            break;
+          }
+          MbarExpectTx(&a_full[s], p.box_tx * halves);
+          for (int h = 0; h < halves; ++h) {
+            const int u = 2 * mt + h;
+            TmaLoad4D(smem + (s * 2 + h) * p.half_bytes, &maps.a, cb * kBK, -1, (u % p.units_h) * p.th - 1, u / p.units_h,
+                      &a_full[s]);
+          }
+          if (p.b_resident) continue;
+          for (int t = 0; t < 9; ++t, ++ib) {
+            const int slot = ib % p.b_slots;
+            if (!MbarWait(&b_empty[slot], ((ib / p.b_slots) & 1) ^ 1)) {
+              atomicExch(p.error, 1);
+              ok = false;
+              break;
+            }
+            load_b(slot, t, cb, nt);
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    {  // the whole warp walks the loop, one lane issues
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (p.b_mn ? (1u << 16) : 0u) |
+                             (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
+      const uint64_t b_kstep = p.b_mn ? 128 : 2;
+      uint32_t ia = 0, ib = 0;
+      int local = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
+        const int mt = tile / p.n_tiles;
+        const int halves = p.units - 2 * mt < 2 ? 1 : 2;
+        const int buf = local & 1;
+        if (!MbarWaitWarp(&tmem_empty[buf], ((local >> 1) & 1) ^ 1)) {
+          if (lane == 0) atomicExch(p.error, 4);
+          break;
+        }
+        TcFenceAfter();
+        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * 2 * BN);
+        for (int cb = 0; cb < p.cblocks && ok; ++cb, ++ia) {
+          const int s = ia % kHaloStages;
+          if (!MbarWaitWarp(&a_full[s], (ia / kHaloStages) & 1)) {
+            if (lane == 0) atomicExch(p.error, 2);
+            ok = false;
+            break;
+          }
+          const uint32_t a_addr = SmemAddr(smem + s * 2 * p.half_bytes);
+          for (int t = 0; t < 9; ++t) {
+            const int slot = p.b_resident ? cb * 9 + t : static_cast<int>(ib % p.b_slots);
+            // resident blocks complete phase 0 once; the wait is then a single test
+            if (!MbarWaitWarp(&b_full[slot], p.b_resident ? 0 : (ib / p.b_slots) & 1)) {
+              if (lane == 0) atomicExch(p.error, 5);
+              ok = false;
+              break;
+            }
+            TcFenceAfter();
+            const uint32_t b_addr = SmemAddr(b_smem + slot * kBBytes);
+            const uint64_t bdesc  = p.b_mn ? SmemDescMnSw128(b_addr, 8192) : SmemDescSw128(b_addr);
+            if (ElectOne()) {
+              for (int h = 0; h < halves; ++h) {
+                const uint64_t adesc = SmemDescSw128(a_addr + h * p.half_bytes + p.row_shift[t] * 128);
+#pragma unroll
+                for (int k = 0; k < kBK / 16; ++k)
+                  UmmaBf16(tmem_d + static_cast<uint32_t>(h * BN), adesc + 2 * k, bdesc + b_kstep * k, idesc,
+                           (cb > 0 || t > 0 || k > 0) ? 1u : 0u);
+              }
+              if (!p.b_resident) UmmaCommit(&b_empty[slot]);
+            }
+            if (!p.b_resident) ++ib;
+          }
+          if (ElectOne()) UmmaCommit(&a_empty[s]);
+        }
+        if (ok && ElectOne()) UmmaCommit(&tmem_full[buf]);
+      }
+    }
+  } else if (warp < 6) {
+    // Epilogue: accumulator row r is pixel (r / pitch, r % pitch) of the unit; the real ones go, densely, into a box of
+    // [th x w] pixels x 64 channels for the TMA store unit.
+    const int q  = warp & 3;
+    const int r  = q * 32 + lane;
+    const int ph = r / p.pitch, pw = r % p.pitch;
+    const bool real = pw < p.w && ph < p.th;
+    const int dst   = ph * p.w + pw;
+    const int bar_threads = p.stat_sum != nullptr ? 256 : 128;
+    int local = 0;
+    uint32_t boxes = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
+      const int mt = tile / p.n_tiles, nt = tile % p.n_tiles;
+      const int halves = p.units - 2 * mt < 2 ? 1 : 2;
+      const int buf = local & 1;
+      if (ok && !MbarWait(&tmem_full[buf], (local >> 1) & 1)) {
+        if (lane == 0) atomicExch(p.error, 3);
+        ok = false;
+      }
+      TcFenceAfter();
+      for (int h = 0; h < halves; ++h) {
+        const int u = 2 * mt + h;
+        const uint32_t tsrc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>((buf * 2 + h) * BN);
+#pragma unroll 1
+        for (int b = 0; b < BN / 64; ++b, ++boxes) {
+          uint8_t* box = staging + (boxes & 1) * (kBM * 128);
+          uint32_t acc[2][32];
+          if (ok) {
+            TmemLoad32Async(tsrc + static_cast<uint32_t>(b * 64), acc[0]);
+            TmemLoad32Async(tsrc + static_cast<uint32_t>(b * 64 + 32), acc[1]);
+          }
+          if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          NamedBarSync(1, bar_threads);
+          if (ok) {
+            TmemLoadWait(acc[0]);
+            TmemLoadWait(acc[1]);
+            if (real) {
+#pragma unroll
+              for (int g = 0; g < 8; ++g) {
+                alignas(16) __nv_bfloat16 o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16_rn(__uint_as_float(acc[g >> 2][(g & 3) * 8 + j]));
+                *reinterpret_cast<uint4*>(box + dst * 128 + ((g ^ (dst & 7)) << 4)) = *reinterpret_cast<uint4*>(o);
+              }
+            }
+          }
+          if (h == halves - 1 && b == BN / 64 - 1 && ok) {
+            TcFenceBefore();
+            __syncwarp();
+            if (lane == 0) MbarArrive(&tmem_empty[buf]);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          NamedBarSync(1, bar_threads);
+          if (warp == 2 && lane == 0) {
+            if (ok) {
+              const int ch = nt * BN + b * 64, h0 = (u % p.units_h) * p.th, n0 = u / p.units_h;
+              if (p.accumulate) TmaReduceAdd4D(&maps.c, ch, 0, h0, n0, box);
+              else TmaStore4D(&maps.c, ch, 0, h0, n0, box);
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+      }
+    }
+    if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  } else if (p.stat_sum != nullptr) {
+    // Statistics of the staged boxes, as in the tap kernel; a box holds th * w pixels, fewer in the last unit of an image.
+    float* partial   = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a_full) + 512);  // [2][4 warps][64][2]
+    const int st     = threadIdx.x - 192;
+    const int chunk  = st & 7;
+    const int rg     = st >> 3;
+    const int sw     = st >> 5;
+    uint32_t boxes = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      const int mt = tile / p.n_tiles, nt = tile % p.n_tiles;
+      const int halves = p.units - 2 * mt < 2 ? 1 : 2;
+      for (int h = 0; h < halves; ++h) {
+        const int h0   = ((2 * mt + h) % p.units_h) * p.th;
+        const int rows = (p.ho - h0 < p.th ? p.ho - h0 : p.th) * p.w;
+#pragma unroll 1
+        for (int b = 0; b < BN / 64; ++b, ++boxes) {
+          NamedBarSync(1, 256);
+          NamedBarSync(1, 256);
+          const uint8_t* box = staging + (boxes & 1) * (kBM * 128);
+          float s1[8], s2[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) s1[j] = s2[j] = 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int row = rg + 16 * i;
+            if (row < rows) {
+              const uint4 v = *reinterpret_cast<const uint4*>(box + row * 128 + ((chunk ^ (row & 7)) << 4));
+              const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(hv[j]);
+                s1[2 * j] += f.x; s2[2 * j] += f.x * f.x;
+                s1[2 * j + 1] += f.y; s2[2 * j + 1] += f.y * f.y;
+              }
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], 8);
+            s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], 16);
+            s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 8);
+            s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 16);
+          }
+          float* P = partial + (boxes & 1) * (4 * 64 * 2);
+          if (lane < 8) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              P[(sw * 64 + lane * 8 + j) * 2]     = s1[j];
+              P[(sw * 64 + lane * 8 + j) * 2 + 1] = s2[j];
+            }
+          }
+          NamedBarSync(2, 128);
+          const int col = st & 63, which = st >> 6;
+          const float tot = P[(0 * 64 + col) * 2 + which] + P[(1 * 64 + col) * 2 + which] +
+                            P[(2 * 64 + col) * 2 + which] + P[(3 * 64 + col) * 2 + which];
+          const int ch = nt * BN + b * 64 + col;
+          if (ch < p.cout) atomicAdd((which ? p.stat_sq : p.stat_sum) + ch, tot);
+        }
+      }
+    }
+  }
+  TcFenceBefore();
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
+                 "r"(static_cast<uint32_t>(kTmemCols))
+                 : "memory");
+  }
+}
+
 // ------------------------------------------------------------------ weight gradient
 // dw[co, tap, ci] = sum over output pixels p of dy[p, co] * x[p*stride + tap - pad, ci].  The contraction runs
 // over pixels, which are the ROWS of both tiles as the TMA unit delivers them, so both operands are
@@ -466,7 +785,7 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ElectOne()) {
       for (int kt = 0; kt < num_k; ++kt) {
         const int s = kt % Cfg::kStages;
         if (!MbarWait(&empty_bar[s], ((kt / Cfg::kStages) & 1) ^ 1)) {
@@ -489,7 +808,7 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {  // the whole warp walks the loop, one lane issues
       // both operands MN-major: bits 15 and 16
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                                  (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
@@ -497,26 +816,28 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
       bool ok = true;
       for (int kt = 0; kt < num_k && ok; ++kt) {
         const int s = kt % Cfg::kStages;
-        if (!MbarWait(&full_bar[s], (kt / Cfg::kStages) & 1)) {
-          atomicExch(p.error, 2);
+        if (!MbarWaitWarp(&full_bar[s], (kt / Cfg::kStages) & 1)) {
+          if (lane == 0) atomicExch(p.error, 2);
           ok = false;
           break;
         }
         TcFenceAfter();
         const uint32_t a_addr = SmemAddr(smem + s * Cfg::kStageBytes);
         const uint64_t bdesc  = SmemDescMnSw128(a_addr + Cfg::kABytes, Cfg::kBoxBytes);
+        if (ElectOne()) {
 #pragma unroll
-        for (int h = 0; h < kMH; ++h) {
-          const uint64_t adesc = SmemDescMnSw128(a_addr + h * 2 * Cfg::kBoxBytes, Cfg::kBoxBytes);
-          for (int k = 0; k < ksteps; ++k) {
-            // 16 pixels further along K = 16 rows of 128 bytes
-            UmmaBf16(tmem_base + static_cast<uint32_t>(h * BN), adesc + static_cast<uint64_t>(k) * (2048 >> 4),
-                     bdesc + static_cast<uint64_t>(k) * (2048 >> 4), idesc, (kt > 0 || k > 0) ? 1u : 0u);
+          for (int h = 0; h < kMH; ++h) {
+            const uint64_t adesc = SmemDescMnSw128(a_addr + h * 2 * Cfg::kBoxBytes, Cfg::kBoxBytes);
+            for (int k = 0; k < ksteps; ++k) {
+              // 16 pixels further along K = 16 rows of 128 bytes
+              UmmaBf16(tmem_base + static_cast<uint32_t>(h * BN), adesc + static_cast<uint64_t>(k) * (2048 >> 4),
+                       bdesc + static_cast<uint64_t>(k) * (2048 >> 4), idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            }
           }
+          UmmaCommit(&empty_bar[s]);
         }
-        UmmaCommit(&empty_bar[s]);
       }
-      UmmaCommit(tmem_full);
+      if (ElectOne()) UmmaCommit(tmem_full);
     }
   } else {
     const int q = warp & 3;
@@ -549,6 +870,144 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(static_cast<uint32_t>(Cfg::kTmemCols))
                  : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ weight gradient, 3x3, stride 1, 64 -> 64 channels
+// The kernel above fetches dy and x once per tap for these few channels, 32 KB for 64 x 64 x 128 products, and leaves half
+// of the MMA's rows empty.  Here a CTA walks over units of `th` image rows, loads dy ([th + 1] rows) and x with its border
+// ([th + 2] rows) once, both with the same pitch (w + 2 rounded up to the 16 pixels of an MMA step), and keeps all nine
+// taps in TMEM.  With p a pixel of the unit, tap (r, s) needs x at row p + r * pitch + s of its box, so
+//   B  N = 192: the three horizontal taps are three 64-channel chunks of one operand, one pixel (128 bytes) apart;
+//   A  M = 128: dy at p and dy at p + pitch, one image row further down.  The second chunk meets the x of tap r at tap
+//      r - 1, so B at r = 2 yields tap 2 and B at r = 1 yields taps 1 and 0: two MMAs per 16 pixels instead of nine.
+// The second chunk runs over dy rows 1 .. h: row h is zero fill, and row 0 only meets the zero padding at tap 0.  Columns
+// w .. pitch - 1 of dy are zero fill, so what x holds beside them does not count (as long as it is finite).
+// 256 images of 56 x 56: 69 us, 180 with a launch row per tap.
+struct WgradHaloParams {
+  int32_t* error;
+  float* dw;              // [64, 9 * 64] fp32, accumulated into
+  int pitch, th, units_h, units;
+  int dy_bytes, x_bytes;  // of the boxes; 1 KB behind x stays zero (the last shifted rows reach two pixels beyond it)
+  int stages;
+};
+
+struct WgradHaloMaps {
+  CUtensorMap x, dy;
+};
+
+constexpr int kWgradHaloMaxStages = 4;
+constexpr int kWgradHaloN         = 192;
+
+__global__ void __launch_bounds__(kGemmThreads, 1)
+ConvWgradHaloKernel(const __grid_constant__ WgradHaloMaps maps, const __grid_constant__ WgradHaloParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int stage_bytes = p.dy_bytes + p.x_bytes + 1024;
+  uint64_t* full_bar  = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
+  uint64_t* empty_bar = full_bar + kWgradHaloMaxStages;
+  uint64_t* tmem_full = empty_bar + kWgradHaloMaxStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+
+  for (int i = threadIdx.x; i < p.stages * 64; i += kGemmThreads)  // the zero kilobyte of every stage
+    *reinterpret_cast<uint4*>(smem + (i >> 6) * stage_bytes + p.dy_bytes + p.x_bytes + (i & 63) * 16) = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      MbarInit(&full_bar[s], 1);
+      MbarInit(&empty_bar[s], 1);
+    }
+    MbarInit(tmem_full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(tmem_slot)), "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  TcFenceBefore();
+  __syncthreads();
+  TcFenceAfter();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+
+  if (warp == 0) {
+    if (ElectOne()) {
+      int it = 0;
+      for (int u = blockIdx.x; u < p.units; u += gridDim.x, ++it) {
+        const int s = it % p.stages;
+        if (!MbarWait(&empty_bar[s], ((it / p.stages) & 1) ^ 1)) {
+          atomicExch(p.error, 1);
+          break;
+        }
+        const int h0 = (u % p.units_h) * p.th, n0 = u / p.units_h;
+        uint8_t* dst = smem + s * stage_bytes;
+        MbarExpectTx(&full_bar[s], static_cast<uint32_t>(p.dy_bytes + p.x_bytes));
+        TmaLoad4D(dst, &maps.dy, 0, 0, h0, n0, &full_bar[s]);
+        TmaLoad4D(dst + p.dy_bytes, &maps.x, 0, -1, h0 - 1, n0, &full_bar[s]);
+      }
+    }
+  } else if (warp == 1) {
+    {  // the whole warp walks the loop, one lane issues
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                                 (static_cast<uint32_t>(kWgradHaloN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
+      const int ksteps = p.th * p.pitch / 16;
+      int it = 0;
+      for (int u = blockIdx.x; u < p.units; u += gridDim.x, ++it) {
+        const int s = it % p.stages;
+        if (!MbarWaitWarp(&full_bar[s], (it / p.stages) & 1)) {
+          if (lane == 0) atomicExch(p.error, 2);
+          break;
+        }
+        TcFenceAfter();
+        const uint32_t a_addr = SmemAddr(smem + s * stage_bytes);
+        const uint32_t b_addr = a_addr + p.dy_bytes;
+        const uint64_t adesc  = SmemDescMnSw128(a_addr, p.pitch * 128);
+        const uint64_t bdesc2 = SmemDescMnSw128(b_addr + 2 * p.pitch * 128, 128);
+        const uint64_t bdesc1 = SmemDescMnSw128(b_addr + p.pitch * 128, 128);
+        if (ElectOne()) {
+          for (int k = 0; k < ksteps; ++k) {
+            const uint32_t acc = (it > 0 || k > 0) ? 1u : 0u;
+            UmmaBf16(tmem_base, adesc + 128 * k, bdesc2 + 128 * k, idesc, acc);
+            UmmaBf16(tmem_base + 256, adesc + 128 * k, bdesc1 + 128 * k, idesc, acc);
+          }
+          UmmaCommit(&empty_bar[s]);
+        }
+      }
+      if (ElectOne()) UmmaCommit(tmem_full);
+    }
+  } else {
+    const int q = warp & 3;
+    const bool ok = MbarWait(tmem_full, 0);
+    if (!ok && lane == 0) atomicExch(p.error, 3);
+    TcFenceAfter();
+    if (ok && blockIdx.x < p.units) {
+      // lanes 0..63: taps 2 (columns 0..191) and 1 (256..447) of output channel `lane`; lanes 64..127: tap 0 (256..447)
+      const int row = (q & 1) * 32 + lane;
+      const bool second = q >= 2;
+#pragma unroll 1
+      for (int c = second ? 6 : 0; c < 12; ++c) {
+        const int part = c / 6, cc = c % 6;  // accumulator, 32-column chunk of it
+        uint32_t acc[32];
+        TmemLoad32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(part * 256 + cc * 32), acc);
+        const int tap_row = part == 0 ? 2 : second ? 0 : 1;
+        float* dst = p.dw + row * 576 + (tap_row * 3 + cc / 2) * 64 + (cc & 1) * 32;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + g * 4),
+                       "f"(__uint_as_float(acc[g * 4])), "f"(__uint_as_float(acc[g * 4 + 1])),
+                       "f"(__uint_as_float(acc[g * 4 + 2])), "f"(__uint_as_float(acc[g * 4 + 3]))
+                       : "memory");
+        }
+      }
+    }
+  }
+  TcFenceBefore();
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
 }
 
@@ -679,6 +1138,80 @@ int LaunchWgrad(const WgradMaps& maps, const WgradParams& p, int splits, cudaStr
   return 0;
 }
 
+// Image rows of a unit of the halo kernel (0: the image is too wide for two).
+int HaloRows(int w, int h) {
+  const int th = kBM / (w + 2);
+  return th < 2 ? 0 : std::min(th, h);
+}
+int HaloHalfBytes(int w, int th) { return CeilDiv(static_cast<int64_t>(w + 2) * (th + 2) * 128, 1024) * 1024; }
+
+// Whether the halo kernel should run a 3x3 / stride 1 convolution into `w_rows` channels of [n, h, w] pixels: narrow
+// output tiles (a 256-channel tile does enough work per loaded byte), and units that fill the 128 rows of an MMA about
+// as well as the tap kernel's boxes do.
+bool PreferHalo(int n, int h, int w, int w_rows) {
+  const int th = HaloRows(w, h);
+  if (th == 0 || w_rows % 256 == 0) return false;
+  const int64_t units = static_cast<int64_t>(n) * CeilDiv(h, th);
+  const Box box       = PickBox(w, h, n, false);
+  const int64_t boxes = static_cast<int64_t>(CeilDiv(w, box.tw)) * CeilDiv(h, box.th) * CeilDiv(n, box.tn);
+  return units >= 2 * NumSMs() && units * 10 <= boxes * 12;
+}
+
+template <int BN>
+int LaunchHalo(const HaloMaps& maps, const HaloParams& p, cudaStream_t s) {
+  static bool configured = false;
+  if (!configured) {
+    TIPSK_CUDA(cudaFuncSetAttribute(ConvHaloKernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
+    configured = true;
+  }
+  const int64_t tiles = static_cast<int64_t>((p.units + 1) / 2) * p.n_tiles;
+  const int grid = static_cast<int>(std::min<int64_t>(tiles, NumSMs()));
+  const int smem = kHaloStages * 2 * p.half_bytes + p.b_slots * BN * 128 + kHaloFixed;
+  ConvHaloKernel<BN><<<grid, kConvThreads, smem, s>>>(maps, p);
+  TIPSK_LAUNCH_CHECK();
+  return 0;
+}
+
+// out = 3x3 / stride 1 convolution of `in` (both [n, h, w] pixels) with the tap list of RunTaps.
+int RunHalo(const View& in, const ConvTap* taps, int cin, const void* weights, int w_rows, int64_t w_cols,
+            const View& out, float* stat_sum, float* stat_sq, cudaStream_t s, int accumulate, int b_mn) {
+  TIPSK_REQUIRE(cin % 64 == 0 && w_rows % 64 == 0, "conv: channel counts must be multiples of 64");
+  const int w = static_cast<int>(out.w), h = static_cast<int>(out.h), n = static_cast<int>(out.n);
+  const int th = HaloRows(w, h);
+  const int bn = w_rows % 128 == 0 ? 128 : 64;
+  HaloMaps maps;
+  HaloParams p{};
+  int rc = MapOf(&maps.a, in, Box{w + 2, th + 2, 1});
+  if (rc) return rc;
+  rc = b_mn ? MakeTmap2D(&maps.b, weights, cin, w_cols, 64) : MakeTmap2D(&maps.b, weights, w_rows, w_cols, bn);
+  if (rc) return rc;
+  rc = MapOf(&maps.c, out, Box{w, th, 1});
+  if (rc) return rc;
+  p.error = ConvErrorWord();
+  TIPSK_REQUIRE(p.error != nullptr, "conv: cannot allocate the error word");
+  p.stat_sum = stat_sum;
+  p.stat_sq  = stat_sq;
+  p.accumulate = accumulate;
+  p.b_mn    = b_mn;
+  p.cblocks = cin / 64;
+  p.pitch = w + 2; p.th = th; p.w = w; p.ho = h;
+  p.units_h = CeilDiv(h, th);
+  p.units   = n * p.units_h;
+  p.half_bytes = HaloHalfBytes(w, th);
+  p.box_tx     = static_cast<uint32_t>(w + 2) * (th + 2) * 128u;
+  p.cout    = w_rows;
+  p.n_tiles = w_rows / bn;
+  const int room = kMaxSmemBytes - kHaloFixed - kHaloStages * 2 * p.half_bytes;
+  p.b_slots    = std::min(kHaloMaxSlots, room / (bn * 128));
+  p.b_resident = (p.n_tiles == 1 && 9 * p.cblocks <= p.b_slots) ? 1 : 0;
+  TIPSK_REQUIRE(p.b_slots >= 2, "conv: the halo box leaves no shared memory for the weights");
+  for (int t = 0; t < 9; ++t) {
+    p.row_shift[t] = (taps[t].dh + 1) * p.pitch + taps[t].dw + 1;
+    p.kofs[t]      = taps[t].kofs;
+  }
+  return bn == 64 ? LaunchHalo<64>(maps, p, s) : LaunchHalo<128>(maps, p, s);
+}
+
 // Runs the tap kernel: out[view_out pixel, co] = sum over taps and 64-channel blocks.
 int RunTaps(const View* in_views, int n_views, const ConvTap* taps, int n_taps, int cin, const void* weights,
             int w_rows, int64_t w_cols, const View& out, float* stat_sum, float* stat_sq, cudaStream_t s,
@@ -694,7 +1227,9 @@ int RunTaps(const View* in_views, int n_views, const ConvTap* taps, int n_taps, 
   p.tiles_n = CeilDiv(out.n, box.tn);
   const int64_t m_tiles = static_cast<int64_t>(p.tiles_w) * p.tiles_h * p.tiles_n;
   int bn = 128;
-  if (w_rows % 128 != 0) bn = 64;
+  // Few tiles (a request of one or a few images): a CTA's chain of K steps is bound by the bytes it loads per step, and
+  // half as wide a tile loads a quarter less and runs on twice as many SMs.
+  if (w_rows % 128 != 0 || m_tiles * (w_rows / 128) * 2 <= NumSMs()) bn = 64;
   else if (w_rows % 256 == 0 && m_tiles * (w_rows / 256) >= NumSMs()) bn = 256;
   int rc;
   for (int i = 0; i < n_views; ++i) {
@@ -811,6 +1346,43 @@ int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, 
   return bn == 128 ? LaunchWgrad<128, 128>(maps, p, splits, st) : LaunchWgrad<64, 128>(maps, p, splits, st);
 }
 
+// The halo weight gradient: 64 -> 64 channels, images whose rows fill most of the pitch, and units for every SM.
+bool PreferWgradHalo(int n, int h, int w, int cin, int cout) {
+  if (cin != 64 || cout != 64 || w + 2 > 64) return false;
+  const int pitch = (w + 2 + 15) / 16 * 16, th = std::min(256 / pitch, h);
+  return w * 10 >= pitch * 8 && static_cast<int64_t>(n) * CeilDiv(h, th) >= 2 * NumSMs();
+}
+
+int RunWgradHalo(const void* x, const void* dy, float* dw, int n, int h, int w, cudaStream_t st) {
+  WgradHaloMaps maps;
+  WgradHaloParams p{};
+  p.pitch   = (w + 2 + 15) / 16 * 16;
+  p.th      = std::min(256 / p.pitch, h);
+  p.units_h = CeilDiv(h, p.th);
+  p.units   = n * p.units_h;
+  p.dy_bytes = (p.th + 1) * p.pitch * 128;
+  p.x_bytes  = (p.th + 2) * p.pitch * 128;
+  const int stage = p.dy_bytes + p.x_bytes + 1024;
+  p.stages = std::min(kWgradHaloMaxStages, (kMaxSmemBytes - 1024 - 256) / stage);
+  TIPSK_REQUIRE(p.stages >= 2, "conv wgrad: the halo boxes do not fit in shared memory");
+  int rc = MapOf(&maps.dy, FullView(dy, n, h, w, 64), Box{p.pitch, p.th + 1, 1});
+  if (rc) return rc;
+  rc = MapOf(&maps.x, FullView(x, n, h, w, 64), Box{p.pitch, p.th + 2, 1});
+  if (rc) return rc;
+  p.error = ConvErrorWord();
+  TIPSK_REQUIRE(p.error != nullptr, "conv: cannot allocate the error word");
+  p.dw = dw;
+  TIPSK_CUDA(cudaMemsetAsync(dw, 0, sizeof(float) * 64 * 576, st));
+  static bool configured = false;
+  if (!configured) {
+    TIPSK_CUDA(cudaFuncSetAttribute(ConvWgradHaloKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
+    configured = true;
+  }
+  ConvWgradHaloKernel<<<std::min(p.units, NumSMs()), kGemmThreads, p.stages * stage + 1024 + 256, st>>>(maps, p);
+  TIPSK_LAUNCH_CHECK();
+  return 0;
+}
+
 // Copies a 3-channel NHWC image into the zero-padded 8-channel buffer of the stem convolution.
 __global__ void __launch_bounds__(256)
 StemPadKernel(const __nv_bfloat16* __restrict__ x, uint4* __restrict__ xp, int n, int h, int w, int hp, int wp) {
@@ -910,6 +1482,9 @@ int tipsk_conv2d_fwd(const void* x, const void* wgt, void* y, int n, int h, int 
     nv = 4;
     for (int b = 0; b < 4; ++b) views[b] = PhaseView(x, n, h, w, cin, b >> 1, b & 1);
   }
+  if (r == 3 && stride == 1 && PreferHalo(n, h, w, cout))
+    return RunHalo(views[0], taps, cin, wgt, cout, static_cast<int64_t>(r) * s * cin, out, stat_sum, stat_sq,
+                   static_cast<cudaStream_t>(stream), 0, 0);
   return RunTaps(views, nv, taps, nt, cin, wgt, cout, static_cast<int64_t>(r) * s * cin, out, stat_sum, stat_sq,
                  static_cast<cudaStream_t>(stream));
 }
@@ -951,6 +1526,8 @@ static int DgradImpl(const void* dy, const void* wgt_t, void* dx, int n, int h, 
       }
     View in  = r == 1 ? FlatView(dy, n, ho, wo, cout) : FullView(dy, n, ho, wo, cout);
     View out = r == 1 ? FlatView(dx, n, h, w, cin) : FullView(dx, n, h, w, cin);
+    if (r == 3 && PreferHalo(n, h, w, cin))
+      return RunHalo(in, taps, cout, wgt_t, cin, w_cols, out, nullptr, nullptr, st, accumulate, ohwi);
     return RunTaps(&in, 1, taps, nt, cout, wgt_t, cin, w_cols, out, nullptr, nullptr, st, accumulate, ohwi);
   }
   // stride 2: the input pixels of parity class (bh, bw) receive the taps with (b + pad - f) even
@@ -990,6 +1567,8 @@ int tipsk_conv2d_wgrad(const void* x, const void* dy, float* dw, int n, int h, i
   ConvTap taps[kMaxTaps];
   const int nt = ForwardTaps(r, s, stride, pad, cin, taps);
   const bool flat = (r == 1 && stride == 1);
+  if (r == 3 && stride == 1 && PreferWgradHalo(n, h, w, cin, cout))
+    return RunWgradHalo(x, dy, dw, n, h, w, static_cast<cudaStream_t>(stream));
   const View dyv = flat ? FlatView(dy, n, ho, wo, cout) : FullView(dy, n, ho, wo, cout);
   View xv[4];
   int nv = 1;

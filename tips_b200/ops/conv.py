@@ -19,6 +19,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import base
+from .linear import _weight_grad as linear_weight_grad
 
 
 # TIPS_CONV_DGRAD_TRANSPOSED_COPY=1: give the data gradient a transposed copy of the weights (K-major operand)
@@ -108,6 +109,16 @@ def conv2d_wgrad(x, dy, weight_shape, stride, padding):
     return dw
 
 
+def _weight_gradient(x, dy, weight, stride, padding):
+    """Gradient of `weight` in its own dtype.  A 1x1 convolution is a matrix product over the pixels: in bf16 it takes the
+    GEMM's weight-gradient path, which rounds the fp32 sums once instead of leaving an fp32 copy to cast."""
+    cout, r, _, cin = weight.shape
+    if r == 1 and stride == 1 and weight.dtype == torch.bfloat16:
+        flat = lambda t: _nhwc(t).permute(0, 2, 3, 1).reshape(-1, t.shape[1])
+        return linear_weight_grad(flat(dy), flat(x), weight.dtype).view(weight.shape).to(weight.dtype)
+    return conv2d_wgrad(x, dy, tuple(weight.shape), stride, padding).to(weight.dtype)
+
+
 class _Conv2dFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, stride, padding, stats):
@@ -123,7 +134,7 @@ class _Conv2dFn(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             dx = conv2d_dgrad(dy, weight, tuple(xc.shape), ctx.stride, ctx.padding)
         if ctx.needs_input_grad[1]:
-            dw = conv2d_wgrad(xc, dy, tuple(weight.shape), ctx.stride, ctx.padding).to(weight.dtype)
+            dw = _weight_gradient(xc, dy, weight, ctx.stride, ctx.padding)
         return dx, dw, None, None, None
 
 
@@ -150,7 +161,7 @@ class _Conv2dPassFn(torch.autograd.Function):
                 into = d_alias if d_alias.is_contiguous(memory_format=torch.channels_last) else _nhwc(d_alias)
             dx = conv2d_dgrad(dy, weight, tuple(xc.shape), ctx.stride, ctx.padding, into=into)
         if ctx.needs_input_grad[1]:
-            dw = conv2d_wgrad(xc, dy, tuple(weight.shape), ctx.stride, ctx.padding).to(weight.dtype)
+            dw = _weight_gradient(xc, dy, weight, ctx.stride, ctx.padding)
         return dx, dw, None, None, None
 
 
