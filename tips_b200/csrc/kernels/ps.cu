@@ -164,6 +164,24 @@ TableInitKernel(float* shard, int64_t rows_local, int dim, int field, int rank, 
   }
 }
 
+// System-scope 16-byte load of data that no one writes while the kernel runs (rows between two fences, inbox
+// entries after the fence): not volatile and without a "memory" clobber, so several of them can be in flight.
+__device__ __forceinline__ U4 LdSysFree(const void* addr) {
+  U4 v;
+  asm("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(addr));
+  return v;
+}
+
+constexpr int kRowsInFlight = 8;  // rows that a lane group loads before it stores the first one
+
+// Pull and scatter are bound by latency: a row is 64 to 256 bytes somewhere in memory, found through a chain of dependent
+// loads and 64-bit divisions.  So every lane of a warp resolves one item of its own (the ids of a warp in one load), and
+// then the warp moves the rows of all of them, kRowsInFlight loads per lane before the first is consumed.  With one item
+// per lane group at a time (8192 x 26 x 64): pull 35 us, scatter 36; like this 14 and 29.  The same form of the apply pass,
+// which has three loads per row, needs 128 registers and was slower (32 against 27 us).  Large batches take 32 items per
+// warp; small ones 8, so that they still spread over the SMs.
+__device__ __forceinline__ int WarpChunk(int64_t total) { return total >= 65536 ? 32 : 8; }
+
 template <typename OutT>
 __global__ void __launch_bounds__(256)
 PsPullKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t out_ld, int64_t out_col0) {
@@ -175,34 +193,56 @@ PsPullKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t out_ld, int64_t 
   const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps      = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const int64_t total       = batch * meta.nfields;
+  const int chunk           = WarpChunk(total);
   OutT* out = static_cast<OutT*>(pr.out);
-  for (int64_t base = warp_global * L.ipw; base < total; base += nwarps * L.ipw) {
-    const int64_t item = base + L.sub;
-    if (item >= total) continue;
-    const int f      = static_cast<int>(item % meta.nfields);
-    const int64_t b  = item / meta.nfields;
-    const int64_t id = pr.ids[item];
-    OutT* dst        = out + b * out_ld + out_col0 + static_cast<int64_t>(f) * dim;
-    int owner;
-    int64_t lrow;
-    PsPlace(f, id < 0 ? 0 : id, n, &owner, &lrow);
-    if (id < 0 || lrow >= meta.rows_per_shard[f]) {
-      if (L.sublane == 0) atomicExch(pr.error, 2);
-      for (int v = L.sublane; v < vecs; v += L.lpi)
-        for (int k = 0; k < 4; ++k) dst[v * 4 + k] = FromFloat<OutT>(0.f);
-      continue;
-    }
-    const char* row = pr.slab[owner] + meta.field_off[f] + static_cast<uint64_t>(lrow) * dim * 4;
-    for (int v = L.sublane; v < vecs; v += L.lpi) {
-      U4 q = owner == pr.my_server ? *reinterpret_cast<const U4*>(row + v * 16) : LdSys(row + v * 16);
-      const float fv[4] = {__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
-      if (sizeof(OutT) == 4) {
-        *reinterpret_cast<U4*>(dst + v * 4) = q;
+  for (int64_t base = warp_global * chunk; base < total; base += nwarps * chunk) {
+    const int64_t item = base + L.lane;
+    const char* src = nullptr;  // null: a bad id, whose row reads as zeros
+    int64_t dst     = -1;       // element offset of the item's row in the output; negative: no item
+    bool own        = true;
+    if (L.lane < chunk && item < total) {
+      const int64_t b  = item / meta.nfields;
+      const int f      = static_cast<int>(item - b * meta.nfields);
+      const int64_t id = pr.ids[item];
+      dst = b * out_ld + out_col0 + static_cast<int64_t>(f) * dim;
+      int owner;
+      int64_t lrow;
+      PsPlace(f, id < 0 ? 0 : id, n, &owner, &lrow);
+      if (id < 0 || lrow >= meta.rows_per_shard[f]) {
+        atomicExch(pr.error, 2);
       } else {
-        OutT o[4];
+        src = pr.slab[owner] + meta.field_off[f] + static_cast<uint64_t>(lrow) * dim * 4;
+        own = owner == pr.my_server;
+      }
+    }
+    for (int j = 0; j < chunk; j += L.ipw * kRowsInFlight) {
+      for (int v0 = 0; v0 < vecs; v0 += L.lpi) {
+        const int v = v0 + L.sublane;
+        U4 q[kRowsInFlight];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) o[k] = FromFloat<OutT>(fv[k]);
-        *reinterpret_cast<uint2*>(dst + v * 4) = *reinterpret_cast<uint2*>(o);
+        for (int u = 0; u < kRowsInFlight; ++u) {
+          const int from   = j + u * L.ipw + L.sub;
+          const char* row  = reinterpret_cast<const char*>(
+              __shfl_sync(kFullMask, reinterpret_cast<unsigned long long>(src), from & 31));
+          const bool local = __shfl_sync(kFullMask, own, from & 31);
+          q[u] = U4{0, 0, 0, 0};
+          if (from < chunk && v < vecs && row != nullptr)
+            q[u] = local ? *reinterpret_cast<const U4*>(row + v * 16) : LdSysFree(row + v * 16);
+        }
+#pragma unroll
+        for (int u = 0; u < kRowsInFlight; ++u) {
+          const int from   = j + u * L.ipw + L.sub;
+          const int64_t at = __shfl_sync(kFullMask, dst, from & 31);
+          if (from >= chunk || v >= vecs || at < 0) continue;
+          OutT* to = out + at + v * 4;
+          if (sizeof(OutT) == 4) {
+            *reinterpret_cast<U4*>(to) = q[u];
+          } else {
+            OutT o[4] = {FromFloat<OutT>(__uint_as_float(q[u].x)), FromFloat<OutT>(__uint_as_float(q[u].y)),
+                         FromFloat<OutT>(__uint_as_float(q[u].z)), FromFloat<OutT>(__uint_as_float(q[u].w))};
+            *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(o);
+          }
+        }
       }
     }
   }
@@ -248,14 +288,6 @@ __device__ __forceinline__ void RedAdd4(float* addr, float a, float b, float c, 
   asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d));
 }
 
-// System-scope 16-byte load of data that no one writes while the kernel runs (rows between two fences, inbox
-// entries after the fence): not volatile and without a "memory" clobber, so several of them can be in flight.
-__device__ __forceinline__ U4 LdSysFree(const void* addr) {
-  U4 v;
-  asm("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(addr));
-  return v;
-}
-
 template <typename GradT, bool kVec>
 __device__ __forceinline__ void LoadGrad4(const GradT* g, float* out) {
   if (kVec) {
@@ -273,8 +305,6 @@ __device__ __forceinline__ void LoadGrad4(const GradT* g, float* out) {
     for (int k = 0; k < 4; ++k) out[k] = ToFloat<GradT>(g[k]);
   }
 }
-
-constexpr int kRowsInFlight = 8;  // rows that a lane group loads before it stores the first one
 
 // Resolves every (sample, field) item of the batch into a slot of the local table: the distinct rows land in
 // the list, item_slot[item] holds the slot (kNoSlot for a bad id or a full table).
@@ -450,15 +480,19 @@ PsScatterKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t grad_ld, int6
   const GradT* grads        = static_cast<const GradT*>(pr.grads);
   unsigned long long* keys  = reinterpret_cast<unsigned long long*>(pr.acc);
   float* sums_base          = reinterpret_cast<float*>(pr.acc + slots * 8);
-  for (int64_t base = warp_global * 32; base < total; base += nwarps * 32) {
+  const int chunk           = WarpChunk(total);
+  for (int64_t base = warp_global * chunk; base < total; base += nwarps * chunk) {
     const int64_t mine = base + L.lane;
+    const bool have    = L.lane < chunk && mine < total;
+    const int64_t b    = have ? mine / meta.nfields : 0;
+    const int f        = static_cast<int>(have ? mine - b * meta.nfields : 0);
+    const int64_t at   = b * grad_ld + grad_col0 + static_cast<int64_t>(f) * dim;  // of the item's gradient row
     uint32_t slot = kNoSlot;
     if (kIndexed) {
-      if (mine < total) slot = pr.item_slot[mine];
+      if (have) slot = pr.item_slot[mine];
     } else {
       bool claimed = false;
-      if (mine < total) {
-        const int f      = static_cast<int>(mine % meta.nfields);
+      if (have) {
         const int64_t id = pr.ids[mine];
         if (id < 0 || id / n >= meta.rows_per_shard[f]) {
           atomicExch(pr.error, 2);
@@ -469,19 +503,24 @@ PsScatterKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t grad_ld, int6
       }
       AppendSlots(pr.ulist, &pr.ctl->ucount, claimed, slot, L.lane);
     }
-    for (int j = 0; j < 32; j += L.ipw) {
-      const int src      = j + L.sub;
-      const uint32_t s   = __shfl_sync(kFullMask, slot, src);
-      const int64_t item = base + src;
-      if (item >= total || s == kNoSlot) continue;
-      const int f     = static_cast<int>(item % meta.nfields);
-      const int64_t b = item / meta.nfields;
-      float* sums     = sums_base + static_cast<uint64_t>(s) * dim;
-      const GradT* g  = grads + b * grad_ld + grad_col0 + static_cast<int64_t>(f) * dim;
-      for (int v = L.sublane; v < vecs; v += L.lpi) {
-        float gv[4];
-        LoadGrad4<GradT, kVec>(g + v * 4, gv);
-        RedAdd4(sums + v * 4, gv[0] * grad_scale, gv[1] * grad_scale, gv[2] * grad_scale, gv[3] * grad_scale);
+    for (int j = 0; j < chunk; j += L.ipw * kRowsInFlight) {
+      for (int v0 = 0; v0 < vecs; v0 += L.lpi) {
+        const int v = v0 + L.sublane;
+        float gv[kRowsInFlight][4];
+        uint32_t to[kRowsInFlight];
+#pragma unroll
+        for (int u = 0; u < kRowsInFlight; ++u) {
+          const int from    = j + u * L.ipw + L.sub;
+          const int64_t row = __shfl_sync(kFullMask, at, from & 31);
+          to[u]             = __shfl_sync(kFullMask, slot, from & 31);
+          if (from >= chunk || v >= vecs) to[u] = kNoSlot;
+          if (to[u] != kNoSlot) LoadGrad4<GradT, kVec>(grads + row + v * 4, gv[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kRowsInFlight; ++u)
+          if (to[u] != kNoSlot)
+            RedAdd4(sums_base + static_cast<uint64_t>(to[u]) * dim + v * 4, gv[u][0] * grad_scale, gv[u][1] * grad_scale,
+                    gv[u][2] * grad_scale, gv[u][3] * grad_scale);
       }
     }
   }
