@@ -495,20 +495,24 @@ GemmTnPersistentKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 // same product took 183 us).  A second output
 // (the value before the activation, which the backward pass of GELU reads) leaves through the same staging boxes.
 // Bound by the tensor cores.  Measured against the single-CTA kernels it took over from (us, M x N x K): 16384 x 4096 x
-// 1024 with bias 100 : 114 (1377 TFLOP/s), the same with GELU and the second output 159 : 307, 1232 x 30528 x 1024 71 : 105;
+// 1024 with bias 100 : 114 (1377 TFLOP/s), the same with GELU and the second output 139 : 307 (159 with two staging boxes), 1232 x 30528 x 1024 71 : 105;
 // A and B MN-major (a weight gradient) 4096 x 1024 x 16384 92 : 114, 30528 x 1024 x 1232 57 : 128.
-struct PairCfg {
+template <bool kPre>
+struct PairCfgOf {
   static constexpr int kBN            = 256;
-  static constexpr int kStages        = 5;
+  static constexpr int kStages        = kPre ? 4 : 5;
   static constexpr int kABytes        = kBM * kBK * 2;
   static constexpr int kBBytes        = (kBN / 2) * kBK * 2;
   static constexpr int kStageBytes    = kABytes + kBBytes;      // 32 KB per CTA
   static constexpr int kBoxBytes      = kBM * 128;              // 128 rows x 64 columns
-  static constexpr int kStagingBytes  = 4 * kBoxBytes;          // two boxes per epilogue group
+  static constexpr int kGroupBoxes    = kPre ? 3 : 2;           // staging boxes of an epilogue group, used in turn
+  static constexpr int kStagingBytes  = 2 * kGroupBoxes * kBoxBytes;
   static constexpr int kTmemCols      = 512;
   static constexpr int kThreads       = 320;                    // TMA warp, MMA warp, eight epilogue warps
   static constexpr int kSmemBytes     = kStages * kStageBytes + kStagingBytes + 1024 + 256;
 };
+
+using PairCfg = PairCfgOf<false>;
 
 // What the epilogue of the pair kernel writes: the bf16 result, also the value before the activation, or fp32 partials.
 constexpr int kOutPlain = 0, kOutPre = 1, kOutPartial = 2;
@@ -521,9 +525,9 @@ template <bool kAMn, bool kBMn, int kOut>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg::kThreads, 1)
 GemmPairKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_pre, GemmParams p) {
-  using Cfg = PairCfg;
-  constexpr int BN = Cfg::kBN;
   constexpr bool kPre = kOut == kOutPre, kSplit = kOut == kOutPartial;
+  using Cfg = PairCfgOf<kPre>;
+  constexpr int BN = Cfg::kBN;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem    = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + Cfg::kStages * Cfg::kStageBytes;
@@ -651,7 +655,8 @@ GemmPairKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const int g = (warp - 2) >> 2;
     const int r = q * 32 + lane;           // row of this CTA's half tile
     const bool issuer = (warp == 2 || warp == 6) && lane == 0;
-    uint8_t* boxes = staging + g * 2 * Cfg::kBoxBytes;
+    uint8_t* boxes = staging + g * Cfg::kGroupBoxes * Cfg::kBoxBytes;
+    int slot = 0;  // next staging box
     int local = 0;
     bool ok = true;
     for (int tile = pair; tile < num_tiles; tile += pairs, ++local) {
@@ -691,13 +696,12 @@ GemmPairKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       }
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
-        uint8_t* box  = boxes + (kPre ? 0 : b) * Cfg::kBoxBytes;
-        uint8_t* pbox = boxes + Cfg::kBoxBytes;
-        // without a second output the boxes alternate, so the one written two boxes ago must have been read
-        if (issuer) {
-          if constexpr (kPre) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        }
+        uint8_t* box = boxes + slot * Cfg::kBoxBytes;
+        slot = slot + 1 == Cfg::kGroupBoxes ? 0 : slot + 1;
+        uint8_t* pbox = boxes + slot * Cfg::kBoxBytes;
+        if (kPre) slot = slot + 1 == Cfg::kGroupBoxes ? 0 : slot + 1;
+        // every store is a group of its own, and all but the newest have been read: two boxes of the three, one of the two
+        if (issuer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
         NamedBarSync(1 + g, 128);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -736,7 +740,10 @@ GemmPairKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         if (issuer) {
           if (ok && n0 + b * 64 < p.n && m0 < p.m) {
             TmaStoreOrAdd2D(&tmap_c, n0 + b * 64, m0, box, p.accumulate);
-            if (kPre) TmaStoreOrAdd2D(&tmap_pre, n0 + b * 64, m0, pbox, 0);
+            if (kPre) {
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              TmaStoreOrAdd2D(&tmap_pre, n0 + b * 64, m0, pbox, 0);
+            }
           }
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
@@ -755,50 +762,35 @@ GemmPairKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   }
 }
 
-// Sum of the partial products, then bias and activation as in the other epilogues: eight columns per `lanes` threads,
-// which take every lanes-th split each and add up by shuffles (with few outputs a thread per output leaves most SMs
-// idle: 512 x 128 from 37 splits took 11 us).  With `accumulate` the sum is added to what C holds.
+// Sum of the partial products in the order of the splits, then bias and activation as in the other epilogues: four
+// columns per thread, so that a warp reads 512 contiguous bytes of each share and small outputs still fill the SMs.  With
+// `accumulate` the sum is added to what C holds.
 __global__ void __launch_bounds__(256)
-GemmSplitSumKernel(GemmParams p, int lanes) {
-  const int vecs      = p.n / 8;
+GemmSplitSumKernel(GemmParams p) {
+  const int vecs      = p.n / 4;
   const int64_t total = static_cast<int64_t>(p.m) * vecs, plane = static_cast<int64_t>(p.m) * p.n;
-  const int64_t step  = static_cast<int64_t>(gridDim.x) * 256 / lanes;
-  const int64_t first = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) / lanes;
-  const int part      = threadIdx.x % lanes;
-  // whole warps run the same number of rounds, so that the shuffles below meet
-  for (int64_t i0 = first - (threadIdx.x & 31) / lanes; i0 < total; i0 += step) {
-    const int64_t i = i0 + (threadIdx.x & 31) / lanes;
-    const int64_t at  = i < total ? i : total - 1;
-    const int64_t row = at / vecs;
-    const int col     = static_cast<int>(at - row * vecs) * 8;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * 256) {
+    const int64_t row = i / vecs;
+    const int col     = static_cast<int>(i - row * vecs) * 4;
     const float* src  = p.partial + row * p.n + col;
-    float v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
-    for (int s = part; s < p.splits; s += lanes) {
-      const float4 a = *reinterpret_cast<const float4*>(src + s * plane), b = *reinterpret_cast<const float4*>(src + s * plane + 4);
+    for (int s = 0; s < p.splits; ++s) {
+      const float4 a = *reinterpret_cast<const float4*>(src + s * plane);
       v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-      v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
     }
-    for (int o = 1; o < lanes; o <<= 1)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-    if (i >= total || part != 0) continue;
-    float bv[8];
-    LoadBias8(p, col, bv);
     __nv_bfloat16* dst = p.c + row * p.ldc + col;
-    Vec16<__nv_bfloat16> o, pr;
-    if (p.accumulate) o = LoadVec(dst);
+    alignas(8) __nv_bfloat16 o[4], pr[4];
+    if (p.accumulate) *reinterpret_cast<uint2*>(o) = *reinterpret_cast<const uint2*>(dst);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float x = v[j] + bv[j];
-      pr.v[j] = __float2bfloat16_rn(x);
-      x       = GemmAct(x, p.act);
-      o.v[j]  = __float2bfloat16_rn(p.accumulate ? __bfloat162float(o.v[j]) + x : x);
+    for (int j = 0; j < 4; ++j) {
+      float x = v[j] + (p.bias ? __bfloat162float(p.bias[col + j]) : 0.f);
+      pr[j] = __float2bfloat16_rn(x);
+      x     = GemmAct(x, p.act);
+      o[j]  = __float2bfloat16_rn(p.accumulate ? __bfloat162float(o[j]) + x : x);
     }
-    if (p.pre) StoreVec(p.pre + row * p.ldc + col, pr);
-    StoreVec(dst, o);
+    if (p.pre) *reinterpret_cast<uint2*>(p.pre + row * p.ldc + col) = *reinterpret_cast<const uint2*>(pr);
+    *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
   }
 }
 
@@ -868,7 +860,7 @@ int LaunchGemmPersistent(const CUtensorMap& ta, const CUtensorMap& tb, const CUt
 template <bool kAMn, bool kBMn, int kOut>
 int LaunchPair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tp,
                const GemmParams& p, cudaStream_t s) {
-  using Cfg = PairCfg;
+  using Cfg = PairCfgOf<kOut == kOutPre>;
   static std::atomic<int> resident{0};
   int pairs = resident.load(std::memory_order_acquire);
   if (pairs == 0) {
@@ -899,11 +891,9 @@ template <bool kAMn, bool kBMn>
 int LaunchPairSplit(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t s) {
   int rc = LaunchPair<kAMn, kBMn, kOutPartial>(ta, tb, ta, ta, p, s);
   if (rc) return rc;
-  const int64_t vecs = static_cast<int64_t>(p.m) * (p.n / 8);
-  int lanes = 1;
-  while (lanes < 8 && lanes * 2 <= p.splits && vecs * lanes < static_cast<int64_t>(NumSMs()) * 1024) lanes *= 2;
-  const int64_t grid = std::min<int64_t>((vecs * lanes + 255) / 256, NumSMs() * 8);
-  GemmSplitSumKernel<<<static_cast<int>(grid), 256, 0, s>>>(p, lanes);
+  const int64_t vecs = static_cast<int64_t>(p.m) * (p.n / 4);
+  const int64_t grid = std::min<int64_t>((vecs + 255) / 256, NumSMs() * 8);
+  GemmSplitSumKernel<<<static_cast<int>(grid), 256, 0, s>>>(p);
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
