@@ -112,6 +112,19 @@ def test_conv3x3(n, h, w, cin, cout):
     assert base.K().tipsk_conv_status() == 0
 
 
+@pytest.mark.parametrize("n,h,w,cout,stride", [(2, 6, 7, 64, 1), (3, 20, 20, 256, 1), (9, 15, 13, 320, 2), (40, 70, 70, 64, 1)])
+def test_weight_gradient_of_64_channels_in_tap_groups(n, h, w, cout, stride):
+    from tips_b200.ops.conv import conv2d_wgrad
+    from tips_b200.ops import base
+    x = _rand(n, 64, h, w).contiguous(memory_format=torch.channels_last)
+    ho, wo = (h - 1) // stride + 1, (w - 1) // stride + 1
+    dy = _rand(n, cout, ho, wo, seed=1).contiguous(memory_format=torch.channels_last)
+    got = conv2d_wgrad(x, dy, (cout, 3, 3, 64), stride, 1)
+    ref = torch.nn.grad.conv2d_weight(x.double(), (cout, 64, 3, 3), dy.double(), stride=stride, padding=1)
+    assert base.K().tipsk_conv_status() == 0
+    _close(got, ref.permute(0, 2, 3, 1))
+
+
 @pytest.mark.parametrize("n,c,h,w", [(1, 8, 1, 1), (2, 8, 2, 3), (3, 72, 5, 8), (2, 64, 31, 33), (1, 2056, 4, 4)])
 def test_maxpool_edges(n, c, h, w):
     from tips_b200.ops.pool import max_pool_3x3_s2

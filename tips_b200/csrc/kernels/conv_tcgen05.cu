@@ -548,6 +548,7 @@ ConvHaloKernel(const __grid_constant__ HaloMaps maps, const __grid_constant__ Ha
             const uint32_t b_addr = SmemAddr(b_smem + slot * kBBytes);
             const uint64_t bdesc  = p.b_mn ? SmemDescMnSw128(b_addr, 8192) : SmemDescSw128(b_addr);
             if (ElectOne()) {
+              // one half after the other: alternating between them per MMA measured 120 us instead of 108
               for (int h = 0; h < halves; ++h) {
                 const uint64_t adesc = SmemDescSw128(a_addr + h * p.half_bytes + p.row_shift[t] * 128);
 #pragma unroll
@@ -717,6 +718,7 @@ struct WgradParams {
   int tw, th, tn;   // tw * th * tn is a multiple of 16, at most 128
   int cout, cin;
   int a_boxes;      // 64-channel boxes of dy to load per stage: 1 when cout <= 64 (rows 64..127 are then unused)
+  int group;        // taps per CTA: with 64 input channels the columns of a tile are several taps side by side
   ConvTap tap[kMaxTaps];  // kofs = first column of the tap inside a row of dw
 };
 
@@ -757,13 +759,14 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
   int id = blockIdx.x;
   const int cin_t  = id % p.cin_tiles;  id /= p.cin_tiles;
   const int cout_t = id % p.cout_tiles; id /= p.cout_tiles;
-  const ConvTap tap = p.tap[id];
+  const int tap0    = id * p.group;  // with group == 1 the one tap of this CTA
+  const int b_boxes = p.group == 1 ? BN / 64 : (p.taps - tap0 < p.group ? p.taps - tap0 : p.group);
   const int box_rows = p.tw * p.th * p.tn;
   const int k_tiles  = p.tiles_w * p.tiles_h * p.tiles_n;
   const int k_begin  = static_cast<int>(static_cast<int64_t>(k_tiles) * blockIdx.y / gridDim.y);
   const int k_end    = static_cast<int>(static_cast<int64_t>(k_tiles) * (blockIdx.y + 1) / gridDim.y);
   const int num_k    = k_end - k_begin;
-  const uint32_t stage_tx = static_cast<uint32_t>(box_rows) * 128u * (p.a_boxes + BN / 64);
+  const uint32_t stage_tx = static_cast<uint32_t>(box_rows) * 128u * (p.a_boxes + b_boxes);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::kStages; ++s) {
@@ -801,10 +804,11 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
         MbarExpectTx(&full_bar[s], stage_tx);
         for (int j = 0; j < p.a_boxes; ++j)
           TmaLoad4D(a_dst + j * Cfg::kBoxBytes, &maps.dy, cout_t * kBM * kMH + j * 64, w0, h0, n0, &full_bar[s]);
-#pragma unroll
-        for (int j = 0; j < BN / 64; ++j)
-          TmaLoad4D(b_dst + j * Cfg::kBoxBytes, &maps.x[tap.map], cin_t * BN + j * 64, w0 + tap.dw, h0 + tap.dh, n0,
-                    &full_bar[s]);
+        for (int j = 0; j < b_boxes; ++j) {
+          const ConvTap& tap = p.tap[p.group == 1 ? tap0 : tap0 + j];
+          TmaLoad4D(b_dst + j * Cfg::kBoxBytes, &maps.x[tap.map], p.group == 1 ? cin_t * BN + j * 64 : 0, w0 + tap.dw,
+                    h0 + tap.dh, n0, &full_bar[s]);
+        }
       }
     }
   } else if (warp == 1) {
@@ -850,9 +854,10 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
         uint32_t acc[32];
         TmemLoad32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(c * 32), acc);
         const int row  = (cout_t * kMH + c / (BN / 32)) * kBM + q * 32 + lane;  // accumulator c / (BN/32) = its half
-        const int col0 = cin_t * BN + (c % (BN / 32)) * 32;
-        if (row < p.cout && col0 < p.cin) {
-          float* dst = p.dw + static_cast<int64_t>(row) * p.ldw + tap.kofs + col0;
+        const int box  = (c % (BN / 32)) / 2;  // 64-column box: a channel block, or a tap of the group
+        const int col0 = p.group == 1 ? cin_t * BN + (c % (BN / 32)) * 32 : (c & 1) * 32;
+        if (row < p.cout && col0 < p.cin && box < b_boxes) {
+          float* dst = p.dw + static_cast<int64_t>(row) * p.ldw + p.tap[p.group == 1 ? tap0 : tap0 + box].kofs + col0;
 #pragma unroll
           for (int g = 0; g < 8; ++g) {
             asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + g * 4),
@@ -1132,7 +1137,7 @@ int LaunchWgrad(const WgradMaps& maps, const WgradParams& p, int splits, cudaStr
                                     Cfg::kSmemBytes));
     configured = true;
   }
-  dim3 grid(p.taps * p.cout_tiles * p.cin_tiles, splits);
+  dim3 grid(CeilDiv(p.taps, p.group) * p.cout_tiles * p.cin_tiles, splits);
   ConvWgradKernel<BN, kBoxRows, kMH><<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(maps, p);
   TIPSK_LAUNCH_CHECK();
   return 0;
@@ -1299,7 +1304,13 @@ int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, 
   WgradParams p{};
   p.taps = n_taps;
   for (int i = 0; i < n_taps; ++i) p.tap[i] = taps[i];
-  const int bn  = cin % 256 == 0 ? 256 : cin % 128 == 0 ? 128 : 64;
+  // With 64 input channels and several taps a tile takes up to four taps as its columns: dy is loaded once for all of
+  // them and the MMAs are 256 columns wide (stem, 64 images of 224 x 224: 117 -> 103 us).  The groups are even (nine taps:
+  // three groups of three, seven: four and three).
+  const int groups = CeilDiv(n_taps, 4);
+  const bool group = cin == 64 && n_taps > 1;
+  const int bn  = group || cin % 256 == 0 ? 256 : cin % 128 == 0 ? 128 : 64;
+  p.group = group ? CeilDiv(n_taps, groups) : 1;
   const Box box = PickBox(static_cast<int>(dyv.w), static_cast<int>(dyv.h), static_cast<int>(dyv.n), true,
                           bn == 256 ? 64 : 128);
   int rc = MapOf(&maps.dy, dyv, box);
@@ -1321,7 +1332,7 @@ int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, 
   // 14x14 and 7x7 convolutions, where it leaves too few CTAs).
   static const bool no_big = getenv("TIPS_WGRAD_NO_BM256") != nullptr;
   int mh = 1;
-  if (!no_big && bn == 256 && cout % 256 == 0) {
+  if (!no_big && !group && bn == 256 && cout % 256 == 0) {
     const int64_t kt    = static_cast<int64_t>(CeilDiv(dyv.w, box.tw)) * CeilDiv(dyv.h, box.th) * CeilDiv(dyv.n, box.tn);
     const int64_t base2 = static_cast<int64_t>(n_taps) * (cout / 256) * (cin / 256);
     const int64_t sp2   = std::max<int64_t>(1, 2 * NumSMs() / base2);
@@ -1336,7 +1347,7 @@ int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, 
   p.cout = cout; p.cin = cin;
   p.a_boxes = mh == 2 ? 4 : (cout <= 64 ? 1 : 2);
   const int64_t k_tiles = static_cast<int64_t>(p.tiles_w) * p.tiles_h * p.tiles_n;
-  const int base = p.taps * p.cout_tiles * p.cin_tiles;
+  const int base = CeilDiv(p.taps, p.group) * p.cout_tiles * p.cin_tiles;
   int splits = 2 * NumSMs() / base;  // one CTA per SM at a time: at most two full waves, no straggler wave
   if (splits > k_tiles) splits = static_cast<int>(k_tiles);
   if (splits < 1) splits = 1;

@@ -113,7 +113,7 @@ def _weight_gradient(x, dy, weight, stride, padding):
     """Gradient of `weight` in its own dtype.  A 1x1 convolution is a matrix product over the pixels: in bf16 it takes the
     GEMM's weight-gradient path, which rounds the fp32 sums once instead of leaving an fp32 copy to cast."""
     cout, r, _, cin = weight.shape
-    if r == 1 and stride == 1 and weight.dtype == torch.bfloat16:
+    if r == 1 and stride == 1 and weight.dtype == torch.bfloat16 and x.numel() >= 16 * cin:
         flat = lambda t: _nhwc(t).permute(0, 2, 3, 1).reshape(-1, t.shape[1])
         return linear_weight_grad(flat(dy), flat(x), weight.dtype).view(weight.shape).to(weight.dtype)
     return conv2d_wgrad(x, dy, tuple(weight.shape), stride, padding).to(weight.dtype)
