@@ -81,7 +81,7 @@ def test_split_contraction(m, n, k):
 # n, h, w, cin, cout: widths at both ends of the halo kernel's range, image heights that leave a short last unit, an odd
 # number of units, weights resident (64 -> 64) and streamed
 HALO = [(300, 2, 62, 64, 64), (43, 56, 56, 64, 64), (149, 28, 28, 128, 128), (75, 17, 28, 64, 192), (40, 31, 33, 128, 64),
-        (297, 9, 9, 64, 128), (601, 5, 24, 192, 64)]
+        (297, 9, 9, 64, 128), (601, 5, 24, 192, 64), (50, 55, 56, 64, 64), (149, 31, 33, 64, 64), (300, 5, 20, 64, 64)]
 
 
 @pytest.mark.parametrize("n,h,w,cin,cout", HALO)

@@ -416,9 +416,9 @@ constexpr int kHaloStages   = 2;    // halo boxes in flight, two halves each
 constexpr int kHaloMaxSlots = 12;
 constexpr int kHaloFixed    = 2 * kBM * 128 + 1024 /*alignment*/ + 512 /*barriers*/ + 4096 /*statistics*/;
 
-template <int BN>
 __global__ void __launch_bounds__(kConvThreads, 1)
 ConvHaloKernel(const __grid_constant__ HaloMaps maps, const __grid_constant__ HaloParams p) {
+  constexpr int BN        = 64;
   constexpr int kBBytes   = BN * kBK * 2;
   constexpr int kTmemCols = 4 * BN;  // two tiles of two halves
   extern __shared__ uint8_t smem_raw[];
@@ -698,6 +698,261 @@ ConvHaloKernel(const __grid_constant__ HaloMaps maps, const __grid_constant__ Ha
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(static_cast<uint32_t>(kTmemCols))
                  : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ the same for 64 -> 64 channels: two output rows per MMA
+// A 64-column MMA takes about as long as a 128-column one, so here the columns are the same 64 channels of two output rows,
+// h and h + 1.  Input row h - 1 + j reaches row h through filter row j and row h + 1 through filter row j - 1:
+//   j = 0  row h only      j = 1, 2  both, with the weights [W_j | W_(j-1)] side by side      j = 3  row h + 1 only
+// i.e. 12 operand shifts for 18 taps.  A unit is `rp` such row pairs; the odd and the even input rows are loaded as two
+// boxes (maps over every other row), in which one pair further is one box row further, so all pairs of a unit are the 128
+// rows of one MMA as above.  The weights stay in shared memory, filter rows in descending order for each column tap.
+// 256 images of 56 x 56: 62 us forward and data gradient, 108 with one output row per MMA.
+struct RowPairParams {
+  int32_t* error;
+  float* stat_sum;
+  float* stat_sq;
+  int accumulate, b_mn;
+  int pitch, rp, w, ho;
+  int units_h, units;
+  int box_bytes;           // shared memory of one box, a multiple of 1024
+  uint32_t box_tx;
+  int32_t kofs[9];         // first weight column of the tap (filter row r, column s) = (dh + 1, dw + 1), at r * 3 + s
+};
+
+struct RowPairMaps {
+  CUtensorMap odd, even, b;  // input rows 1, 3, .. and 0, 2, ..; weights
+  CUtensorMap c[2];          // output rows 0, 2, .. and 1, 3, ..
+};
+
+constexpr int kPairWeightBytes = 9 * 8192;
+
+__global__ void __launch_bounds__(kConvThreads, 1)
+ConvRowPairKernel(const __grid_constant__ RowPairMaps maps, const __grid_constant__ RowPairParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem    = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* b_smem  = smem + kHaloStages * 2 * p.box_bytes;
+  uint8_t* staging = b_smem + kPairWeightBytes;
+  uint64_t* a_full     = reinterpret_cast<uint64_t*>(staging + 2 * kBM * 128);
+  uint64_t* a_empty    = a_full + kHaloStages;
+  uint64_t* b_full     = a_empty + kHaloStages;
+  uint64_t* tmem_full  = b_full + 1;      // [2]
+  uint64_t* tmem_empty = tmem_full + 2;   // [2]
+  uint32_t* tmem_slot  = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kHaloStages; ++s) {
+      MbarInit(&a_full[s], 1);
+      MbarInit(&a_empty[s], 1);
+    }
+    MbarInit(b_full, 1);
+    for (int b = 0; b < 2; ++b) {
+      MbarInit(&tmem_full[b], 1);
+      MbarInit(&tmem_empty[b], 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(tmem_slot)), "r"(256u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  TcFenceBefore();
+  __syncthreads();
+  TcFenceAfter();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+
+  if (warp == 0) {
+    if (ElectOne()) {
+      MbarExpectTx(b_full, kPairWeightBytes);
+      for (int s = 0; s < 3; ++s)
+        for (int r = 0; r < 3; ++r) {
+          uint8_t* dst = b_smem + (s * 3 + 2 - r) * 8192;  // W_2, W_1, W_0
+          const int k0 = p.kofs[r * 3 + s];
+          TmaLoad2D(dst, &maps.b, k0, 0, b_full);  // one 64 x 64 box in either operand order
+        }
+      int it = 0;
+      for (int u = blockIdx.x; u < p.units; u += gridDim.x, ++it) {
+        const int s = it % kHaloStages;
+        if (!MbarWait(&a_empty[s], ((it / kHaloStages) & 1) ^ 1)) {
+          atomicExch(p.error, 1);
+          break;
+        }
+        const int pair0 = (u % p.units_h) * p.rp, n0 = u / p.units_h;  // first row pair: rows 2 * pair0, ..
+        uint8_t* dst = smem + s * 2 * p.box_bytes;
+        MbarExpectTx(&a_full[s], 2 * p.box_tx);
+        TmaLoad4D(dst, &maps.odd, 0, -1, pair0 - 1, n0, &a_full[s]);             // rows 2 * pair0 - 1, + 1, ..
+        TmaLoad4D(dst + p.box_bytes, &maps.even, 0, -1, pair0, n0, &a_full[s]);  // rows 2 * pair0, + 2, ..
+      }
+    }
+  } else if (warp == 1) {
+    {  // the whole warp walks the loop, one lane issues
+      const uint32_t base_desc = (1u << 4) | (1u << 7) | (1u << 10) | (p.b_mn ? (1u << 16) : 0u) |
+                                 (static_cast<uint32_t>(kBM >> 4) << 24);
+      const uint32_t idesc64 = base_desc | (8u << 17), idesc128 = base_desc | (16u << 17);
+      const uint64_t b_kstep = p.b_mn ? 128 : 2;
+      const uint32_t w_addr  = SmemAddr(b_smem);
+      int it  = 0;
+      bool ok = MbarWaitWarp(b_full, 0);
+      if (!ok && lane == 0) atomicExch(p.error, 5);
+      for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x, ++it) {
+        const int buf = it & 1, s = it % kHaloStages;
+        if (!MbarWaitWarp(&tmem_empty[buf], ((it >> 1) & 1) ^ 1)) {
+          if (lane == 0) atomicExch(p.error, 4);
+          break;
+        }
+        if (!MbarWaitWarp(&a_full[s], (it / kHaloStages) & 1)) {
+          if (lane == 0) atomicExch(p.error, 2);
+          break;
+        }
+        TcFenceAfter();
+        const uint32_t a_addr = SmemAddr(smem + s * 2 * p.box_bytes);
+        const uint32_t d      = tmem_base + static_cast<uint32_t>(buf * 128);
+        if (ElectOne()) {
+          // j = 1 first: it initialises both halves
+          for (int jj = 0; jj < 4; ++jj) {
+            const int j = jj == 0 ? 1 : jj == 1 ? 0 : jj;
+            const uint32_t a_row = a_addr + ((j & 1) ? p.box_bytes : 0) + (j >> 1) * p.pitch * 128;
+            const uint32_t idesc = (j == 1 || j == 2) ? idesc128 : idesc64;
+            const uint32_t d_j   = j == 3 ? d + 64 : d;
+            const int w_tile     = j == 0 ? 2 : j == 1 ? 1 : 0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const uint64_t adesc  = SmemDescSw128(a_row + c * 128);
+              const uint32_t b_addr = w_addr + (c * 3 + w_tile) * 8192;
+              const uint64_t bdesc  = p.b_mn ? SmemDescMnSw128(b_addr, 8192) : SmemDescSw128(b_addr);
+#pragma unroll
+              for (int k = 0; k < kBK / 16; ++k)
+                UmmaBf16(d_j, adesc + 2 * k, bdesc + b_kstep * k, idesc, (jj > 0 || c > 0 || k > 0) ? 1u : 0u);
+            }
+          }
+          UmmaCommit(&a_empty[s]);
+          UmmaCommit(&tmem_full[buf]);
+        }
+      }
+    }
+  } else if (warp < 6) {
+    const int q  = warp & 3;
+    const int r  = q * 32 + lane;
+    const int ph = r / p.pitch, pw = r % p.pitch;
+    const bool real = pw < p.w && ph < p.rp;
+    const int dst   = ph * p.w + pw;
+    const int bar_threads = p.stat_sum != nullptr ? 256 : 128;
+    int it  = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < p.units; u += gridDim.x, ++it) {
+      const int buf = it & 1;
+      if (ok && !MbarWait(&tmem_full[buf], (it >> 1) & 1)) {
+        if (lane == 0) atomicExch(p.error, 3);
+        ok = false;
+      }
+      TcFenceAfter();
+#pragma unroll 1
+      for (int b = 0; b < 2; ++b) {  // output row parity, one staging box each
+        uint8_t* box = staging + b * (kBM * 128);
+        const uint32_t tsrc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * 128 + b * 64);
+        uint32_t acc[2][32];
+        if (ok) {
+          TmemLoad32Async(tsrc, acc[0]);
+          TmemLoad32Async(tsrc + 32, acc[1]);
+        }
+        if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        NamedBarSync(1, bar_threads);
+        if (ok) {
+          TmemLoadWait(acc[0]);
+          TmemLoadWait(acc[1]);
+          if (real) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+              alignas(16) __nv_bfloat16 o[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16_rn(__uint_as_float(acc[g >> 2][(g & 3) * 8 + j]));
+              *reinterpret_cast<uint4*>(box + dst * 128 + ((g ^ (dst & 7)) << 4)) = *reinterpret_cast<uint4*>(o);
+            }
+          }
+          if (b == 1) {
+            TcFenceBefore();
+            __syncwarp();
+            if (lane == 0) MbarArrive(&tmem_empty[buf]);
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        NamedBarSync(1, bar_threads);
+        if (warp == 2 && lane == 0) {
+          const int pair0 = (u % p.units_h) * p.rp, n0 = u / p.units_h;
+          if (ok && 2 * pair0 + b < p.ho) {
+            if (p.accumulate) TmaReduceAdd4D(&maps.c[b], 0, 0, pair0, n0, box);
+            else TmaStore4D(&maps.c[b], 0, 0, pair0, n0, box);
+          }
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+    }
+    if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  } else if (p.stat_sum != nullptr) {
+    // Statistics of the staged boxes: rp rows of w pixels, of one parity, fewer in the last unit of an image.
+    float* partial   = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a_full) + 512);  // [2][4 warps][64][2]
+    const int st     = threadIdx.x - 192;
+    const int chunk  = st & 7;
+    const int rg     = st >> 3;
+    const int sw     = st >> 5;
+    for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+      const int h0 = (u % p.units_h) * p.rp * 2;
+#pragma unroll 1
+      for (int b = 0; b < 2; ++b) {
+        const int left = (p.ho - h0 - b + 1) / 2;  // rows of this parity from the unit's first on
+        const int rows = (left < 0 ? 0 : left < p.rp ? left : p.rp) * p.w;
+        NamedBarSync(1, 256);
+        NamedBarSync(1, 256);
+        const uint8_t* box = staging + b * (kBM * 128);
+        float s1[8], s2[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s1[j] = s2[j] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = rg + 16 * i;
+          if (row < rows) {
+            const uint4 v = *reinterpret_cast<const uint4*>(box + row * 128 + ((chunk ^ (row & 7)) << 4));
+            const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = __bfloat1622float2(hv[j]);
+              s1[2 * j] += f.x; s2[2 * j] += f.x * f.x;
+              s1[2 * j + 1] += f.y; s2[2 * j + 1] += f.y * f.y;
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], 8);
+          s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], 16);
+          s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 8);
+          s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 16);
+        }
+        float* P = partial + b * (4 * 64 * 2);
+        if (lane < 8) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            P[(sw * 64 + lane * 8 + j) * 2]     = s1[j];
+            P[(sw * 64 + lane * 8 + j) * 2 + 1] = s2[j];
+          }
+        }
+        NamedBarSync(2, 128);
+        const int col = st & 63, which = st >> 6;
+        const float tot = P[(0 * 64 + col) * 2 + which] + P[(1 * 64 + col) * 2 + which] +
+                          P[(2 * 64 + col) * 2 + which] + P[(3 * 64 + col) * 2 + which];
+        atomicAdd((which ? p.stat_sq : p.stat_sum) + col, tot);
+      }
+    }
+  }
+  TcFenceBefore();
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(256u) : "memory");
   }
 }
 
@@ -1150,29 +1405,84 @@ int HaloRows(int w, int h) {
 }
 int HaloHalfBytes(int w, int th) { return CeilDiv(static_cast<int64_t>(w + 2) * (th + 2) * 128, 1024) * 1024; }
 
-// Whether the halo kernel should run a 3x3 / stride 1 convolution into `w_rows` channels of [n, h, w] pixels: narrow
-// output tiles (a 256-channel tile does enough work per loaded byte), and units that fill the 128 rows of an MMA about
-// as well as the tap kernel's boxes do.
+// Whether the halo kernel should run a 3x3 / stride 1 convolution into `w_rows` channels of [n, h, w] pixels: 64-column
+// output tiles (128 columns do enough work per loaded byte: 128 images of 28 x 28, 128 -> 128, 54 us against 44 with a box
+// per tap), and units that fill the 128 rows of an MMA about as well as the tap kernel's boxes do.
 bool PreferHalo(int n, int h, int w, int w_rows) {
   const int th = HaloRows(w, h);
-  if (th == 0 || w_rows % 256 == 0) return false;
+  if (th == 0 || w_rows % 128 == 0) return false;
   const int64_t units = static_cast<int64_t>(n) * CeilDiv(h, th);
   const Box box       = PickBox(w, h, n, false);
   const int64_t boxes = static_cast<int64_t>(CeilDiv(w, box.tw)) * CeilDiv(h, box.th) * CeilDiv(n, box.tn);
   return units >= 2 * NumSMs() && units * 10 <= boxes * 12;
 }
 
-template <int BN>
+// Whether the row-pair kernel should run a 3x3 / stride 1 convolution of 64 into 64 channels: the rule of the halo kernel
+// for units of two MMA tiles.
+bool PreferRowPairs(int n, int h, int w, int cin, int w_rows) {
+  if (cin != 64 || w_rows != 64 || w + 2 > kBM || h < 2) return false;
+  const int rp        = std::min(kBM / (w + 2), (h + 1) / 2);
+  const int64_t units = static_cast<int64_t>(n) * CeilDiv(h, 2 * rp);
+  const Box box       = PickBox(w, h, n, false);
+  const int64_t boxes = static_cast<int64_t>(CeilDiv(w, box.tw)) * CeilDiv(h, box.th) * CeilDiv(n, box.tn);
+  return units >= NumSMs() && 2 * units * 10 <= boxes * 12;
+}
+
+View RowPhaseView(const View& v, int parity) {  // every other row of a full view
+  return View{static_cast<const char*>(v.base) + parity * v.sh * 2, v.c, v.w, (v.h - parity + 1) / 2, v.n, v.sw, 2 * v.sh,
+              v.sn};
+}
+
+int RunRowPairs(const View& in, const ConvTap* taps, const void* weights, int64_t w_cols, const View& out, float* stat_sum,
+                float* stat_sq, cudaStream_t s, int accumulate, int b_mn) {
+  const int w = static_cast<int>(out.w), h = static_cast<int>(out.h), n = static_cast<int>(out.n);
+  RowPairMaps maps;
+  RowPairParams p{};
+  p.pitch = w + 2; p.w = w; p.ho = h;
+  p.rp      = std::min(kBM / p.pitch, (h + 1) / 2);
+  p.units_h = CeilDiv(h, 2 * p.rp);
+  p.units   = n * p.units_h;
+  p.box_tx    = static_cast<uint32_t>(p.pitch) * (p.rp + 1) * 128u;
+  p.box_bytes = CeilDiv(p.box_tx, 1024) * 1024;
+  int rc = MapOf(&maps.odd, RowPhaseView(in, 1), Box{p.pitch, p.rp + 1, 1});
+  if (rc) return rc;
+  rc = MapOf(&maps.even, RowPhaseView(in, 0), Box{p.pitch, p.rp + 1, 1});
+  if (rc) return rc;
+  rc = MakeTmap2D(&maps.b, weights, 64, w_cols, 64);
+  if (rc) return rc;
+  for (int b = 0; b < 2; ++b) {
+    rc = MapOf(&maps.c[b], RowPhaseView(out, b), Box{w, p.rp, 1});
+    if (rc) return rc;
+  }
+  p.error = ConvErrorWord();
+  TIPSK_REQUIRE(p.error != nullptr, "conv: cannot allocate the error word");
+  p.stat_sum = stat_sum;
+  p.stat_sq  = stat_sq;
+  p.accumulate = accumulate;
+  p.b_mn       = b_mn;
+  for (int t = 0; t < 9; ++t) p.kofs[(taps[t].dh + 1) * 3 + taps[t].dw + 1] = taps[t].kofs;
+  static bool configured = false;
+  if (!configured) {
+    TIPSK_CUDA(cudaFuncSetAttribute(ConvRowPairKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
+    configured = true;
+  }
+  const int smem = kHaloStages * 2 * p.box_bytes + kPairWeightBytes + kHaloFixed;
+  TIPSK_REQUIRE(smem <= kMaxSmemBytes, "conv: the row-pair boxes do not fit in shared memory");
+  ConvRowPairKernel<<<std::min(p.units, NumSMs()), kConvThreads, smem, s>>>(maps, p);
+  TIPSK_LAUNCH_CHECK();
+  return 0;
+}
+
 int LaunchHalo(const HaloMaps& maps, const HaloParams& p, cudaStream_t s) {
   static bool configured = false;
   if (!configured) {
-    TIPSK_CUDA(cudaFuncSetAttribute(ConvHaloKernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
+    TIPSK_CUDA(cudaFuncSetAttribute(ConvHaloKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
     configured = true;
   }
   const int64_t tiles = static_cast<int64_t>((p.units + 1) / 2) * p.n_tiles;
   const int grid = static_cast<int>(std::min<int64_t>(tiles, NumSMs()));
-  const int smem = kHaloStages * 2 * p.half_bytes + p.b_slots * BN * 128 + kHaloFixed;
-  ConvHaloKernel<BN><<<grid, kConvThreads, smem, s>>>(maps, p);
+  const int smem = kHaloStages * 2 * p.half_bytes + p.b_slots * 64 * 128 + kHaloFixed;
+  ConvHaloKernel<<<grid, kConvThreads, smem, s>>>(maps, p);
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
@@ -1182,8 +1492,10 @@ int RunHalo(const View& in, const ConvTap* taps, int cin, const void* weights, i
             const View& out, float* stat_sum, float* stat_sq, cudaStream_t s, int accumulate, int b_mn) {
   TIPSK_REQUIRE(cin % 64 == 0 && w_rows % 64 == 0, "conv: channel counts must be multiples of 64");
   const int w = static_cast<int>(out.w), h = static_cast<int>(out.h), n = static_cast<int>(out.n);
+  if (PreferRowPairs(n, h, w, cin, w_rows))
+    return RunRowPairs(in, taps, weights, w_cols, out, stat_sum, stat_sq, s, accumulate, b_mn);
   const int th = HaloRows(w, h);
-  const int bn = w_rows % 128 == 0 ? 128 : 64;
+  constexpr int bn = 64;
   HaloMaps maps;
   HaloParams p{};
   int rc = MapOf(&maps.a, in, Box{w + 2, th + 2, 1});
@@ -1214,7 +1526,7 @@ int RunHalo(const View& in, const ConvTap* taps, int cin, const void* weights, i
     p.row_shift[t] = (taps[t].dh + 1) * p.pitch + taps[t].dw + 1;
     p.kofs[t]      = taps[t].kofs;
   }
-  return bn == 64 ? LaunchHalo<64>(maps, p, s) : LaunchHalo<128>(maps, p, s);
+  return LaunchHalo(maps, p, s);
 }
 
 // Runs the tap kernel: out[view_out pixel, co] = sum over taps and 64-channel blocks.
