@@ -1019,7 +1019,12 @@ int tipsk_gemm_bf16_nn(const void* a, const void* b, void* c, int m, int n, int 
 /* Whether the pair kernel is the one to run a product of this kind (the kinds of tipsk_gemm_bf16_split). */
 int tipsk_gemm_prefers_pair(int kind, int m, int n, int k) {
   if (m < 64 || n < 64 || n % 8 != 0 || k <= 0) return 0;
-  return (kind == 2 || PreferPair(m, n, k)) ? 1 : 0;
+  if (kind != 2) return PreferPair(m, n, k) ? 1 : 0;
+  // Weight gradients: the alternative spreads K over all SMs and costs 10 us plus a fill and a cast (3.5 us); a pair walks
+  // its K alone, 8 us plus 0.28 us per 64 rows, unless K is long enough to be split.  Measured with two tiles: 13 : 17 us at
+  // K = 2000, 21 : 26 at 3920; with 16 tiles 32 : 20 at 2048.
+  const int64_t tiles = static_cast<int64_t>(CeilDiv(m, 2 * kBM)) * CeilDiv(n, PairCfg::kBN);
+  return (k <= 1024 || tiles >= 12 || tipsk_gemm_splits(m, n, k) > 1) ? 1 : 0;
 }
 
 /* Number of K splits with which tipsk_gemm_bf16_split should run the product (1: use the unsplit entry points). */
