@@ -172,13 +172,80 @@ LnBwdKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restri
   }
 }
 
-// Backward with a GROUP of cols / 8 threads per row: each thread owns 8 consecutive columns (one 16-byte vector), so the
+// Backward with one BLOCK per row: each thread owns 8 consecutive columns (one 16-byte vector), so the per-column
+// dgamma / dbeta accumulators are 16 registers instead of 64 and many more rows are in flight per SM than with a
+// warp per row.  The two row sums go through shared memory (one barrier per row, double-buffered).
+template <typename T>
+__global__ void __launch_bounds__(1024)
+LnBwdBlockRowKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
+                    const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
+                    float* __restrict__ dgamma_partial, float* __restrict__ dbeta_partial, int64_t rows, int cols) {
+  constexpr int N = 8;
+  __shared__ float red[2][2][32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
+  float gm[N], dg[N], db[N];
+  {
+    const Vec16<T> g = LoadVec(gamma + t * N);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      gm[i] = ToFloat<T>(g.v[i]);
+      dg[i] = db[i] = 0.f;
+    }
+  }
+  const float inv_cols = 1.f / static_cast<float>(cols);
+  int it = 0;
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, ++it) {
+    const float mu = mean[r], rs = rstd[r];
+    const Vec16<T> qx = LoadVec(x + r * cols + t * N), qd = LoadVec(dy + r * cols + t * N);
+    float xh[N], dyg[N];
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      xh[i] = (ToFloat<T>(qx.v[i]) - mu) * rs;
+      const float d = ToFloat<T>(qd.v[i]);
+      dyg[i] = d * gm[i];
+      s1 += dyg[i];
+      s2 += dyg[i] * xh[i];
+      dg[i] += d * xh[i];
+      db[i] += d;
+    }
+    s1 = WarpSum(s1);
+    s2 = WarpSum(s2);
+    const int p = it & 1;
+    if (lane == 0) {
+      red[p][0][warp] = s1;
+      red[p][1][warp] = s2;
+    }
+    __syncthreads();
+    s1 = s2 = 0.f;
+    for (int w = 0; w < nwarps; ++w) {
+      s1 += red[p][0][w];
+      s2 += red[p][1][w];
+    }
+    s1 *= inv_cols;
+    s2 *= inv_cols;
+    Vec16<T> o;
+#pragma unroll
+    for (int i = 0; i < N; ++i) o.v[i] = FromFloat<T>(rs * (dyg[i] - s1 - xh[i] * s2));
+    StoreVec(dx + r * cols + t * N, o);
+  }
+  float* pg = dgamma_partial + static_cast<int64_t>(blockIdx.x) * cols + t * N;
+  float* pb = dbeta_partial + static_cast<int64_t>(blockIdx.x) * cols + t * N;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    pg[i] = dg[i];
+    pb[i] = db[i];
+  }
+}
+
+// The same with a GROUP of cols / 8 threads per row, for shorter inputs: each thread owns 8 consecutive columns (one 16-byte vector), so the
 // per-column dgamma / dbeta accumulators are 16 registers instead of 64.  A block is as many groups as 768 threads and
 // the 15 named barriers allow; every group walks its own rows, with the next row's loads in flight while it reduces the
 // current one (the two row sums go through shared memory, one barrier of the group per row, double-buffered), and the
 // groups' column sums are added up in shared memory at the end.  One block per SM: with eight small blocks per SM a block
 // of the 4096 x 1024 gradient of an encoder layer had 3.5 rows, and its partial rows were 40 % of the traffic.  That
-// shape: 16 -> 13 us, and the sum of the partial rows 8 -> 3 us.
+// shape: 16 -> 13 us, and the sum of the partial rows 8 -> 3 us.  From 16384 rows on the partial rows are 10 % or less,
+// and the 1024 threads per SM of the small blocks keep more bytes in flight.
 constexpr int kLnGroupThreads = 768;  // with 1024 the accumulators and the prefetched row spill
 
 inline int LnGroups(int group) {
@@ -306,7 +373,9 @@ LnReducePartialsKernel(const float* __restrict__ pg, const float* __restrict__ p
   }
 }
 
-// Rows of whole warps of 16-byte vectors in a 16-bit type, one group of threads each.
+constexpr int64_t kLnLongRows = 16384;
+
+// Rows of whole warps of 16-byte vectors in a 16-bit type, one group of threads (or one block) each.
 bool LnUsesGroups(int cols, int dtype) { return dtype != kF32 && cols % 256 == 0 && cols / 8 <= 1024; }
 
 int LnGrid(int64_t rows) {
@@ -378,6 +447,7 @@ int tipsk_ln_bwd_partials(int64_t rows, int cols) {
 /* The number of partial rows with which tipsk_ln_bwd should be called for this dtype. */
 int tipsk_ln_bwd_partial_rows(int64_t rows, int cols, int dtype) {
   if (!LnUsesGroups(cols, dtype)) return LnGrid(rows);
+  if (rows >= kLnLongRows) return LnGrid(rows);
   const int64_t blocks = (rows + LnGroups(cols / 8) - 1) / LnGroups(cols / 8);
   return static_cast<int>(blocks < NumSMs() ? (blocks < 1 ? 1 : blocks) : NumSMs());
 }
@@ -390,6 +460,19 @@ int tipsk_ln_bwd(const void* dy, const void* x, const void* gamma, const float* 
   TIPSK_REQUIRE(partial_rows == LnGrid(rows) || partial_rows == tipsk_ln_bwd_partial_rows(rows, cols, dtype),
                 "layer norm backward: wrong number of partial rows");
   cudaStream_t s    = static_cast<cudaStream_t>(stream);
+  if (LnUsesGroups(cols, dtype) && rows >= kLnLongRows) {
+    if (dtype == kBF16)
+      LnBwdBlockRowKernel<__nv_bfloat16><<<partial_rows, cols / 8, 0, s>>>(
+          static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+          static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma_partial,
+          dbeta_partial, rows, cols);
+    else
+      LnBwdBlockRowKernel<__half><<<partial_rows, cols / 8, 0, s>>>(
+          static_cast<const __half*>(dy), static_cast<const __half*>(x), static_cast<const __half*>(gamma), mean, rstd,
+          static_cast<__half*>(dx), dgamma_partial, dbeta_partial, rows, cols);
+    TIPSK_LAUNCH_CHECK();
+    return 0;
+  }
   if (LnUsesGroups(cols, dtype)) {
     const int threads  = LnGroups(cols / 8) * (cols / 8);
     const size_t bytes = sizeof(float) * 2 * cols;  // at most 64 KB, above the default limit from 5120 columns on
