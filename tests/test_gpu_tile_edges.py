@@ -166,7 +166,8 @@ def test_pack_many_tensors(src, flat, accumulate):
 
 
 @pytest.mark.parametrize("dtype", [BF16, torch.float32])
-@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 4096), (5, 4104), (700, 1000), (4, 30522), (3, 32768), (3, 32776)])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 4096), (5, 4104), (700, 1000), (4, 30522), (3, 32768), (3, 32776), (4097, 64), (5000, 10),
+                                       (3, 1024), (3, 1032), (3, 2056), (3, 16392)])
 def test_softmax_cross_entropy_rows(dtype, rows, cols):
     from tips_b200.ops.pointwise import softmax_cross_entropy
     z = _rand(rows, cols, scale=3.0, dtype=dtype).requires_grad_()

@@ -4,6 +4,8 @@
 // softmax cross-entropy (loss, count and gradient per row in one kernel).
 // The reference leaves all of this to TensorFlow ops; here they are fused so
 // that each activation tensor is touched once per direction.
+#include <algorithm>
+
 #include "kernels/common.cuh"
 #include "kernels/tips_kernels.h"
 
@@ -364,11 +366,26 @@ __device__ __forceinline__ float BlockReduce(float v, bool is_max, float* scratc
   return r;
 }
 
-// What a row's loss and gradient are multiplied with: `scale`, or with `mean` one over the rows that count (every block
-// counts the labels itself, a few kilobytes from L2, so that the gradient is written finished in the same pass).
+// Adds the number of labels that count to *count.
+__global__ void __launch_bounds__(256)
+CountLabelsKernel(const int64_t* __restrict__ labels, int64_t rows, int cols, int64_t ignore_index, float* __restrict__ count) {
+  int mine = 0;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; r < rows; r += static_cast<int64_t>(gridDim.x) * 256) {
+    const int64_t l = labels[r];
+    mine += !(l == ignore_index || l < 0 || l >= cols);
+  }
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(count, static_cast<float>(mine));
+}
+
+// What a row's loss and gradient are multiplied with: `scale`, or with `mean` one over the rows that count, so that the
+// gradient is written finished in the same pass.  Up to kXentSelfCount rows every block counts the labels itself, a few
+// kilobytes from L2; beyond, CountLabelsKernel has done it and `counted` holds the number.
+constexpr int kXentSelfCount = 4096;
 __device__ __forceinline__ float XentScale(const int64_t* __restrict__ labels, int64_t rows, int cols,
-                                           int64_t ignore_index, float scale, int mean) {
+                                           int64_t ignore_index, float scale, int mean, const float* counted) {
   if (!mean) return scale;
+  if (rows > kXentSelfCount) return 1.f / fmaxf(*counted, 1.f);
   __shared__ int total;
   if (threadIdx.x == 0) total = 0;
   __syncthreads();
@@ -390,7 +407,7 @@ SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labe
                   float* __restrict__ count, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index,
                   float grad_scale, int mean) {
   __shared__ float scratch[8];
-  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean);
+  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean, count);
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const T* row        = logits + r * cols;
     const int64_t label = labels[r];
@@ -410,7 +427,7 @@ SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labe
     if (threadIdx.x == 0) {
       const float loss = lse - ToFloat<T>(row[label]);
       atomicAdd(loss_sum, mean ? loss * scale : loss);
-      if (count) atomicAdd(count, 1.f);
+      if (count && !mean) atomicAdd(count, 1.f);
     }
     if (dlogits) {
       const float inv = 1.f / se;
@@ -423,19 +440,18 @@ SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labe
   }
 }
 
-// Rows of whole 16-byte vectors, up to 512 * VPT of them: one block of 512 threads per row, which it reads from HBM once
+// Rows of whole 16-byte vectors, up to kThreads * VPT of them: one block per row, which it reads from HBM once
 // into VPT vectors per thread and keeps for all three sweeps (maximum, sum of exponentials, gradient).  Bound by HBM
 // (one read, one write) and, close behind, by two exponentials per logit.  1232 x 30528 bf16 (150 MB): 46 us; the general
 // form, which reads scalars from L2 in each sweep, 221 us.
-constexpr int kXentThreads = 512;
-
+template <int kThreads>
 __device__ __forceinline__ float XentReduce(float v, bool is_max, float* scratch) {
   v = is_max ? WarpMax(v) : WarpSum(v);
   if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
   __syncthreads();
   float o = scratch[0];
 #pragma unroll
-  for (int w = 1; w < kXentThreads / 32; ++w) o = is_max ? fmaxf(o, scratch[w]) : o + scratch[w];
+  for (int w = 1; w < kThreads / 32; ++w) o = is_max ? fmaxf(o, scratch[w]) : o + scratch[w];
   return o;  // the caller alternates between two scratch arrays, so no second barrier is needed
 }
 
@@ -450,14 +466,14 @@ __device__ __forceinline__ void KeepPacked(Vec16<T> (&v)[VPT]) {
   }
 }
 
-template <typename T, int VPT>
-__global__ void __launch_bounds__(kXentThreads, 2)
+template <typename T, int VPT, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads)
 SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ loss_sum,
                      float* __restrict__ count, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index,
                      float grad_scale, int mean) {
   constexpr int N = 16 / sizeof(T);
-  __shared__ float smax[kXentThreads / 32], ssum[kXentThreads / 32];
-  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean);
+  __shared__ float smax[kThreads / 32], ssum[kThreads / 32];
+  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean, count);
   const int nvec    = cols / N;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const T* row        = logits + r * cols;
@@ -468,46 +484,46 @@ SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ l
         Vec16<T> z;
 #pragma unroll
         for (int j = 0; j < N; ++j) z.v[j] = FromFloat<T>(0.f);
-        for (int i = threadIdx.x; i < nvec; i += kXentThreads) StoreVec(drow + i * N, z);
+        for (int i = threadIdx.x; i < nvec; i += kThreads) StoreVec(drow + i * N, z);
       }
       continue;
     }
     Vec16<T> v[VPT];
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
-      const int i = k * kXentThreads + threadIdx.x;
+      const int i = k * kThreads + threadIdx.x;
       if (i < nvec) v[k] = LoadVec(row + i * N);
       else *reinterpret_cast<uint4*>(&v[k]) = make_uint4(0, 0, 0, 0);
     }
     float mx = -INFINITY;
 #pragma unroll
     for (int k = 0; k < VPT; ++k)
-      if (k * kXentThreads + threadIdx.x < nvec) {
+      if (k * kThreads + threadIdx.x < nvec) {
 #pragma unroll
         for (int j = 0; j < N; ++j) mx = fmaxf(mx, ToFloat<T>(v[k].v[j]));
       }
-    mx = XentReduce(mx, true, smax);
+    mx = XentReduce<kThreads>(mx, true, smax);
     KeepPacked(v);
     float se = 0.f;
 #pragma unroll
     for (int k = 0; k < VPT; ++k)
-      if (k * kXentThreads + threadIdx.x < nvec) {
+      if (k * kThreads + threadIdx.x < nvec) {
 #pragma unroll
         for (int j = 0; j < N; ++j) se += __expf(ToFloat<T>(v[k].v[j]) - mx);
       }
-    se = XentReduce(se, false, ssum);
+    se = XentReduce<kThreads>(se, false, ssum);
     KeepPacked(v);
     if (threadIdx.x == 0) {
       const float loss = mx + logf(se) - ToFloat<T>(row[label]);
       atomicAdd(loss_sum, mean ? loss * scale : loss);
-      if (count) atomicAdd(count, 1.f);
+      if (count && !mean) atomicAdd(count, 1.f);
     }
     if (drow) {
       const float inv = 1.f / se;
       const int lvec = static_cast<int>(label) / N, lj = static_cast<int>(label) % N;
 #pragma unroll
       for (int k = 0; k < VPT; ++k) {
-        const int i = k * kXentThreads + threadIdx.x;
+        const int i = k * kThreads + threadIdx.x;
         if (i < nvec) {
           Vec16<T> o;
 #pragma unroll
@@ -710,15 +726,25 @@ static int SoftmaxXentImpl(const void* logits, const int64_t* labels, float* los
   const int n        = 16 / static_cast<int>(DTypeSize(dtype));
   const bool aligned = cols % n == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0 &&
                        reinterpret_cast<uintptr_t>(dlogits) % 16 == 0;
-  const int per_thread = CeilDiv(cols / n, kXentThreads);
-  if (aligned && per_thread <= 8) {
-    const int grid = static_cast<int>(rows < NumSMs() * 2 ? rows : NumSMs() * 2);
+  const int vecs = cols / n;
+  if (mean && rows > kXentSelfCount) {
+    const int64_t blocks = std::min<int64_t>((rows + 1023) / 1024, NumSMs());
+    CountLabelsKernel<<<static_cast<int>(blocks), 256, 0, s>>>(labels, rows, cols, ignore_index, count);
+    TIPSK_LAUNCH_CHECK();
+  }
+  if (aligned && vecs <= 4096) {
+    // short rows take small blocks, of which many share an SM: a row is a chain of two reductions (forward and backward of
+    // 65536 x 1000 bf16 187 us, 433 with the general form and a separate scale; 65536 x 64 140 and 257)
+    const int threads = vecs <= 512 ? 128 : vecs <= 2048 ? 256 : 512;
+    const int64_t cap = static_cast<int64_t>(NumSMs()) * (threads == 128 ? 12 : 1024 / threads);
+    const int grid    = static_cast<int>(rows < cap ? rows : cap);
     EPI_DISPATCH(dtype, {
-      auto* kernel = per_thread <= 1   ? SoftmaxXentRowKernel<T, 1>
-                     : per_thread <= 2 ? SoftmaxXentRowKernel<T, 2>
-                     : per_thread <= 4 ? SoftmaxXentRowKernel<T, 4>
-                                       : SoftmaxXentRowKernel<T, 8>;
-      kernel<<<grid, kXentThreads, 0, s>>>(static_cast<const T*>(logits), labels, loss_sum, count,
+      auto* kernel = vecs <= 128    ? SoftmaxXentRowKernel<T, 1, 128>
+                     : vecs <= 256  ? SoftmaxXentRowKernel<T, 2, 128>
+                     : vecs <= 512  ? SoftmaxXentRowKernel<T, 4, 128>
+                     : vecs <= 2048 ? SoftmaxXentRowKernel<T, 8, 256>
+                                    : SoftmaxXentRowKernel<T, 8, 512>;
+      kernel<<<grid, threads, 0, s>>>(static_cast<const T*>(logits), labels, loss_sum, count,
                                            static_cast<T*>(dlogits), rows, cols, ignore_index, grad_scale, mean);
     });
     TIPSK_LAUNCH_CHECK();
@@ -738,10 +764,12 @@ int tipsk_softmax_xent(const void* logits, const int64_t* labels, float* loss_su
   return SoftmaxXentImpl(logits, labels, loss_sum, count, dlogits, rows, cols, ignore_index, grad_scale, 0, dtype, stream);
 }
 
-/* Mean over the rows whose label counts: *loss (zeroed by the caller) receives the mean loss, dlogits its gradient. */
-int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, void* dlogits, int64_t rows, int cols,
-                            int64_t ignore_index, int dtype, void* stream) {
-  return SoftmaxXentImpl(logits, labels, loss, nullptr, dlogits, rows, cols, ignore_index, 1.f, 1, dtype, stream);
+/* Mean over the rows whose label counts: *loss receives the mean loss, dlogits its gradient.  *count is scratch, needed
+ * beyond 4096 rows.  Both are zeroed by the caller. */
+int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, float* count, void* dlogits,
+                            int64_t rows, int cols, int64_t ignore_index, int dtype, void* stream) {
+  TIPSK_REQUIRE(count != nullptr || rows <= kXentSelfCount, "softmax_xent_mean: a row counter is needed");
+  return SoftmaxXentImpl(logits, labels, loss, count, dlogits, rows, cols, ignore_index, 1.f, 1, dtype, stream);
 }
 
 /* y = x * s, s one fp32 value on the device. */

@@ -114,8 +114,8 @@ int tipsk_sigmoid_bce(const void* logits, const float* targets, float* loss_sum,
  * loss_sum / count accumulated into fp32 scalars, dlogits = (softmax - onehot) * scale. */
 int tipsk_softmax_xent(const void* logits, const int64_t* labels, float* loss_sum, float* count, void* dlogits,
                        int64_t rows, int cols, int64_t ignore_index, float grad_scale, int dtype, void* stream);
-int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, void* dlogits, int64_t rows, int cols,
-                            int64_t ignore_index, int dtype, void* stream);
+int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, float* count, void* dlogits,
+                            int64_t rows, int cols, int64_t ignore_index, int dtype, void* stream);
 int tipsk_scale_by(const void* x, const float* s, void* y, int64_t n, int dtype, void* stream);
 
 /* ---- NVLink collectives (comm.cu, comm_executor.cu) ----

@@ -182,9 +182,10 @@ class _SoftmaxXentFn(torch.autograd.Function):
         rows = z.numel() // cols
         lab = labels.contiguous().view(-1)
         loss = torch.zeros((), dtype=torch.float32, device=z.device)
+        count = torch.zeros((), dtype=torch.float32, device=z.device) if rows > 4096 else None  # the kernel's scratch
         dz = torch.empty_like(z)
-        base.check(base.K().tipsk_softmax_xent_mean(z.data_ptr(), lab.data_ptr(), loss.data_ptr(), dz.data_ptr(), rows,
-                                                    cols, ignore_index, base.code(z), base.stream()), "softmax_xent")
+        base.check(base.K().tipsk_softmax_xent_mean(z.data_ptr(), lab.data_ptr(), loss.data_ptr(), base.ptr(count),
+                                                    dz.data_ptr(), rows, cols, ignore_index, base.code(z), base.stream()), "softmax_xent")
         ctx.save_for_backward(dz)  # the gradient of the mean loss
         return loss
 
