@@ -181,8 +181,32 @@ def test_softmax_cross_entropy_rows(dtype, rows, cols):
     ref = F.cross_entropy(zr, labels, ignore_index=-100)
     (ref * 3.0).backward()
     assert torch.allclose(loss.double(), ref.detach(), rtol=1e-5)
-    # rounded once as the gradient of the mean, once after the factor 3: twice 2^-8, their product, and fp32 terms
+    # rounded once as softmax - onehot, once after the factors: twice 2^-8, their product, and fp32 terms
     _close(z.grad, zr.grad, slack=2.0 ** -18, rel=2.0 ** -7 + 2.0 ** -13)
+
+
+# the row kernel and, with more than 4096 vectors per row or a ragged length, the general one; labels counted by every block and once
+@pytest.mark.parametrize("rows,cols,up", [(1232, 30528, 1024.0), (1232, 30528, 65536.0), (300, 30522, 65536.0), (4097, 4096, 65536.0),
+                                          (40, 32776, 65536.0)])
+def test_softmax_cross_entropy_fp16_loss_scale(rows, cols, up):
+    """Off-label entries of the mean's gradient are below fp16's range until the loss scale is applied."""
+    from tips_b200.ops.pointwise import softmax_cross_entropy
+    z = _rand(rows, cols, scale=1.0, dtype=torch.float16).requires_grad_()
+    labels = torch.randint(0, cols, (rows,), device=DEV, generator=torch.Generator(device=DEV).manual_seed(1))
+    labels[3] = -100
+    (softmax_cross_entropy(z, labels) * up).backward()
+    zr = z.detach().double()
+    ref = torch.softmax(zr, 1)
+    ref[torch.arange(rows, device=DEV), labels.clamp(min=0)] -= 1.0
+    ref[3] = 0.0
+    ref *= up / (rows - 1)
+    # stored once as softmax - onehot and once more after the factor up / (rows - 1): two roundings of 2^-11 each plus fp32 terms,
+    # or half a subnormal unit, 2^-25, each
+    bound = ref.abs() * (2.0 ** -10 + 2.0 ** -13) + (up / (rows - 1) + 1.0) * 2.0 ** -25
+    bad = (z.grad.double() - ref).abs() > bound
+    assert not bool(bad.any()), float((z.grad.double() - ref).abs().max())
+    off = z.grad[0].index_select(0, (labels[0] + 1 + torch.arange(cols - 1, device=DEV)) % cols)
+    assert float((off == 0).float().mean()) < 0.01
 
 
 def test_softmax_cross_entropy_without_counted_rows():

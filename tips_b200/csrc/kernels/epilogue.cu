@@ -378,14 +378,19 @@ CountLabelsKernel(const int64_t* __restrict__ labels, int64_t rows, int cols, in
   if ((threadIdx.x & 31) == 0 && mine) atomicAdd(count, static_cast<float>(mine));
 }
 
-// What a row's loss and gradient are multiplied with: `scale`, or with `mean` one over the rows that count, so that the
-// gradient is written finished in the same pass.  Up to kXentSelfCount rows every block counts the labels itself, a few
-// kilobytes from L2; beyond, CountLabelsKernel has done it and `counted` holds the number.
+// One over the number of rows that count: what a row adds to the mean loss is scaled with it here, the gradient only in
+// the backward pass, by ScaleByKernel.  The gradient is stored as softmax - onehot, because in fp16 that divided by the
+// rows of a batch is zero for most classes of a large vocabulary, and no loss scale brings it back.  Up to
+// kXentSelfCount rows every block counts the labels itself, a few kilobytes from L2; beyond, CountLabelsKernel has done
+// it.  norm[0] is its counter, norm[1] receives the result.
 constexpr int kXentSelfCount = 4096;
 __device__ __forceinline__ float XentScale(const int64_t* __restrict__ labels, int64_t rows, int cols,
-                                           int64_t ignore_index, float scale, int mean, const float* counted) {
-  if (!mean) return scale;
-  if (rows > kXentSelfCount) return 1.f / fmaxf(*counted, 1.f);
+                                           int64_t ignore_index, float* __restrict__ norm) {
+  if (rows > kXentSelfCount) {
+    const float scale = 1.f / fmaxf(norm[0], 1.f);
+    if (blockIdx.x == 0 && threadIdx.x == 0) norm[1] = scale;
+    return scale;
+  }
   __shared__ int total;
   if (threadIdx.x == 0) total = 0;
   __syncthreads();
@@ -397,17 +402,18 @@ __device__ __forceinline__ float XentScale(const int64_t* __restrict__ labels, i
   mine = __reduce_add_sync(0xffffffffu, mine);
   if ((threadIdx.x & 31) == 0) atomicAdd(&total, mine);
   __syncthreads();
-  return 1.f / static_cast<float>(total > 1 ? total : 1);
+  const float scale = 1.f / static_cast<float>(total > 1 ? total : 1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) norm[1] = scale;
+  return scale;
 }
 
 // General form: any row length and alignment.
 template <typename T>
 __global__ void __launch_bounds__(256)
-SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ loss_sum,
-                  float* __restrict__ count, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index,
-                  float grad_scale, int mean) {
+SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ loss,
+                  float* __restrict__ norm, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index) {
   __shared__ float scratch[8];
-  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean, count);
+  const float scale = XentScale(labels, rows, cols, ignore_index, norm);
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const T* row        = logits + r * cols;
     const int64_t label = labels[r];
@@ -424,17 +430,13 @@ SoftmaxXentKernel(const T* __restrict__ logits, const int64_t* __restrict__ labe
     for (int c = threadIdx.x; c < cols; c += blockDim.x) se += __expf(ToFloat<T>(row[c]) - mx);
     se = BlockReduce(se, false, scratch);
     const float lse = mx + logf(se);
-    if (threadIdx.x == 0) {
-      const float loss = lse - ToFloat<T>(row[label]);
-      atomicAdd(loss_sum, mean ? loss * scale : loss);
-      if (count && !mean) atomicAdd(count, 1.f);
-    }
+    if (threadIdx.x == 0) atomicAdd(loss, (lse - ToFloat<T>(row[label])) * scale);
     if (dlogits) {
       const float inv = 1.f / se;
       for (int c = threadIdx.x; c < cols; c += blockDim.x) {
         float p = __expf(ToFloat<T>(row[c]) - mx) * inv;
         if (c == label) p -= 1.f;
-        dlogits[r * cols + c] = FromFloat<T>(p * scale);
+        dlogits[r * cols + c] = FromFloat<T>(p);
       }
     }
   }
@@ -468,12 +470,11 @@ __device__ __forceinline__ void KeepPacked(Vec16<T> (&v)[VPT]) {
 
 template <typename T, int VPT, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
-SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ loss_sum,
-                     float* __restrict__ count, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index,
-                     float grad_scale, int mean) {
+SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ loss,
+                     float* __restrict__ norm, T* __restrict__ dlogits, int64_t rows, int cols, int64_t ignore_index) {
   constexpr int N = 16 / sizeof(T);
   __shared__ float smax[kThreads / 32], ssum[kThreads / 32];
-  const float scale = XentScale(labels, rows, cols, ignore_index, grad_scale, mean, count);
+  const float scale = XentScale(labels, rows, cols, ignore_index, norm);
   const int nvec    = cols / N;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
     const T* row        = logits + r * cols;
@@ -513,11 +514,7 @@ SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ l
       }
     se = XentReduce<kThreads>(se, false, ssum);
     KeepPacked(v);
-    if (threadIdx.x == 0) {
-      const float loss = mx + logf(se) - ToFloat<T>(row[label]);
-      atomicAdd(loss_sum, mean ? loss * scale : loss);
-      if (count && !mean) atomicAdd(count, 1.f);
-    }
+    if (threadIdx.x == 0) atomicAdd(loss, (mx + logf(se) - ToFloat<T>(row[label])) * scale);
     if (drow) {
       const float inv = 1.f / se;
       const int lvec = static_cast<int>(label) / N, lj = static_cast<int>(label) % N;
@@ -530,7 +527,7 @@ SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ l
           for (int j = 0; j < N; ++j) {
             float p = __expf(ToFloat<T>(v[k].v[j]) - mx) * inv;
             if (i == lvec && j == lj) p -= 1.f;
-            o.v[j] = FromFloat<T>(p * scale);
+            o.v[j] = FromFloat<T>(p);
           }
           StoreVec(drow + i * N, o);
         }
@@ -541,12 +538,13 @@ SoftmaxXentRowKernel(const T* __restrict__ logits, const int64_t* __restrict__ l
   }
 }
 
-// y = x * s for a scalar s on the device: 37.6 M bf16 values (150 MB) 25 us, 6 TB/s.
+// y = x * (s * t) for two scalars on the device: 37.6 M bf16 values (150 MB) 25 us, 6 TB/s.
 template <typename T>
 __global__ void __launch_bounds__(256)
-ScaleByKernel(const T* __restrict__ x, const float* __restrict__ s, T* __restrict__ y, int64_t n) {
+ScaleByKernel(const T* __restrict__ x, const float* __restrict__ s, const float* __restrict__ t, T* __restrict__ y,
+              int64_t n) {
   constexpr int N = 16 / sizeof(T), U = 4;
-  const float f = *s;
+  const float f = *s * *t;
   const int64_t vecs = n / N, stride = static_cast<int64_t>(gridDim.x) * 256;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < vecs; i += U * stride) {
     Vec16<T> v[U];
@@ -716,9 +714,11 @@ int tipsk_embed_sum_bwd(const int64_t* ids, const void* dx, void* dtok, void* dp
   return 0;
 }
 
-static int SoftmaxXentImpl(const void* logits, const int64_t* labels, float* loss_sum, float* count, void* dlogits,
-                           int64_t rows, int cols, int64_t ignore_index, float grad_scale, int mean, int dtype,
-                           void* stream) {
+/* Mean over the rows whose label counts: *loss, zeroed by the caller, receives the mean loss, dlogits softmax - onehot,
+ * and norm[1] one over the number of rows that count, by which the gradient of the mean is still to be multiplied
+ * (tipsk_scale_by).  norm[0] is scratch. */
+int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, float* norm, void* dlogits,
+                            int64_t rows, int cols, int64_t ignore_index, int dtype, void* stream) {
   if (rows <= 0 || cols <= 0) return 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // The row kernel needs whole, aligned 16-byte vectors and at most eight of them per thread (it is the faster one
@@ -727,9 +727,10 @@ static int SoftmaxXentImpl(const void* logits, const int64_t* labels, float* los
   const bool aligned = cols % n == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0 &&
                        reinterpret_cast<uintptr_t>(dlogits) % 16 == 0;
   const int vecs = cols / n;
-  if (mean && rows > kXentSelfCount) {
+  if (rows > kXentSelfCount) {
+    TIPSK_CUDA(cudaMemsetAsync(norm, 0, sizeof(float), s));
     const int64_t blocks = std::min<int64_t>((rows + 1023) / 1024, NumSMs());
-    CountLabelsKernel<<<static_cast<int>(blocks), 256, 0, s>>>(labels, rows, cols, ignore_index, count);
+    CountLabelsKernel<<<static_cast<int>(blocks), 256, 0, s>>>(labels, rows, cols, ignore_index, norm);
     TIPSK_LAUNCH_CHECK();
   }
   if (aligned && vecs <= 4096) {
@@ -744,36 +745,23 @@ static int SoftmaxXentImpl(const void* logits, const int64_t* labels, float* los
                      : vecs <= 512  ? SoftmaxXentRowKernel<T, 4, 128>
                      : vecs <= 2048 ? SoftmaxXentRowKernel<T, 8, 256>
                                     : SoftmaxXentRowKernel<T, 8, 512>;
-      kernel<<<grid, threads, 0, s>>>(static_cast<const T*>(logits), labels, loss_sum, count,
-                                           static_cast<T*>(dlogits), rows, cols, ignore_index, grad_scale, mean);
+      kernel<<<grid, threads, 0, s>>>(static_cast<const T*>(logits), labels, loss, norm, static_cast<T*>(dlogits), rows,
+                                      cols, ignore_index);
     });
     TIPSK_LAUNCH_CHECK();
     return 0;
   }
   const int grid = static_cast<int>(rows < NumSMs() * 8 ? rows : NumSMs() * 8);
   EPI_DISPATCH(dtype, {
-    SoftmaxXentKernel<T><<<grid, 256, 0, s>>>(static_cast<const T*>(logits), labels, loss_sum, count,
-                                              static_cast<T*>(dlogits), rows, cols, ignore_index, grad_scale, mean);
+    SoftmaxXentKernel<T><<<grid, 256, 0, s>>>(static_cast<const T*>(logits), labels, loss, norm,
+                                              static_cast<T*>(dlogits), rows, cols, ignore_index);
   });
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
 
-int tipsk_softmax_xent(const void* logits, const int64_t* labels, float* loss_sum, float* count, void* dlogits,
-                       int64_t rows, int cols, int64_t ignore_index, float grad_scale, int dtype, void* stream) {
-  return SoftmaxXentImpl(logits, labels, loss_sum, count, dlogits, rows, cols, ignore_index, grad_scale, 0, dtype, stream);
-}
-
-/* Mean over the rows whose label counts: *loss receives the mean loss, dlogits its gradient.  *count is scratch, needed
- * beyond 4096 rows.  Both are zeroed by the caller. */
-int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, float* count, void* dlogits,
-                            int64_t rows, int cols, int64_t ignore_index, int dtype, void* stream) {
-  TIPSK_REQUIRE(count != nullptr || rows <= kXentSelfCount, "softmax_xent_mean: a row counter is needed");
-  return SoftmaxXentImpl(logits, labels, loss, count, dlogits, rows, cols, ignore_index, 1.f, 1, dtype, stream);
-}
-
-/* y = x * s, s one fp32 value on the device. */
-int tipsk_scale_by(const void* x, const float* s, void* y, int64_t n, int dtype, void* stream) {
+/* y = x * (s * t), s and t one fp32 value each on the device. */
+int tipsk_scale_by(const void* x, const float* s, const float* t, void* y, int64_t n, int dtype, void* stream) {
   if (n <= 0) return 0;
   TIPSK_REQUIRE(reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0,
                 "scale_by: 16-byte aligned buffers are required");
@@ -783,7 +771,7 @@ int tipsk_scale_by(const void* x, const float* s, void* y, int64_t n, int dtype,
   if (grid > NumSMs() * 8) grid = NumSMs() * 8;
   if (grid < 1) grid = 1;
   EPI_DISPATCH(dtype, {
-    ScaleByKernel<T><<<static_cast<int>(grid), 256, 0, st>>>(static_cast<const T*>(x), s, static_cast<T*>(y), n);
+    ScaleByKernel<T><<<static_cast<int>(grid), 256, 0, st>>>(static_cast<const T*>(x), s, t, static_cast<T*>(y), n);
   });
   TIPSK_LAUNCH_CHECK();
   return 0;

@@ -110,13 +110,11 @@ int tipsk_embed_sum_bwd(const int64_t* ids, const void* dx, void* dtok, void* dp
                         int hidden, int64_t vocab, int dtype, void* stream);
 int tipsk_sigmoid_bce(const void* logits, const float* targets, float* loss_sum, void* dlogits, int64_t n,
                       float grad_scale, int dtype, void* stream);
-/* Softmax cross entropy over [rows, cols] with int64 labels (ignore_index skipped):
- * loss_sum / count accumulated into fp32 scalars, dlogits = (softmax - onehot) * scale. */
-int tipsk_softmax_xent(const void* logits, const int64_t* labels, float* loss_sum, float* count, void* dlogits,
-                       int64_t rows, int cols, int64_t ignore_index, float grad_scale, int dtype, void* stream);
-int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, float* count, void* dlogits,
+/* Softmax cross entropy over [rows, cols] with int64 labels (ignore_index skipped): *loss (zeroed by the caller) = mean
+ * over the rows that count, dlogits = softmax - onehot, norm[1] = 1 / number of rows that count (norm[0] is scratch). */
+int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* loss, float* norm, void* dlogits,
                             int64_t rows, int cols, int64_t ignore_index, int dtype, void* stream);
-int tipsk_scale_by(const void* x, const float* s, void* y, int64_t n, int dtype, void* stream);
+int tipsk_scale_by(const void* x, const float* s, const float* t, void* y, int64_t n, int dtype, void* stream);
 
 /* ---- NVLink collectives (comm.cu, comm_executor.cu) ----
  * A "window" is a buffer of identical size on every rank, mapped into every process

@@ -182,22 +182,25 @@ class _SoftmaxXentFn(torch.autograd.Function):
         rows = z.numel() // cols
         lab = labels.contiguous().view(-1)
         loss = torch.zeros((), dtype=torch.float32, device=z.device)
-        count = torch.zeros((), dtype=torch.float32, device=z.device) if rows > 4096 else None  # the kernel's scratch
+        norm = torch.empty(2, dtype=torch.float32, device=z.device)  # the kernel's counter, 1 / rows that count
         dz = torch.empty_like(z)
-        base.check(base.K().tipsk_softmax_xent_mean(z.data_ptr(), lab.data_ptr(), loss.data_ptr(), base.ptr(count),
-                                                    dz.data_ptr(), rows, cols, ignore_index, base.code(z), base.stream()), "softmax_xent")
-        ctx.save_for_backward(dz)  # the gradient of the mean loss
+        base.check(base.K().tipsk_softmax_xent_mean(z.data_ptr(), lab.data_ptr(), loss.data_ptr(), norm.data_ptr(),
+                                                    dz.data_ptr(), rows, cols, ignore_index, base.code(z), base.stream()),
+                   "softmax_xent")
+        # dz = softmax - onehot: the mean's factor and the upstream gradient are applied together, in fp32, so that a
+        # loss scale reaches an fp16 gradient before it is rounded
+        ctx.save_for_backward(dz, norm)
         return loss
 
     @staticmethod
     def backward(ctx, dloss):
-        (dz,) = ctx.saved_tensors
+        dz, norm = ctx.saved_tensors
         if torch.is_grad_enabled() or not base.plain(dloss):  # create_graph, or gradients batched by vmap
-            return dz * dloss.to(dz.dtype), None, None
+            return dz * (dloss * norm[1]).to(dz.dtype), None, None
         up = dloss.to(torch.float32)
         out = torch.empty_like(dz)
-        base.check(base.K().tipsk_scale_by(dz.data_ptr(), up.data_ptr(), out.data_ptr(), dz.numel(), base.code(dz),
-                                           base.stream()), "scale_by")
+        base.check(base.K().tipsk_scale_by(dz.data_ptr(), up.data_ptr(), norm.data_ptr() + 4, out.data_ptr(), dz.numel(),
+                                           base.code(dz), base.stream()), "scale_by")
         return out, None, None
 
 
