@@ -209,6 +209,29 @@ def test_softmax_cross_entropy_fp16_loss_scale(rows, cols, up):
     assert float((off == 0).float().mean()) < 0.01
 
 
+@pytest.mark.parametrize("dtype", [BF16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows", [1, 7])
+def test_softmax_cross_entropy_create_graph(dtype, rows):
+    """A loss scale of 65536 is infinite in fp16; the gradient that it leads to is not."""
+    from tips_b200.ops.pointwise import softmax_cross_entropy
+    z = _rand(rows, 264, dtype=dtype).requires_grad_()
+    labels = torch.arange(rows, device=DEV)
+    up = torch.full((), 65536.0, device=DEV, requires_grad=True)
+    (g,) = torch.autograd.grad(softmax_cross_entropy(z, labels), z, up, create_graph=True)
+    zr = z.detach().double()
+    ref = torch.softmax(zr, 1) - F.one_hot(labels, 264)
+    ref1 = ref * 65536.0 / rows
+    eps = {BF16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -20}[dtype]
+    top = float(torch.finfo(dtype).max)
+    ok = ref1.abs() < top * (1 - 2 * eps)  # one row's label entry, -65536 (1 - p), is in fp16's range but for the rounding
+    assert bool(ok[:, rows:].all())
+    # two roundings to the type (softmax - onehot, the product) and fp32 terms
+    assert bool(((g.detach().double() - ref1).abs() <= ref1.abs() * (2 * eps + 2.0 ** -13) + 2.0 ** -9)[ok].all())
+    (gu,) = torch.autograd.grad(g[:, rows:].float().sum(), up)  # the gradient is linear in the upstream factor
+    want = ref[:, rows:].sum() / rows
+    assert abs(float(gu) - float(want)) <= float(ref[:, rows:].abs().sum()) / rows * (2 * eps + 2.0 ** -13)
+
+
 def test_softmax_cross_entropy_without_counted_rows():
     from tips_b200.ops.pointwise import softmax_cross_entropy
     z = _rand(4, 64).requires_grad_()

@@ -196,7 +196,7 @@ class _SoftmaxXentFn(torch.autograd.Function):
     def backward(ctx, dloss):
         dz, norm = ctx.saved_tensors
         if torch.is_grad_enabled() or not base.plain(dloss):  # create_graph, or gradients batched by vmap
-            return dz * (dloss * norm[1]).to(dz.dtype), None, None
+            return (dz.float() * (dloss.float() * norm[1])).to(dz.dtype), None, None  # a loss scale may exceed fp16
         up = dloss.to(torch.float32)
         out = torch.empty_like(dz)
         base.check(base.K().tipsk_scale_by(dz.data_ptr(), up.data_ptr(), norm.data_ptr() + 4, out.data_ptr(), dz.numel(),
