@@ -232,6 +232,27 @@ def test_softmax_cross_entropy_create_graph(dtype, rows):
     assert abs(float(gu) - float(want)) <= float(ref[:, rows:].abs().sum()) / rows * (2 * eps + 2.0 ** -13)
 
 
+@pytest.mark.parametrize("layout", ["offset", "strided"])
+def test_softmax_cross_entropy_saved_tensor_hooks(layout):
+    """Hooks may hand the saved gradient back anywhere in memory."""
+    from tips_b200.ops.pointwise import softmax_cross_entropy
+
+    def unpack(t):
+        if t.dim() != 2:
+            return t
+        if layout == "offset":
+            return torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)[1:].view(t.shape).copy_(t)
+        return torch.empty(t.shape[0], 2 * t.shape[1], dtype=t.dtype, device=DEV)[:, ::2].copy_(t)
+
+    z = _rand(9, 64).requires_grad_()
+    labels = torch.arange(9, device=DEV)
+    (want,) = torch.autograd.grad(softmax_cross_entropy(z, labels), z)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        loss = softmax_cross_entropy(z, labels)
+    (got,) = torch.autograd.grad(loss, z)
+    assert torch.equal(got, want)
+
+
 def test_softmax_cross_entropy_without_counted_rows():
     from tips_b200.ops.pointwise import softmax_cross_entropy
     z = _rand(4, 64).requires_grad_()

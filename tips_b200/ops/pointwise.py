@@ -195,7 +195,8 @@ class _SoftmaxXentFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         dz, norm = ctx.saved_tensors
-        if torch.is_grad_enabled() or not base.plain(dloss):  # create_graph, or gradients batched by vmap
+        # create_graph, gradients batched by vmap, or a saved-tensor hook that changed the layout
+        if torch.is_grad_enabled() or not base.plain(dloss) or not dz.is_contiguous() or dz.data_ptr() % 16:
             return (dz.float() * (dloss.float() * norm[1])).to(dz.dtype), None, None  # a loss scale may exceed fp16
         up = dloss.to(torch.float32)
         out = torch.empty_like(dz)
