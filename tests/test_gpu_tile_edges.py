@@ -112,6 +112,34 @@ def test_conv3x3(n, h, w, cin, cout):
     assert base.K().tipsk_conv_status() == 0
 
 
+# a last unit of one row, of all its rows, and images one unit high; the pitch beyond the width by 2, 4 and 8 pixels
+@pytest.mark.parametrize("n,h,w", [(100, 17, 28), (50, 56, 56), (300, 3, 62), (43, 55, 56)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_weight_gradient_of_non_finite_pixels(n, h, w, value):
+    """A pixel that is not finite reaches exactly the taps that read it."""
+    from tips_b200.ops.conv import conv2d_wgrad
+    from tips_b200.ops import base
+    x = _rand(n, 64, h, w)
+    # first and last column, last row, a corner, inside; each in a channel of its own
+    for ch, (i, j) in enumerate([(1, 0), (h // 2, w - 1), (h - 1, w // 2), (h - 1, w - 1), (h // 2, w // 2), (0, 0)]):
+        x[n // 2, 9 * ch, i, j] = value
+        x[n - 1, 9 * ch, i, j] = -value
+    x = x.contiguous(memory_format=torch.channels_last)
+    dy = _rand(n, 64, h, w, seed=1).contiguous(memory_format=torch.channels_last)
+    got = conv2d_wgrad(x, dy, (64, 3, 3, 64), 1, 1).permute(0, 3, 1, 2).double()
+    xd, dyd = x.double(), dy.double()
+    for r in range(3):
+        for s in range(3):
+            i0, i1, j0, j1 = max(0, 1 - r), h - max(0, r - 1), max(0, 1 - s), w - max(0, s - 1)
+            part = dyd[:, :, i0:i1, j0:j1].permute(1, 0, 2, 3).reshape(64, -1)
+            ref = part @ xd[:, :, i0 + r - 1:i1 + r - 1, j0 + s - 1:j1 + s - 1].permute(0, 2, 3, 1).reshape(-1, 64)
+            fin = torch.isfinite(ref)
+            assert bool(fin.any()) and torch.equal(got[:, :, r, s].isfinite(), fin), (r, s)
+            assert torch.equal(got[:, :, r, s].isinf(), ref.isinf())
+            _close(torch.where(fin, got[:, :, r, s], 0.0), torch.where(fin, ref, 0.0))
+    assert base.K().tipsk_conv_status() == 0
+
+
 @pytest.mark.parametrize("n,h,w,cout,stride", [(2, 6, 7, 64, 1), (3, 20, 20, 256, 1), (9, 15, 13, 320, 2), (40, 70, 70, 64, 1)])
 def test_weight_gradient_of_64_channels_in_tap_groups(n, h, w, cout, stride):
     from tips_b200.ops.conv import conv2d_wgrad
