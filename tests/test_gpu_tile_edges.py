@@ -78,16 +78,20 @@ def test_split_contraction(m, n, k):
     assert gemm_status() == 0
 
 
-# n, h, w, cin, cout: widths at both ends of the halo kernel's range, image heights that leave a short last unit, an odd
-# number of units, weights resident (64 -> 64) and streamed
-HALO = [(300, 2, 62, 64, 64), (43, 56, 56, 64, 64), (149, 28, 28, 128, 128), (75, 17, 28, 64, 192), (40, 31, 33, 128, 64),
-        (297, 9, 9, 64, 128), (601, 5, 24, 192, 64), (50, 55, 56, 64, 64), (149, 31, 33, 64, 64), (300, 5, 20, 64, 64)]
+# n, h, w, cin, cout, and which kernel that is (1: two output rows per MMA).  Widths at both ends of the row-pair kernel's
+# range, odd heights, a short last unit, one row pair per unit, more units than SMs and one more; the tap kernel beside the
+# lines of the rule and with several channel blocks and output tiles.
+CONV3X3 = [(43, 56, 56, 64, 64, 1), (50, 55, 56, 64, 64, 1), (74, 8, 62, 64, 64, 1), (149, 31, 33, 64, 64, 1), (150, 9, 28, 64, 64, 1),
+           (75, 28, 28, 64, 64, 1), (300, 2, 62, 64, 64, 1), (300, 12, 3, 64, 64, 0), (150, 9, 9, 64, 64, 0), (149, 5, 63, 64, 64, 0),
+           (36, 8, 62, 64, 64, 0), (149, 28, 28, 128, 128, 0), (75, 17, 28, 64, 192, 0), (43, 56, 56, 192, 64, 0),
+           (297, 9, 9, 64, 128, 0), (601, 5, 24, 192, 64, 0)]
 
 
-@pytest.mark.parametrize("n,h,w,cin,cout", HALO)
-def test_conv3x3(n, h, w, cin, cout):
+@pytest.mark.parametrize("n,h,w,cin,cout,path", CONV3X3)
+def test_conv3x3(n, h, w, cin, cout, path):
     from tips_b200.ops.conv import conv2d_dgrad, conv2d_forward, conv2d_wgrad
     from tips_b200.ops import base
+    assert base.K().tipsk_conv2d_path(0, n, h, w, cin, cout) == path == base.K().tipsk_conv2d_path(1, n, h, w, cin, cout)
     x = _rand(n, cin, h, w).contiguous(memory_format=torch.channels_last)
     wgt = _rand(cout, 3, 3, cin, scale=1.0 / (3 * cin ** 0.5), seed=1)
     dy = _rand(n, cout, h, w, seed=2).contiguous(memory_format=torch.channels_last)

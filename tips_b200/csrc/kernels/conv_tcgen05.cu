@@ -383,332 +383,18 @@ ConvTapsKernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   }
 }
 
-// ------------------------------------------------------------------ 3x3, stride 1: one halo box for all nine taps
-// With few channels the tap kernel above is bound by its loads: it fetches the same box of pixels nine times, 16 KB for
-// 128 x 64 x 64 products.  Here a unit of `th` full image rows is loaded once per 64-channel block together with its
-// border, [th + 2] rows x [w + 2] pixels (zero fill outside the image), and the nine taps read it at nine offsets: pixel
-// (h, w) of the unit is row h * pitch + w of the box, pitch = w + 2, so a tap is a shift by whole 128-byte rows and the
-// MMA's A operand starts (dh + 1) * pitch + dw + 1 rows further.  The swizzle is a function of the shared-memory address,
-// so a shifted start needs no other descriptor.  Rows w .. pitch - 1 of every image row are computed and dropped
-// (112 of 128 rows are real pixels at 56 x 56 and 28 x 28).  A tile is two units that share every weight block.  Bound by
-// the rate of 64-column MMAs.  64 -> 64 channels, 256 images of 56 x 56: 111 us forward and data gradient, 157 with a box per
-// tap (59 GFLOP).
-struct HaloParams {
-  int32_t* error;
-  float* stat_sum;
-  float* stat_sq;
-  int cblocks, accumulate, b_mn;
-  int b_slots, b_resident;       // weight blocks in shared memory; 1: all 9 * cblocks of them stay for the whole kernel
-  int pitch, th, w, ho;          // box pitch in pixels, image rows of a unit, image width and height
-  int units_h, units;            // units per image, units in all
-  int half_bytes;                // shared memory of one halo box, a multiple of 1024
-  uint32_t box_tx;               // bytes that the TMA unit delivers for it
-  int cout, n_tiles;
-  int row_shift[kMaxTaps];       // first A row of the tap
-  int32_t kofs[kMaxTaps];        // first column of the tap in the weight matrix
-};
-
-struct HaloMaps {
-  CUtensorMap a, b, c;
-};
-
-constexpr int kHaloStages   = 2;    // halo boxes in flight, two halves each
-constexpr int kHaloMaxSlots = 12;
-constexpr int kHaloFixed    = 2 * kBM * 128 + 1024 /*alignment*/ + 512 /*barriers*/ + 4096 /*statistics*/;
-
-__global__ void __launch_bounds__(kConvThreads, 1)
-ConvHaloKernel(const __grid_constant__ HaloMaps maps, const __grid_constant__ HaloParams p) {
-  constexpr int BN        = 64;
-  constexpr int kBBytes   = BN * kBK * 2;
-  constexpr int kTmemCols = 4 * BN;  // two tiles of two halves
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem    = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* b_smem  = smem + kHaloStages * 2 * p.half_bytes;
-  uint8_t* staging = b_smem + p.b_slots * kBBytes;
-  uint64_t* a_full     = reinterpret_cast<uint64_t*>(staging + 2 * kBM * 128);
-  uint64_t* a_empty    = a_full + kHaloStages;
-  uint64_t* b_full     = a_empty + kHaloStages;
-  uint64_t* b_empty    = b_full + kHaloMaxSlots;
-  uint64_t* tmem_full  = b_empty + kHaloMaxSlots;  // [2]
-  uint64_t* tmem_empty = tmem_full + 2;            // [2]
-  uint32_t* tmem_slot  = reinterpret_cast<uint32_t*>(tmem_empty + 2);
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int m_tiles   = (p.units + 1) / 2;
-  const int num_tiles = m_tiles * p.n_tiles;
-  const int num_k     = 9 * p.cblocks;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kHaloStages; ++s) {
-      MbarInit(&a_full[s], 1);
-      MbarInit(&a_empty[s], 1);
-    }
-    for (int s = 0; s < p.b_slots; ++s) {
-      MbarInit(&b_full[s], 1);
-      MbarInit(&b_empty[s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      MbarInit(&tmem_full[b], 1);
-      MbarInit(&tmem_empty[b], 4);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(tmem_slot)),
-                 "r"(static_cast<uint32_t>(kTmemCols))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  TcFenceBefore();
-  __syncthreads();
-  TcFenceAfter();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-
-  if (warp == 0) {
-    if (ElectOne()) {
-      uint32_t ia = 0, ib = 0;
-      bool ok = true;
-      auto load_b = [&](int slot, int t, int cb, int nt) {
-        uint8_t* dst = b_smem + slot * kBBytes;
-        MbarExpectTx(&b_full[slot], kBBytes);
-        if (p.b_mn) {
-          for (int j = 0; j < BN / 64; ++j)
-            TmaLoad2D(dst + j * 8192, &maps.b, p.kofs[t] + nt * BN + j * 64, cb * kBK, &b_full[slot]);
-        } else {
-          TmaLoad2D(dst, &maps.b, p.kofs[t] + cb * kBK, nt * BN, &b_full[slot]);
-        }
-      };
-      if (p.b_resident)
-        for (int k = 0; k < num_k; ++k) load_b(k, k % 9, k / 9, 0);
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int mt = tile / p.n_tiles, nt = tile % p.n_tiles;
-        const int halves = p.units - 2 * mt < 2 ? 1 : 2;
-        for (int cb = 0; cb < p.cblocks && ok; ++cb, ++ia) {
-          const int s = ia % kHaloStages;
-          if (!MbarWait(&a_empty[s], ((ia / kHaloStages) & 1) ^ 1)) {
-            atomicExch(p.error, 1);
-            ok = false;
-            break;
-          }
-          MbarExpectTx(&a_full[s], p.box_tx * halves);
-          for (int h = 0; h < halves; ++h) {
-            const int u = 2 * mt + h;
-            TmaLoad4D(smem + (s * 2 + h) * p.half_bytes, &maps.a, cb * kBK, -1, (u % p.units_h) * p.th - 1, u / p.units_h,
-                      &a_full[s]);
-          }
-          if (p.b_resident) continue;
-          for (int t = 0; t < 9; ++t, ++ib) {
-            const int slot = ib % p.b_slots;
-            if (!MbarWait(&b_empty[slot], ((ib / p.b_slots) & 1) ^ 1)) {
-              atomicExch(p.error, 1);
-              ok = false;
-              break;
-            }
-            load_b(slot, t, cb, nt);
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    {  // the whole warp walks the loop, one lane issues
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (p.b_mn ? (1u << 16) : 0u) |
-                             (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
-      const uint64_t b_kstep = p.b_mn ? 128 : 2;
-      uint32_t ia = 0, ib = 0;
-      int local = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
-        const int mt = tile / p.n_tiles;
-        const int halves = p.units - 2 * mt < 2 ? 1 : 2;
-        const int buf = local & 1;
-        if (!MbarWaitWarp(&tmem_empty[buf], ((local >> 1) & 1) ^ 1)) {
-          if (lane == 0) atomicExch(p.error, 4);
-          break;
-        }
-        TcFenceAfter();
-        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * 2 * BN);
-        for (int cb = 0; cb < p.cblocks && ok; ++cb, ++ia) {
-          const int s = ia % kHaloStages;
-          if (!MbarWaitWarp(&a_full[s], (ia / kHaloStages) & 1)) {
-            if (lane == 0) atomicExch(p.error, 2);
-            ok = false;
-            break;
-          }
-          const uint32_t a_addr = SmemAddr(smem + s * 2 * p.half_bytes);
-          for (int t = 0; t < 9; ++t) {
-            const int slot = p.b_resident ? cb * 9 + t : static_cast<int>(ib % p.b_slots);
-            // resident blocks complete phase 0 once; the wait is then a single test
-            if (!MbarWaitWarp(&b_full[slot], p.b_resident ? 0 : (ib / p.b_slots) & 1)) {
-              if (lane == 0) atomicExch(p.error, 5);
-              ok = false;
-              break;
-            }
-            TcFenceAfter();
-            const uint32_t b_addr = SmemAddr(b_smem + slot * kBBytes);
-            const uint64_t bdesc  = p.b_mn ? SmemDescMnSw128(b_addr, 8192) : SmemDescSw128(b_addr);
-            if (ElectOne()) {
-              // one half after the other: alternating between them per MMA measured 120 us instead of 108
-              for (int h = 0; h < halves; ++h) {
-                const uint64_t adesc = SmemDescSw128(a_addr + h * p.half_bytes + p.row_shift[t] * 128);
-#pragma unroll
-                for (int k = 0; k < kBK / 16; ++k)
-                  UmmaBf16(tmem_d + static_cast<uint32_t>(h * BN), adesc + 2 * k, bdesc + b_kstep * k, idesc,
-                           (cb > 0 || t > 0 || k > 0) ? 1u : 0u);
-              }
-              if (!p.b_resident) UmmaCommit(&b_empty[slot]);
-            }
-            if (!p.b_resident) ++ib;
-          }
-          if (ElectOne()) UmmaCommit(&a_empty[s]);
-        }
-        if (ok && ElectOne()) UmmaCommit(&tmem_full[buf]);
-      }
-    }
-  } else if (warp < 6) {
-    // Epilogue: accumulator row r is pixel (r / pitch, r % pitch) of the unit; the real ones go, densely, into a box of
-    // [th x w] pixels x 64 channels for the TMA store unit.
-    const int q  = warp & 3;
-    const int r  = q * 32 + lane;
-    const int ph = r / p.pitch, pw = r % p.pitch;
-    const bool real = pw < p.w && ph < p.th;
-    const int dst   = ph * p.w + pw;
-    const int bar_threads = p.stat_sum != nullptr ? 256 : 128;
-    int local = 0;
-    uint32_t boxes = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
-      const int mt = tile / p.n_tiles, nt = tile % p.n_tiles;
-      const int halves = p.units - 2 * mt < 2 ? 1 : 2;
-      const int buf = local & 1;
-      if (ok && !MbarWait(&tmem_full[buf], (local >> 1) & 1)) {
-        if (lane == 0) atomicExch(p.error, 3);
-        ok = false;
-      }
-      TcFenceAfter();
-      for (int h = 0; h < halves; ++h) {
-        const int u = 2 * mt + h;
-        const uint32_t tsrc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>((buf * 2 + h) * BN);
-#pragma unroll 1
-        for (int b = 0; b < BN / 64; ++b, ++boxes) {
-          uint8_t* box = staging + (boxes & 1) * (kBM * 128);
-          uint32_t acc[2][32];
-          if (ok) {
-            TmemLoad32Async(tsrc + static_cast<uint32_t>(b * 64), acc[0]);
-            TmemLoad32Async(tsrc + static_cast<uint32_t>(b * 64 + 32), acc[1]);
-          }
-          if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          NamedBarSync(1, bar_threads);
-          if (ok) {
-            TmemLoadWait(acc[0]);
-            TmemLoadWait(acc[1]);
-            if (real) {
-#pragma unroll
-              for (int g = 0; g < 8; ++g) {
-                alignas(16) __nv_bfloat16 o[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16_rn(__uint_as_float(acc[g >> 2][(g & 3) * 8 + j]));
-                *reinterpret_cast<uint4*>(box + dst * 128 + ((g ^ (dst & 7)) << 4)) = *reinterpret_cast<uint4*>(o);
-              }
-            }
-          }
-          if (h == halves - 1 && b == BN / 64 - 1 && ok) {
-            TcFenceBefore();
-            __syncwarp();
-            if (lane == 0) MbarArrive(&tmem_empty[buf]);
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          NamedBarSync(1, bar_threads);
-          if (warp == 2 && lane == 0) {
-            if (ok) {
-              const int ch = nt * BN + b * 64, h0 = (u % p.units_h) * p.th, n0 = u / p.units_h;
-              if (p.accumulate) TmaReduceAdd4D(&maps.c, ch, 0, h0, n0, box);
-              else TmaStore4D(&maps.c, ch, 0, h0, n0, box);
-            }
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          }
-        }
-      }
-    }
-    if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  } else if (p.stat_sum != nullptr) {
-    // Statistics of the staged boxes, as in the tap kernel; a box holds th * w pixels, fewer in the last unit of an image.
-    float* partial   = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a_full) + 512);  // [2][4 warps][64][2]
-    const int st     = threadIdx.x - 192;
-    const int chunk  = st & 7;
-    const int rg     = st >> 3;
-    const int sw     = st >> 5;
-    uint32_t boxes = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      const int mt = tile / p.n_tiles, nt = tile % p.n_tiles;
-      const int halves = p.units - 2 * mt < 2 ? 1 : 2;
-      for (int h = 0; h < halves; ++h) {
-        const int h0   = ((2 * mt + h) % p.units_h) * p.th;
-        const int rows = (p.ho - h0 < p.th ? p.ho - h0 : p.th) * p.w;
-#pragma unroll 1
-        for (int b = 0; b < BN / 64; ++b, ++boxes) {
-          NamedBarSync(1, 256);
-          NamedBarSync(1, 256);
-          const uint8_t* box = staging + (boxes & 1) * (kBM * 128);
-          float s1[8], s2[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) s1[j] = s2[j] = 0.f;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int row = rg + 16 * i;
-            if (row < rows) {
-              const uint4 v = *reinterpret_cast<const uint4*>(box + row * 128 + ((chunk ^ (row & 7)) << 4));
-              const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 f = __bfloat1622float2(hv[j]);
-                s1[2 * j] += f.x; s2[2 * j] += f.x * f.x;
-                s1[2 * j + 1] += f.y; s2[2 * j + 1] += f.y * f.y;
-              }
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], 8);
-            s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], 16);
-            s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 8);
-            s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], 16);
-          }
-          float* P = partial + (boxes & 1) * (4 * 64 * 2);
-          if (lane < 8) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              P[(sw * 64 + lane * 8 + j) * 2]     = s1[j];
-              P[(sw * 64 + lane * 8 + j) * 2 + 1] = s2[j];
-            }
-          }
-          NamedBarSync(2, 128);
-          const int col = st & 63, which = st >> 6;
-          const float tot = P[(0 * 64 + col) * 2 + which] + P[(1 * 64 + col) * 2 + which] +
-                            P[(2 * 64 + col) * 2 + which] + P[(3 * 64 + col) * 2 + which];
-          const int ch = nt * BN + b * 64 + col;
-          if (ch < p.cout) atomicAdd((which ? p.stat_sq : p.stat_sum) + ch, tot);
-        }
-      }
-    }
-  }
-  TcFenceBefore();
-  __syncthreads();
-  if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(static_cast<uint32_t>(kTmemCols))
-                 : "memory");
-  }
-}
-
-// ------------------------------------------------------------------ the same for 64 -> 64 channels: two output rows per MMA
-// A 64-column MMA takes about as long as a 128-column one, so here the columns are the same 64 channels of two output rows,
-// h and h + 1.  Input row h - 1 + j reaches row h through filter row j and row h + 1 through filter row j - 1:
+// ------------------------------------------------------------------ 3x3, stride 1, 64 -> 64 channels: two output rows per MMA
+// The tap kernel above fetches the same box of pixels nine times, 16 KB for 128 x 64 x 64 products, and its 64-column MMAs
+// take about as long as 128-column ones would.  Here the pixels of a unit are loaded once with their border and the taps read
+// them at different offsets: with rows of w + 2 pixels (zero fill outside the image) a tap is a shift by whole 128-byte rows
+// of shared memory, and because the swizzle is a function of the address, a shifted start needs no other descriptor.  The
+// last two pixels of every such row are computed and dropped.  The columns of an MMA are the 64 channels of two output
+// rows, h and h + 1.  Input row h - 1 + j reaches row h through filter row j and row h + 1 through filter row j - 1:
 //   j = 0  row h only      j = 1, 2  both, with the weights [W_j | W_(j-1)] side by side      j = 3  row h + 1 only
 // i.e. 12 operand shifts for 18 taps.  A unit is `rp` such row pairs; the odd and the even input rows are loaded as two
 // boxes (maps over every other row), in which one pair further is one box row further, so all pairs of a unit are the 128
-// rows of one MMA as above.  The weights stay in shared memory, filter rows in descending order for each column tap.
-// 256 images of 56 x 56: 62 us forward and data gradient, 108 with one output row per MMA.
+// rows of one MMA (112 real pixels at 56 x 56 and 28 x 28).  The weights stay in shared memory, filter rows in descending
+// order for each column tap.  256 images of 56 x 56, forward or data gradient: 55 us, 147 with a box per tap (59 GFLOP).
 struct RowPairParams {
   int32_t* error;
   float* stat_sum;
@@ -726,17 +412,19 @@ struct RowPairMaps {
   CUtensorMap c[2];          // output rows 0, 2, .. and 1, 3, ..
 };
 
+constexpr int kPairStages      = 2;  // units in flight, two boxes each
 constexpr int kPairWeightBytes = 9 * 8192;
+constexpr int kPairFixed       = 2 * kBM * 128 + 1024 /*alignment*/ + 512 /*barriers*/ + 4096 /*statistics*/;
 
 __global__ void __launch_bounds__(kConvThreads, 1)
 ConvRowPairKernel(const __grid_constant__ RowPairMaps maps, const __grid_constant__ RowPairParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem    = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* b_smem  = smem + kHaloStages * 2 * p.box_bytes;
+  uint8_t* b_smem  = smem + kPairStages * 2 * p.box_bytes;
   uint8_t* staging = b_smem + kPairWeightBytes;
   uint64_t* a_full     = reinterpret_cast<uint64_t*>(staging + 2 * kBM * 128);
-  uint64_t* a_empty    = a_full + kHaloStages;
-  uint64_t* b_full     = a_empty + kHaloStages;
+  uint64_t* a_empty    = a_full + kPairStages;
+  uint64_t* b_full     = a_empty + kPairStages;
   uint64_t* tmem_full  = b_full + 1;      // [2]
   uint64_t* tmem_empty = tmem_full + 2;   // [2]
   uint32_t* tmem_slot  = reinterpret_cast<uint32_t*>(tmem_empty + 2);
@@ -745,7 +433,7 @@ ConvRowPairKernel(const __grid_constant__ RowPairMaps maps, const __grid_constan
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kHaloStages; ++s) {
+    for (int s = 0; s < kPairStages; ++s) {
       MbarInit(&a_full[s], 1);
       MbarInit(&a_empty[s], 1);
     }
@@ -777,8 +465,8 @@ ConvRowPairKernel(const __grid_constant__ RowPairMaps maps, const __grid_constan
         }
       int it = 0;
       for (int u = blockIdx.x; u < p.units; u += gridDim.x, ++it) {
-        const int s = it % kHaloStages;
-        if (!MbarWait(&a_empty[s], ((it / kHaloStages) & 1) ^ 1)) {
+        const int s = it % kPairStages;
+        if (!MbarWait(&a_empty[s], ((it / kPairStages) & 1) ^ 1)) {
           atomicExch(p.error, 1);
           break;
         }
@@ -800,12 +488,12 @@ ConvRowPairKernel(const __grid_constant__ RowPairMaps maps, const __grid_constan
       bool ok = MbarWaitWarp(b_full, 0);
       if (!ok && lane == 0) atomicExch(p.error, 5);
       for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x, ++it) {
-        const int buf = it & 1, s = it % kHaloStages;
+        const int buf = it & 1, s = it % kPairStages;
         if (!MbarWaitWarp(&tmem_empty[buf], ((it >> 1) & 1) ^ 1)) {
           if (lane == 0) atomicExch(p.error, 4);
           break;
         }
-        if (!MbarWaitWarp(&a_full[s], (it / kHaloStages) & 1)) {
+        if (!MbarWaitWarp(&a_full[s], (it / kPairStages) & 1)) {
           if (lane == 0) atomicExch(p.error, 2);
           break;
         }
@@ -1494,34 +1182,19 @@ int LaunchWgrad(const WgradMaps& maps, const WgradParams& p, int splits, cudaStr
   return 0;
 }
 
-// Image rows of a unit of the halo kernel (0: the image is too wide for two).
-int HaloRows(int w, int h) {
-  const int th = kBM / (w + 2);
-  return th < 2 ? 0 : std::min(th, h);
-}
-int HaloHalfBytes(int w, int th) { return CeilDiv(static_cast<int64_t>(w + 2) * (th + 2) * 128, 1024) * 1024; }
-
-// Whether the halo kernel should run a 3x3 / stride 1 convolution into `w_rows` channels of [n, h, w] pixels: 64-column
-// output tiles (128 columns do enough work per loaded byte: 128 images of 28 x 28, 128 -> 128, 54 us against 44 with a box
-// per tap), and units that fill the 128 rows of an MMA about as well as the tap kernel's boxes do.
-bool PreferHalo(int n, int h, int w, int w_rows) {
-  const int th = HaloRows(w, h);
-  if (th == 0 || w_rows % 128 == 0) return false;
-  const int64_t units = static_cast<int64_t>(n) * CeilDiv(h, th);
-  const Box box       = PickBox(w, h, n, false);
-  const int64_t boxes = static_cast<int64_t>(CeilDiv(w, box.tw)) * CeilDiv(h, box.th) * CeilDiv(n, box.tn);
-  return units >= 2 * NumSMs() && units * 10 <= boxes * 12;
-}
-
-// Whether the row-pair kernel should run a 3x3 / stride 1 convolution of 64 into 64 channels: the rule of the halo kernel
-// for units of two MMA tiles.
+// Whether the row-pair kernel should run a 3x3 / stride 1 convolution of 64 into 64 channels: a unit for every SM, and no more
+// waves of units than the tap kernel has of boxes (a wave takes about 2.3 and 3.6 us).  Measured, row pairs : taps in us:
+// 43 images of 28 x 28 (2 and 2 waves) 9.0 : 10.9, 256 of 28 x 28 (7 and 11) 21.5 : 41.7, 256 of 17 x 17 (4 and 4) 14.0 :
+// 18.1, 256 of 56 x 56 (25 and 43) 55 : 137, but 150 of 9 x 9 (2 and 1) 8.8 : 7.2.  Other channel counts keep a box per tap:
+// with more of them the tap kernel's loads are no longer the bound, and one halo box for all nine taps of one output row was
+// 5 to 20 % slower (64 images of 56 x 56, 128 -> 64: 79 : 68).
 bool PreferRowPairs(int n, int h, int w, int cin, int w_rows) {
-  if (cin != 64 || w_rows != 64 || w + 2 > kBM || h < 2) return false;
+  if (cin != 64 || w_rows != 64 || w > 62 || h < 2) return false;
   const int rp        = std::min(kBM / (w + 2), (h + 1) / 2);
   const int64_t units = static_cast<int64_t>(n) * CeilDiv(h, 2 * rp);
   const Box box       = PickBox(w, h, n, false);
   const int64_t boxes = static_cast<int64_t>(CeilDiv(w, box.tw)) * CeilDiv(h, box.th) * CeilDiv(n, box.tn);
-  return units >= NumSMs() && 2 * units * 10 <= boxes * 12;
+  return units >= NumSMs() && CeilDiv(units, NumSMs()) <= CeilDiv(boxes, NumSMs());
 }
 
 View RowPhaseView(const View& v, int parity) {  // every other row of a full view
@@ -1562,67 +1235,11 @@ int RunRowPairs(const View& in, const ConvTap* taps, const void* weights, int64_
     TIPSK_CUDA(cudaFuncSetAttribute(ConvRowPairKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
     configured = true;
   }
-  const int smem = kHaloStages * 2 * p.box_bytes + kPairWeightBytes + kHaloFixed;
+  const int smem = kPairStages * 2 * p.box_bytes + kPairWeightBytes + kPairFixed;
   TIPSK_REQUIRE(smem <= kMaxSmemBytes, "conv: the row-pair boxes do not fit in shared memory");
   ConvRowPairKernel<<<std::min(p.units, NumSMs()), kConvThreads, smem, s>>>(maps, p);
   TIPSK_LAUNCH_CHECK();
   return 0;
-}
-
-int LaunchHalo(const HaloMaps& maps, const HaloParams& p, cudaStream_t s) {
-  static bool configured = false;
-  if (!configured) {
-    TIPSK_CUDA(cudaFuncSetAttribute(ConvHaloKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes));
-    configured = true;
-  }
-  const int64_t tiles = static_cast<int64_t>((p.units + 1) / 2) * p.n_tiles;
-  const int grid = static_cast<int>(std::min<int64_t>(tiles, NumSMs()));
-  const int smem = kHaloStages * 2 * p.half_bytes + p.b_slots * 64 * 128 + kHaloFixed;
-  ConvHaloKernel<<<grid, kConvThreads, smem, s>>>(maps, p);
-  TIPSK_LAUNCH_CHECK();
-  return 0;
-}
-
-// out = 3x3 / stride 1 convolution of `in` (both [n, h, w] pixels) with the tap list of RunTaps.
-int RunHalo(const View& in, const ConvTap* taps, int cin, const void* weights, int w_rows, int64_t w_cols,
-            const View& out, float* stat_sum, float* stat_sq, cudaStream_t s, int accumulate, int b_mn) {
-  TIPSK_REQUIRE(cin % 64 == 0 && w_rows % 64 == 0, "conv: channel counts must be multiples of 64");
-  const int w = static_cast<int>(out.w), h = static_cast<int>(out.h), n = static_cast<int>(out.n);
-  if (PreferRowPairs(n, h, w, cin, w_rows))
-    return RunRowPairs(in, taps, weights, w_cols, out, stat_sum, stat_sq, s, accumulate, b_mn);
-  const int th = HaloRows(w, h);
-  constexpr int bn = 64;
-  HaloMaps maps;
-  HaloParams p{};
-  int rc = MapOf(&maps.a, in, Box{w + 2, th + 2, 1});
-  if (rc) return rc;
-  rc = b_mn ? MakeTmap2D(&maps.b, weights, cin, w_cols, 64) : MakeTmap2D(&maps.b, weights, w_rows, w_cols, bn);
-  if (rc) return rc;
-  rc = MapOf(&maps.c, out, Box{w, th, 1});
-  if (rc) return rc;
-  p.error = ConvErrorWord();
-  TIPSK_REQUIRE(p.error != nullptr, "conv: cannot allocate the error word");
-  p.stat_sum = stat_sum;
-  p.stat_sq  = stat_sq;
-  p.accumulate = accumulate;
-  p.b_mn    = b_mn;
-  p.cblocks = cin / 64;
-  p.pitch = w + 2; p.th = th; p.w = w; p.ho = h;
-  p.units_h = CeilDiv(h, th);
-  p.units   = n * p.units_h;
-  p.half_bytes = HaloHalfBytes(w, th);
-  p.box_tx     = static_cast<uint32_t>(w + 2) * (th + 2) * 128u;
-  p.cout    = w_rows;
-  p.n_tiles = w_rows / bn;
-  const int room = kMaxSmemBytes - kHaloFixed - kHaloStages * 2 * p.half_bytes;
-  p.b_slots    = std::min(kHaloMaxSlots, room / (bn * 128));
-  p.b_resident = (p.n_tiles == 1 && 9 * p.cblocks <= p.b_slots) ? 1 : 0;
-  TIPSK_REQUIRE(p.b_slots >= 2, "conv: the halo box leaves no shared memory for the weights");
-  for (int t = 0; t < 9; ++t) {
-    p.row_shift[t] = (taps[t].dh + 1) * p.pitch + taps[t].dw + 1;
-    p.kofs[t]      = taps[t].kofs;
-  }
-  return LaunchHalo(maps, p, s);
 }
 
 // Runs the tap kernel: out[view_out pixel, co] = sum over taps and 64-channel blocks.
@@ -1874,6 +1491,12 @@ using namespace tipsk;
 
 extern "C" {
 
+/* Which kernel a 3x3 / stride 1 forward pass (kind 0) or data gradient (kind 1) of these extents takes: 1 the row-pair kernel,
+ * 0 a box per tap. */
+int tipsk_conv2d_path(int kind, int n, int h, int w, int cin, int cout) {
+  return (kind == 0 ? PreferRowPairs(n, h, w, cin, cout) : PreferRowPairs(n, h, w, cout, cin)) ? 1 : 0;
+}
+
 /* 1 when the tcgen05 convolution kernels accept the problem. */
 int tipsk_conv2d_supported(int cin, int cout, int r, int s, int stride, int pad) {
   return (cin % 64 == 0 && cout % 64 == 0 && r == s && (r == 1 || r == 3) && (stride == 1 || stride == 2) &&
@@ -1903,9 +1526,9 @@ int tipsk_conv2d_fwd(const void* x, const void* wgt, void* y, int n, int h, int 
     nv = 4;
     for (int b = 0; b < 4; ++b) views[b] = PhaseView(x, n, h, w, cin, b >> 1, b & 1);
   }
-  if (r == 3 && stride == 1 && PreferHalo(n, h, w, cout))
-    return RunHalo(views[0], taps, cin, wgt, cout, static_cast<int64_t>(r) * s * cin, out, stat_sum, stat_sq,
-                   static_cast<cudaStream_t>(stream), 0, 0);
+  if (r == 3 && stride == 1 && PreferRowPairs(n, h, w, cin, cout))
+    return RunRowPairs(views[0], taps, wgt, static_cast<int64_t>(r) * s * cin, out, stat_sum, stat_sq,
+                       static_cast<cudaStream_t>(stream), 0, 0);
   return RunTaps(views, nv, taps, nt, cin, wgt, cout, static_cast<int64_t>(r) * s * cin, out, stat_sum, stat_sq,
                  static_cast<cudaStream_t>(stream));
 }
@@ -1947,8 +1570,8 @@ static int DgradImpl(const void* dy, const void* wgt_t, void* dx, int n, int h, 
       }
     View in  = r == 1 ? FlatView(dy, n, ho, wo, cout) : FullView(dy, n, ho, wo, cout);
     View out = r == 1 ? FlatView(dx, n, h, w, cin) : FullView(dx, n, h, w, cin);
-    if (r == 3 && PreferHalo(n, h, w, cin))
-      return RunHalo(in, taps, cout, wgt_t, cin, w_cols, out, nullptr, nullptr, st, accumulate, ohwi);
+    if (r == 3 && PreferRowPairs(n, h, w, cout, cin))
+      return RunRowPairs(in, taps, wgt_t, w_cols, out, nullptr, nullptr, st, accumulate, ohwi);
     return RunTaps(&in, 1, taps, nt, cout, wgt_t, cin, w_cols, out, nullptr, nullptr, st, accumulate, ohwi);
   }
   // stride 2: the input pixels of parity class (bh, bw) receive the taps with (b + pad - f) even

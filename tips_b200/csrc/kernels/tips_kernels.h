@@ -234,6 +234,7 @@ int tipsk_maxpool3x3s2_bwd(const void* dy, const void* idx, void* dx, int n, int
                            void* stream);
 
 /* ---- NHWC bf16 convolutions on tcgen05 (conv_tcgen05.cu): 1x1 and 3x3, stride 1 or 2, pad = r/2 ---- */
+int tipsk_conv2d_path(int kind, int n, int h, int w, int cin, int cout);
 int tipsk_conv2d_supported(int cin, int cout, int r, int s, int stride, int pad);
 int tipsk_conv2d_fwd(const void* x, const void* wgt, void* y, int n, int h, int w, int cin, int cout, int r, int s,
                      int stride, int pad, float* stat_sum, float* stat_sq, void* stream);
