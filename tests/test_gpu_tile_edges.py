@@ -144,17 +144,31 @@ def test_weight_gradient_of_non_finite_pixels(n, h, w, value):
     assert base.K().tipsk_conv_status() == 0
 
 
-@pytest.mark.parametrize("n,h,w,cout,stride", [(2, 6, 7, 64, 1), (3, 20, 20, 256, 1), (9, 15, 13, 320, 2), (40, 70, 70, 64, 1)])
-def test_weight_gradient_of_64_channels_in_tap_groups(n, h, w, cout, stride):
+# the smallest pixel counts that take several taps per tile (24 steps of 64 per CTA) and one below, with one and two tiles of
+# output channels, ragged boxes and stride 2; few pixels: one tap per tile
+@pytest.mark.parametrize("n,h,w,cout,stride,path", [(2, 6, 7, 64, 1, 0), (3, 20, 20, 256, 1, 0), (9, 15, 13, 320, 2, 0), (379, 20, 20, 64, 1, 1),
+                                                    (378, 20, 20, 64, 1, 0), (95, 40, 40, 128, 1, 1), (48, 37, 43, 320, 1, 1),
+                                                    (160, 71, 70, 64, 2, 1)])
+def test_weight_gradient_of_64_channels_in_tap_groups(n, h, w, cout, stride, path):
     from tips_b200.ops.conv import conv2d_wgrad
     from tips_b200.ops import base
     x = _rand(n, 64, h, w).contiguous(memory_format=torch.channels_last)
     ho, wo = (h - 1) // stride + 1, (w - 1) // stride + 1
+    assert base.K().tipsk_conv2d_path(2, n, ho, wo, 64, cout) == path
     dy = _rand(n, cout, ho, wo, seed=1).contiguous(memory_format=torch.channels_last)
     got = conv2d_wgrad(x, dy, (cout, 3, 3, 64), stride, 1)
-    ref = torch.nn.grad.conv2d_weight(x.double(), (cout, 64, 3, 3), dy.double(), stride=stride, padding=1)
+    xp = F.pad(x.float(), (1, 1, 1, 1))
+    dyf = dy.float().permute(0, 2, 3, 1).reshape(-1, cout)
+    torch.backends.cuda.matmul.allow_tf32, before = False, torch.backends.cuda.matmul.allow_tf32
+    try:
+        ref = torch.stack([torch.stack([
+            dyf.t() @ xp[:, :, r:r + (ho - 1) * stride + 1:stride, s:s + (wo - 1) * stride + 1:stride].permute(0, 2, 3, 1).reshape(-1, 64)
+            for s in range(3)], 1) for r in range(3)], 1)
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
     assert base.K().tipsk_conv_status() == 0
-    _close(got, ref.permute(0, 2, 3, 1))
+    # fp32 sums of up to 200 000 products in two orders: a random walk of roundings, 2^-12 of the largest value bounds both
+    _close(got, ref)
 
 
 @pytest.mark.parametrize("n,c,h,w", [(1, 8, 1, 1), (2, 8, 2, 3), (3, 72, 5, 8), (2, 64, 31, 33), (1, 2056, 4, 4)])

@@ -661,7 +661,7 @@ struct WgradParams {
   int tw, th, tn;   // tw * th * tn is a multiple of 16, at most 128
   int cout, cin;
   int a_boxes;      // 64-channel boxes of dy to load per stage: 1 when cout <= 64 (rows 64..127 are then unused)
-  int group;        // taps per CTA: with 64 input channels the columns of a tile are several taps side by side
+  int group;        // taps per CTA (kGroup)
   ConvTap tap[kMaxTaps];  // kofs = first column of the tap inside a row of dw
 };
 
@@ -675,6 +675,7 @@ struct WgradMaps {
 // stages still fit; it moves a third fewer bytes per FLOP through L2 than the 128-channel tile.
 // kMH: output-channel halves of 128 per CTA.  With two (256 x 256 tile, both accumulators filling TMEM) a K step moves
 // 64 KB for 1024 tensor-core clocks, which the 64 B/clk/SM L2 path can just sustain; the 128-row tiles are load-bound.
+// kGroup: 64 input channels, and the columns of a tile are p.group taps side by side.
 template <int BN, int kBoxRows, int kMH = 1>
 struct WgradCfg {
   static constexpr int kBoxBytes   = kBoxRows * 128;
@@ -686,7 +687,7 @@ struct WgradCfg {
   static constexpr int kSmemBytes  = kStages * kStageBytes + 1024 + 256;
 };
 
-template <int BN, int kBoxRows, int kMH = 1>
+template <int BN, int kBoxRows, int kMH, bool kGroup>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ WgradParams p) {
   using Cfg = WgradCfg<BN, kBoxRows, kMH>;
@@ -702,8 +703,9 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
   int id = blockIdx.x;
   const int cin_t  = id % p.cin_tiles;  id /= p.cin_tiles;
   const int cout_t = id % p.cout_tiles; id /= p.cout_tiles;
-  const int tap0    = id * p.group;  // with group == 1 the one tap of this CTA
-  const int b_boxes = p.group == 1 ? BN / 64 : (p.taps - tap0 < p.group ? p.taps - tap0 : p.group);
+  const int tap0    = kGroup ? id * p.group : id;
+  const ConvTap tap = p.tap[tap0];  // without kGroup the one tap of this CTA
+  const int b_boxes = !kGroup ? BN / 64 : (p.taps - tap0 < p.group ? p.taps - tap0 : p.group);
   const int box_rows = p.tw * p.th * p.tn;
   const int k_tiles  = p.tiles_w * p.tiles_h * p.tiles_n;
   const int k_begin  = static_cast<int>(static_cast<int64_t>(k_tiles) * blockIdx.y / gridDim.y);
@@ -747,10 +749,16 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
         MbarExpectTx(&full_bar[s], stage_tx);
         for (int j = 0; j < p.a_boxes; ++j)
           TmaLoad4D(a_dst + j * Cfg::kBoxBytes, &maps.dy, cout_t * kBM * kMH + j * 64, w0, h0, n0, &full_bar[s]);
-        for (int j = 0; j < b_boxes; ++j) {
-          const ConvTap& tap = p.tap[p.group == 1 ? tap0 : tap0 + j];
-          TmaLoad4D(b_dst + j * Cfg::kBoxBytes, &maps.x[tap.map], p.group == 1 ? cin_t * BN + j * 64 : 0, w0 + tap.dw,
-                    h0 + tap.dh, n0, &full_bar[s]);
+        if constexpr (kGroup) {
+          for (int j = 0; j < b_boxes; ++j) {
+            const ConvTap& tj = p.tap[tap0 + j];
+            TmaLoad4D(b_dst + j * Cfg::kBoxBytes, &maps.x[tj.map], 0, w0 + tj.dw, h0 + tj.dh, n0, &full_bar[s]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j)
+            TmaLoad4D(b_dst + j * Cfg::kBoxBytes, &maps.x[tap.map], cin_t * BN + j * 64, w0 + tap.dw, h0 + tap.dh, n0,
+                      &full_bar[s]);
         }
       }
     }
@@ -798,9 +806,9 @@ ConvWgradKernel(const __grid_constant__ WgradMaps maps, const __grid_constant__ 
         TmemLoad32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(c * 32), acc);
         const int row  = (cout_t * kMH + c / (BN / 32)) * kBM + q * 32 + lane;  // accumulator c / (BN/32) = its half
         const int box  = (c % (BN / 32)) / 2;  // 64-column box: a channel block, or a tap of the group
-        const int col0 = p.group == 1 ? cin_t * BN + (c % (BN / 32)) * 32 : (c & 1) * 32;
-        if (row < p.cout && col0 < p.cin && box < b_boxes) {
-          float* dst = p.dw + static_cast<int64_t>(row) * p.ldw + p.tap[p.group == 1 ? tap0 : tap0 + box].kofs + col0;
+        const int col0 = kGroup ? (c & 1) * 32 : cin_t * BN + (c % (BN / 32)) * 32;
+        if (row < p.cout && col0 < p.cin && (!kGroup || box < b_boxes)) {
+          float* dst = p.dw + static_cast<int64_t>(row) * p.ldw + (kGroup ? p.tap[tap0 + box].kofs : tap.kofs) + col0;
 #pragma unroll
           for (int g = 0; g < 8; ++g) {
             asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + g * 4),
@@ -1167,17 +1175,17 @@ int LaunchTaps(const ConvMaps& maps, const ConvParams& p, cudaStream_t s) {
   return 0;
 }
 
-template <int BN, int kBoxRows, int kMH = 1>
+template <int BN, int kBoxRows, int kMH = 1, bool kGroup = false>
 int LaunchWgrad(const WgradMaps& maps, const WgradParams& p, int splits, cudaStream_t s) {
   using Cfg = WgradCfg<BN, kBoxRows, kMH>;
   static bool configured = false;
   if (!configured) {
-    TIPSK_CUDA(cudaFuncSetAttribute(ConvWgradKernel<BN, kBoxRows, kMH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TIPSK_CUDA(cudaFuncSetAttribute(ConvWgradKernel<BN, kBoxRows, kMH, kGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     Cfg::kSmemBytes));
     configured = true;
   }
   dim3 grid(CeilDiv(p.taps, p.group) * p.cout_tiles * p.cin_tiles, splits);
-  ConvWgradKernel<BN, kBoxRows, kMH><<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(maps, p);
+  ConvWgradKernel<BN, kBoxRows, kMH, kGroup><<<grid, kGemmThreads, Cfg::kSmemBytes, s>>>(maps, p);
   TIPSK_LAUNCH_CHECK();
   return 0;
 }
@@ -1322,6 +1330,19 @@ int ForwardTaps(int r, int s, int stride, int pad, int cin, ConvTap* taps) {
 }
 
 // Weight gradient over arbitrary activation views and taps: dw[co, tap.kofs + ci] += sum_p dy[p, co] * x_view[p + tap].
+// Taps per tile of the weight gradient: with 64 input channels up to four taps can be the columns of one tile, so that dy is
+// loaded once for all of them and the MMAs are 256 columns wide.  The groups are even (nine taps: three groups of three, the
+// stem's seven: four and three).  Such a tile also adds three or four times as many values into dw, so it takes a long share
+// of the pixels, 24 steps of 64, to pay for them.  Measured, grouped : one tap per tile in us: stem, 64 images of 224 x 224
+// (85 steps) 106 : 142, of 32 x 160 x 160 (22) 40 : 45, 16 x 128 x 128 (4) 26 : 22; 3x3 64 -> 256, 64 of 56 x 56 (64) 88 : 102,
+// 64 -> 128 56 x 56 (32) 59 : 61, 20 x 20 x 256 (16) 37 : 33, 28 x 28 x 16 (2) 21 : 13.
+int WgradGroup(int cin, int cout, int n_taps, int64_t pixels) {
+  if (cin != 64 || n_taps == 1) return 1;
+  const int groups = CeilDiv(n_taps, 4);
+  const int64_t steps = CeilDiv(pixels, 64) * static_cast<int64_t>(groups) * CeilDiv(cout, kBM);
+  return steps >= 24 * 2 * NumSMs() ? CeilDiv(n_taps, groups) : 1;
+}
+
 int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, int n_taps, int cin, int cout, int ldw,
              float* dw, cudaStream_t st) {
   TIPSK_REQUIRE(n_taps >= 1 && n_taps <= kMaxTaps, "conv: 1..9 filter taps are supported");
@@ -1329,13 +1350,9 @@ int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, 
   WgradParams p{};
   p.taps = n_taps;
   for (int i = 0; i < n_taps; ++i) p.tap[i] = taps[i];
-  // With 64 input channels and several taps a tile takes up to four taps as its columns: dy is loaded once for all of
-  // them and the MMAs are 256 columns wide (stem, 64 images of 224 x 224: 117 -> 103 us).  The groups are even (nine taps:
-  // three groups of three, seven: four and three).
-  const int groups = CeilDiv(n_taps, 4);
-  const bool group = cin == 64 && n_taps > 1;
-  const int bn  = group || cin % 256 == 0 ? 256 : cin % 128 == 0 ? 128 : 64;
-  p.group = group ? CeilDiv(n_taps, groups) : 1;
+  const int group = WgradGroup(cin, cout, n_taps, dyv.w * dyv.h * dyv.n);
+  const int bn    = group > 1 || cin % 256 == 0 ? 256 : cin % 128 == 0 ? 128 : 64;
+  p.group = group;
   const Box box = PickBox(static_cast<int>(dyv.w), static_cast<int>(dyv.h), static_cast<int>(dyv.n), true,
                           bn == 256 ? 64 : 128);
   int rc = MapOf(&maps.dy, dyv, box);
@@ -1357,7 +1374,7 @@ int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, 
   // 14x14 and 7x7 convolutions, where it leaves too few CTAs).
   static const bool no_big = getenv("TIPS_WGRAD_NO_BM256") != nullptr;
   int mh = 1;
-  if (!no_big && !group && bn == 256 && cout % 256 == 0) {
+  if (!no_big && group == 1 && bn == 256 && cout % 256 == 0) {
     const int64_t kt    = static_cast<int64_t>(CeilDiv(dyv.w, box.tw)) * CeilDiv(dyv.h, box.th) * CeilDiv(dyv.n, box.tn);
     const int64_t base2 = static_cast<int64_t>(n_taps) * (cout / 256) * (cin / 256);
     const int64_t sp2   = std::max<int64_t>(1, 2 * NumSMs() / base2);
@@ -1377,6 +1394,7 @@ int RunWgrad(const View& dyv, const View* xv, int n_views, const ConvTap* taps, 
   if (splits > k_tiles) splits = static_cast<int>(k_tiles);
   if (splits < 1) splits = 1;
   TIPSK_CUDA(cudaMemsetAsync(dw, 0, sizeof(float) * static_cast<size_t>(cout) * ldw, st));
+  if (group > 1) return LaunchWgrad<256, 64, 1, true>(maps, p, splits, st);
   if (bn == 256 && mh == 2) return LaunchWgrad<256, 64, 2>(maps, p, splits, st);
   if (bn == 256) return LaunchWgrad<256, 64>(maps, p, splits, st);
   return bn == 128 ? LaunchWgrad<128, 128>(maps, p, splits, st) : LaunchWgrad<64, 128>(maps, p, splits, st);
@@ -1492,8 +1510,9 @@ using namespace tipsk;
 extern "C" {
 
 /* Which kernel a 3x3 / stride 1 forward pass (kind 0) or data gradient (kind 1) of these extents takes: 1 the row-pair kernel,
- * 0 a box per tap. */
+ * 0 a box per tap; and a weight gradient (kind 2): 2 the halo kernel, 1 several taps per tile, 0 one tap per tile. */
 int tipsk_conv2d_path(int kind, int n, int h, int w, int cin, int cout) {
+  if (kind == 2) return PreferWgradHalo(n, h, w, cin, cout) ? 2 : WgradGroup(cin, cout, 9, static_cast<int64_t>(n) * h * w) > 1;
   return (kind == 0 ? PreferRowPairs(n, h, w, cin, cout) : PreferRowPairs(n, h, w, cout, cin)) ? 1 : 0;
 }
 
