@@ -50,9 +50,19 @@ def test_linear_products(m, n, k, act):
     assert gemm_status() == 0
 
 
-@pytest.mark.parametrize("rows,n,k", [(16, 64, 64), (77, 256, 128), (1232, 320, 1024), (4096, 1024, 1024), (8200, 4096, 192)])
-def test_weight_gradient_in_bf16(rows, n, k):
+# rows, outputs, inputs, and whether the pair kernel runs it (1) or the convolution's: each line of the rule from both sides,
+# ragged last tiles and a K that is no multiple of a block, unsplit and split
+WEIGHT_GRADIENT = [(16, 128, 128, 1), (16, 64, 64, 0), (256, 192, 128, 1), (257, 192, 128, 0), (77, 256, 128, 1), (1024, 1024, 256, 1),
+                   (1025, 1024, 256, 0), (1232, 320, 1024, 0), (4096, 1024, 1024, 1), (8200, 4096, 192, 0), (8200, 320, 1984, 1),
+                   (32768, 64, 256, 1), (32769, 64, 256, 0), (32769, 128, 256, 1), (65537, 256, 256, 0), (65537, 512, 512, 1),
+                   (12544, 64, 64, 0), (2000, 512, 1728, 1)]
+
+
+@pytest.mark.parametrize("rows,n,k,pair", WEIGHT_GRADIENT)
+def test_weight_gradient_in_bf16(rows, n, k, pair):
+    from tips_b200.ops import base
     from tips_b200.ops.linear import _weight_grad, gemm_status
+    assert base.K().tipsk_gemm_prefers_pair(2, n, k, rows) == pair
     dz, x = _rand(rows, n), _rand(rows, k, seed=1)
     ref = dz.double().t() @ x.double()
     _close(_weight_grad(dz, x, BF16), ref)

@@ -1020,11 +1020,24 @@ int tipsk_gemm_bf16_nn(const void* a, const void* b, void* c, int m, int n, int 
 int tipsk_gemm_prefers_pair(int kind, int m, int n, int k) {
   if (m < 64 || n < 64 || n % 8 != 0 || k <= 0) return 0;
   if (kind != 2) return PreferPair(m, n, k) ? 1 : 0;
-  // Weight gradients: the alternative spreads K over all SMs and costs 10 us plus a fill and a cast (3.5 us); a pair walks
-  // its K alone, 8 us plus 0.28 us per 64 rows, unless K is long enough to be split.  Measured with two tiles: 13 : 17 us at
-  // K = 2000, 21 : 26 at 3920; with 16 tiles 32 : 20 at 2048.
-  const int64_t tiles = static_cast<int64_t>(CeilDiv(m, 2 * kBM)) * CeilDiv(n, PairCfg::kBN);
-  return (k <= 1024 || tiles >= 12 || tipsk_gemm_splits(m, n, k) > 1) ? 1 : 0;
+  // Weight gradients: the alternative is the convolution's kernel, which spreads K over all SMs with 128-row tiles as narrow as
+  // 64 columns, adds fp32 sums into a cleared buffer and is followed by a cast.  Measured, pair : convolution kernel in us
+  // (M x N x K).
+  const int64_t tiles  = static_cast<int64_t>(CeilDiv(m, 2 * kBM)) * CeilDiv(n, PairCfg::kBN);
+  const int64_t splits = tipsk_gemm_splits(m, n, k), pairs = NumSMs() / 2;
+  // Outputs that leave half of their 256 x 256 tiles empty waste the pair's MMAs: 64 x 64 x 401408 44 : 23, 256 x 64 x 200704
+  // 37 : 30, 192 x 320 x 32768 24 : 18.  But columns that fill whole tiles suit the alternative's widest tile no better, and
+  // its sums cost more, up to middling K: 64 x 256 x 12544 14 : 18, 64 x 512 x 16384 16 : 19, 64 x 256 x 200704 39 : 35.
+  const bool few_k = k <= 256 && m >= 128 && n % 128 == 0;  // 192 x 128 x 256 7.3 : 7.8
+  if (!few_k && !(n >= PairCfg::kBN && 2 * static_cast<int64_t>(m) * n >= tiles * 2 * kBM * PairCfg::kBN) &&
+      !(n % PairCfg::kBN == 0 && k <= 32768))
+    return 0;
+  // Very long K amortises the alternative's costs: 256 x 256 x 131072 47 : 44 (74 partial tiles to add), 2304 x 768 x 131072
+  // 359 : 333 (27 tiles in two shares leave 20 of 74 pairs idle); with the pairs busy 768 x 768 x 131072 122 : 131.
+  if (k > 65536 && (tiles < 2 || tiles * splits * 5 < pairs * 4)) return 0;
+  // Few tiles walk an unsplit K on few SMs, 5 us plus 0.35 us per 64 rows: 512 x 256 x 1000 11.0 : 10.6, 256 x 512 x 256 7.6 : 10,
+  // 384 x 1024 x 1000 11 : 18, 512 x 1728 x 2048 16 : 18.
+  return (k <= 256 || (tiles >= 4 && k <= 1024) || tiles >= 12 || splits > 1) ? 1 : 0;
 }
 
 /* Number of K splits with which tipsk_gemm_bf16_split should run the product (1: use the unsplit entry points). */
