@@ -24,14 +24,20 @@ def _rand(*shape, scale=0.5, dtype=BF16, seed=0):
     return (torch.randn(*shape, generator=g, device=DEV) * scale).to(dtype)
 
 
-# one CTA pair, a ragged last tile in each direction, several tiles per pair, a K of one block and with a remainder
-GEMM = [(256, 256, 64), (257, 512, 72), (300, 1000, 200), (512, 264, 1024), (4100, 1032, 136), (20000, 1024, 264)]
+# m, n, k, and whether CTA pairs run it.  Single CTAs: one tile, ragged last tiles, several tiles, a K of one block and with a
+# remainder.  Pairs: N and M that end inside a tile and inside a 64-column box, rows that fill one CTA of a pair's last tile only,
+# K of one block, of less and with a remainder, fewer tiles than two per pair and many.  And the rule's lines from both sides.
+GEMM = [(256, 256, 64, 0), (257, 512, 72, 0), (300, 1000, 200, 0), (512, 264, 1024, 0), (4100, 1032, 136, 0), (4096, 1288, 88, 0),
+        (20000, 1024, 264, 1), (8200, 1032, 64, 1), (4100, 1800, 72, 1), (4100, 1544, 72, 0), (1232, 30536, 136, 1), (16008, 392, 48, 1), (5900, 1000, 320, 1),
+        (2048, 3072, 8, 1), (12000, 384, 264, 0), (14000, 384, 264, 1), (16384, 320, 256, 0), (16384, 320, 264, 1)]
 
 
-@pytest.mark.parametrize("m,n,k", GEMM)
+@pytest.mark.parametrize("m,n,k,pair", GEMM)
 @pytest.mark.parametrize("act", [None, "relu", "gelu"])
-def test_linear_products(m, n, k, act):
+def test_linear_products(m, n, k, pair, act):
+    from tips_b200.ops import base
     from tips_b200.ops.linear import gemm_nn, gemm_status, gemm_tn
+    assert base.K().tipsk_gemm_prefers_pair(0, m, n, k) == base.K().tipsk_gemm_prefers_pair(1, m, n, k) == pair
     a, b, bias = _rand(m, k), _rand(n, k, seed=1), _rand(n, seed=2)
     ref_pre = a.double() @ b.double().t() + bias.double()
     ref = {None: lambda t: t, "relu": F.relu, "gelu": F.gelu}[act](ref_pre)

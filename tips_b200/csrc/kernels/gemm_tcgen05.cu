@@ -902,10 +902,16 @@ int LaunchPairSplit(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPara
 // single-CTA kernels (us, M x N x K): 192 tiles 4096 x 3072 x 1024 32 : 45, 128 tiles 8192 x 1024 x 1024 27 : 32, 96
 // tiles 2048 x 3072 x 1024 26 : 31; below, a pair's single 256 x 256 tile and its exposed epilogue take longer than
 // two small CTAs per SM: 64 tiles 4096 x 1024 x 1024 21 : 17, 8192 x 512 x 1728 25 : 21.
+// Where N ends inside a tile, 128-column tiles cover it more closely.  They stay ahead while all of them are resident at once,
+// two per SM (12000 x 384 x 1024 12.7 : 17.1, 12000 x 264 x 264 9.8 : 12.3; with more 14000 x 384 x 1024 20.7 : 17.5), and
+// with a short K, where the epilogues are most of the time, up to three per SM (16384 x 320 x 128 11.7 : 13.2, 8192 x 640 x
+// 64 10.8 : 13.4, 6000 x 1032 x 256 13.7 : 14.6; with more 12000 x 640 x 64 17.5 : 13.7).
 bool PreferPair(int m, int n, int k) {
-  (void)k;
   const int64_t tiles = static_cast<int64_t>(CeilDiv(m, 2 * kBM)) * CeilDiv(n, PairCfg::kBN);
-  return n > 128 && tiles * 4 >= (NumSMs() / 2) * 5;
+  if (n <= 128 || tiles * 4 < (NumSMs() / 2) * 5) return false;
+  const bool ragged   = static_cast<int64_t>(m) * n * 10 < tiles * 2 * kBM * PairCfg::kBN * 9;
+  const int64_t small = static_cast<int64_t>(CeilDiv(m, kBM)) * CeilDiv(n, 128);
+  return !ragged || small > NumSMs() * (k <= 256 ? 3 : 2);
 }
 
 }  // namespace
