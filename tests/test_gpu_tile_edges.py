@@ -340,9 +340,17 @@ def test_bias_act_backward_rows(dtype, rows, cols, act):
 
 
 @pytest.mark.parametrize("dtype", [BF16, torch.float16])
-@pytest.mark.parametrize("rows,cols", [(1, 256), (14, 256), (2221, 256), (8, 1024), (1185, 1024), (1200, 768), (301, 2048)])
-def test_layer_norm_backward_groups(dtype, rows, cols):
+# the groups' blocks number one per SM at most and the small ones eight: rows below and above the line between them, from
+# blocks with less than one row per group to many, one to fifteen groups per block, and the longest and widest of each
+@pytest.mark.parametrize("rows,cols,groups", [(1, 256, False), (14, 256, False), (2221, 256, False), (4687, 256, False), (4688, 256, True),
+                                              (16383, 256, True), (16384, 256, False), (8, 1024, False), (1185, 1024, True), (1171, 1024, False),
+                                              (1600, 768, True), (586, 2048, True), (301, 2048, False), (2000, 1792, True)])
+def test_layer_norm_backward_groups(dtype, rows, cols, groups):
+    from tips_b200.ops import base
     from tips_b200.ops.norm import layer_norm
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    blocks = min(sms, -(-rows // min(15, 768 // (cols // 8)))) if groups else min(8 * sms, -(-rows // 4))
+    assert base.K().tipsk_ln_bwd_partial_rows(rows, cols, base.code(dtype)) == blocks
     x, dy = _rand(rows, cols, dtype=dtype).requires_grad_(), _rand(rows, cols, dtype=dtype, seed=1)
     w, b = (1 + _rand(cols, dtype=dtype, scale=0.1, seed=2)).requires_grad_(), _rand(cols, dtype=dtype, seed=3).requires_grad_()
     layer_norm(x, w, b).backward(dy)

@@ -5,8 +5,6 @@
 // accumulates dgamma / dbeta for its lane's columns over all the rows it
 // visits; blocks write one partial row each and a small second kernel sums
 // them.  The reference has no model math; this serves the BERT-shaped encoder.
-#include <type_traits>
-
 #include "kernels/common.cuh"
 #include "kernels/tips_kernels.h"
 
@@ -238,23 +236,23 @@ LnBwdBlockRowKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* 
   }
 }
 
-// The same with a GROUP of cols / 8 threads per row, for shorter inputs: each thread owns 8 consecutive columns (one 16-byte vector), so the
-// per-column dgamma / dbeta accumulators are 16 registers instead of 64.  A block is as many groups as 768 threads and
-// the 15 named barriers allow; every group walks its own rows, with the next row's loads in flight while it reduces the
-// current one (the two row sums go through shared memory, one barrier of the group per row, double-buffered), and the
-// groups' column sums are added up in shared memory at the end.  One block per SM: with eight small blocks per SM a block
-// of the 4096 x 1024 gradient of an encoder layer had 3.5 rows, and its partial rows were 40 % of the traffic.  That
-// shape: 16 -> 13 us, and the sum of the partial rows 8 -> 3 us.  From 16384 rows on the partial rows are 10 % or less,
-// and the 1024 threads per SM of the small blocks keep more bytes in flight.
+// The same with a GROUP of cols / 8 threads per row, for inputs of middling length: each thread owns 8 consecutive columns
+// (one 16-byte vector), so the per-column dgamma / dbeta accumulators are 16 registers instead of 64.  A block is as many
+// groups as 768 threads and the 15 named barriers allow; every group walks its own rows, with the next row's loads in
+// flight while it reduces the current one (the two row sums go through shared memory, one barrier of the group per row,
+// double-buffered), and the groups' column sums are added up in shared memory at the end.  One block per SM: with eight
+// small blocks per SM a block of the 4096 x 1024 gradient of an encoder layer had 3.5 rows, and its partial rows were 40 %
+// of the traffic.  That shape, with the sum of the partial rows: 21.8 -> 13.9 us.
 constexpr int kLnGroupThreads = 768;  // with 1024 the accumulators and the prefetched row spill
+constexpr int kLnGroupCols    = 2048;
 
 inline int LnGroups(int group) {
   const int g = kLnGroupThreads / group;
-  return g > 15 ? 15 : g < 1 ? 1 : g;
+  return g > 15 ? 15 : g;
 }
 
-template <typename T, int kThreads>
-__global__ void __launch_bounds__(kThreads, 1)
+template <typename T>
+__global__ void __launch_bounds__(kLnGroupThreads, 1)
 LnBwdGroupKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                  const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
                  float* __restrict__ dgamma_partial, float* __restrict__ dbeta_partial, int64_t rows, int cols) {
@@ -373,10 +371,17 @@ LnReducePartialsKernel(const float* __restrict__ pg, const float* __restrict__ p
   }
 }
 
-constexpr int64_t kLnLongRows = 16384;
+// Rows of whole warps of 16-byte vectors in a 16-bit type: one small block of cols / 8 threads walks them row by row.
+bool LnUsesBlockRows(int cols, int dtype) { return dtype != kF32 && cols % 256 == 0 && cols / 8 <= 1024; }
 
-// Rows of whole warps of 16-byte vectors in a 16-bit type, one group of threads (or one block) each.
-bool LnUsesGroups(int cols, int dtype) { return dtype != kF32 && cols % 256 == 0 && cols / 8 <= 1024; }
+// ... or one block per SM in groups.  Adding up the groups' column sums costs several us, which short inputs do not win back:
+// groups : small blocks in us, gradient and sum of the partial rows, 296 x 256 11.7 : 5.5, 2048 x 512 12.8 : 10.7, 1024 x 1024
+// 10.0 : 9.1, but 3000 x 512 12.9 : 13.5, 1500 x 1024 10.2 : 11.6, 600 x 2048 9.8 : 11.0, 8192 x 768 16.9 : 24.3.  From 16384
+// rows on the partial rows are 10 % of the traffic or less, and the small blocks keep more bytes in flight (16383 x 2048
+// 69.9 : 74.8, 16383 x 4096 203 : 158: with more columns a group is all that fits, one row at a time).
+bool LnUsesGroups(int64_t rows, int cols, int dtype) {
+  return LnUsesBlockRows(cols, dtype) && cols <= kLnGroupCols && rows < 16384 && rows * cols >= 1200000;
+}
 
 int LnGrid(int64_t rows) {
   int64_t blocks = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
@@ -439,15 +444,9 @@ int tipsk_ln_fwd_residual(const void* x, const void* residual, const void* gamma
   return 0;
 }
 
-int tipsk_ln_bwd_partials(int64_t rows, int cols) {
-  (void)cols;
-  return LnGrid(rows);
-}
-
 /* The number of partial rows with which tipsk_ln_bwd should be called for this dtype. */
 int tipsk_ln_bwd_partial_rows(int64_t rows, int cols, int dtype) {
-  if (!LnUsesGroups(cols, dtype)) return LnGrid(rows);
-  if (rows >= kLnLongRows) return LnGrid(rows);
+  if (!LnUsesGroups(rows, cols, dtype)) return LnGrid(rows);
   const int64_t blocks = (rows + LnGroups(cols / 8) - 1) / LnGroups(cols / 8);
   return static_cast<int>(blocks < NumSMs() ? (blocks < 1 ? 1 : blocks) : NumSMs());
 }
@@ -460,41 +459,21 @@ int tipsk_ln_bwd(const void* dy, const void* x, const void* gamma, const float* 
   TIPSK_REQUIRE(partial_rows == LnGrid(rows) || partial_rows == tipsk_ln_bwd_partial_rows(rows, cols, dtype),
                 "layer norm backward: wrong number of partial rows");
   cudaStream_t s    = static_cast<cudaStream_t>(stream);
-  if (LnUsesGroups(cols, dtype) && rows >= kLnLongRows) {
-    if (dtype == kBF16)
-      LnBwdBlockRowKernel<__nv_bfloat16><<<partial_rows, cols / 8, 0, s>>>(
+  if (LnUsesBlockRows(cols, dtype)) {
+    const bool groups  = LnUsesGroups(rows, cols, dtype);
+    const int threads  = groups ? LnGroups(cols / 8) * (cols / 8) : cols / 8;
+    const size_t bytes = groups ? sizeof(float) * 2 * cols : 0;
+    if (dtype == kBF16) {
+      auto* kernel = groups ? LnBwdGroupKernel<__nv_bfloat16> : LnBwdBlockRowKernel<__nv_bfloat16>;
+      kernel<<<partial_rows, threads, bytes, s>>>(
           static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
           static_cast<const __nv_bfloat16*>(gamma), mean, rstd, static_cast<__nv_bfloat16*>(dx), dgamma_partial,
           dbeta_partial, rows, cols);
-    else
-      LnBwdBlockRowKernel<__half><<<partial_rows, cols / 8, 0, s>>>(
+    } else {
+      auto* kernel = groups ? LnBwdGroupKernel<__half> : LnBwdBlockRowKernel<__half>;
+      kernel<<<partial_rows, threads, bytes, s>>>(
           static_cast<const __half*>(dy), static_cast<const __half*>(x), static_cast<const __half*>(gamma), mean, rstd,
           static_cast<__half*>(dx), dgamma_partial, dbeta_partial, rows, cols);
-    TIPSK_LAUNCH_CHECK();
-    return 0;
-  }
-  if (LnUsesGroups(cols, dtype)) {
-    const int threads  = LnGroups(cols / 8) * (cols / 8);
-    const size_t bytes = sizeof(float) * 2 * cols;  // at most 64 KB, above the default limit from 5120 columns on
-    auto launch = [&](auto* kernel, auto* type) {
-      using T = std::remove_pointer_t<decltype(type)>;
-      if (bytes > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        if (e != cudaSuccess) return e;
-      }
-      kernel<<<partial_rows, threads, bytes, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x),
-                                                  static_cast<const T*>(gamma), mean, rstd, static_cast<T*>(dx),
-                                                  dgamma_partial, dbeta_partial, rows, cols);
-      return cudaSuccess;
-    };
-    const bool wide = threads > kLnGroupThreads;
-    if (dtype == kBF16) {
-      auto* type = static_cast<__nv_bfloat16*>(nullptr);
-      TIPSK_CUDA(wide ? launch(LnBwdGroupKernel<__nv_bfloat16, 1024>, type)
-                      : launch(LnBwdGroupKernel<__nv_bfloat16, kLnGroupThreads>, type));
-    } else {
-      auto* type = static_cast<__half*>(nullptr);
-      TIPSK_CUDA(wide ? launch(LnBwdGroupKernel<__half, 1024>, type) : launch(LnBwdGroupKernel<__half, kLnGroupThreads>, type));
     }
     TIPSK_LAUNCH_CHECK();
     return 0;

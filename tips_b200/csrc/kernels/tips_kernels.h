@@ -85,7 +85,6 @@ int tipsk_ln_bwd(const void* dy, const void* x, const void* gamma, const float* 
                  float* dgamma_partial, float* dbeta_partial, int partial_rows, int64_t rows, int cols, int dtype,
                  void* stream);
 int tipsk_ln_bwd_partial_rows(int64_t rows, int cols, int dtype);
-int tipsk_ln_bwd_partials(int64_t rows, int cols);
 int tipsk_ln_reduce_partials(const float* dgamma_partial, const float* dbeta_partial, int partial_rows, int cols,
                              void* dgamma, void* dbeta, int dtype, void* stream);
 
