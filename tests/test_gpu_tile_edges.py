@@ -187,7 +187,9 @@ def test_weight_gradient_of_64_channels_in_tap_groups(n, h, w, cout, stride, pat
     _close(got, ref)
 
 
-@pytest.mark.parametrize("n,c,h,w", [(1, 8, 1, 1), (2, 8, 2, 3), (3, 72, 5, 8), (2, 64, 31, 33), (1, 2056, 4, 4)])
+# rows of one to 128 elements share a block, from 129 on a row has blocks of its own
+@pytest.mark.parametrize("n,c,h,w", [(1, 8, 1, 1), (2, 8, 2, 3), (3, 72, 5, 8), (2, 64, 31, 33), (1, 2056, 4, 4), (700, 8, 3, 3), (5, 1024, 3, 2),
+                                     (5, 1032, 3, 2), (3, 8, 4, 300)])
 def test_maxpool_edges(n, c, h, w):
     from tips_b200.ops.pool import max_pool_3x3_s2
     x = _rand(n, c, h, w).contiguous(memory_format=torch.channels_last).requires_grad_()
