@@ -360,3 +360,34 @@ def test_layer_norm_backward_groups(dtype, rows, cols, groups):
     F.layer_norm(xr, (cols,), wr, br).backward(dy.double())
     for got, ref in ((x.grad, xr.grad), (w.grad, wr.grad), (b.grad, br.grad)):
         _close(got, ref)
+
+
+# pull: an item per lane group up to the line and per lane beyond it; push: 8, 16 and 32 items per warp; one row to 32 rows per
+# warp, row lengths that fill the lanes of a group and that do not
+@pytest.mark.parametrize("batch,fields,dim", [(1, 1, 4), (33, 3, 8), (2520, 26, 16), (2521, 26, 16), (480, 26, 64), (481, 26, 64), (1260, 26, 32),
+                                              (1261, 26, 32), (700, 8, 144), (9, 5, 256), (1300, 26, 24), (2600, 26, 4), (300, 11, 516)])
+@pytest.mark.parametrize("dtype", [BF16, torch.float32])
+def test_pull_and_push_rows(batch, fields, dim, dtype):
+    from tips_b200.ps.gpu import ShardedEmbedding
+    rows = 3000
+    t = ShardedEmbedding(fields, rows, dim, optimizer="sgd", lr=0.5, init_scale=0.1, seed=3, expected_batch=batch, device=torch.device(DEV, 0))
+    g = torch.Generator(device=DEV).manual_seed(batch + dim)
+    ids = torch.randint(0, rows, (batch, fields), device=DEV, generator=g)
+    before = [t.local_shard(f).clone() for f in range(fields)]
+    want = torch.cat([before[f][ids[:, f]] for f in range(fields)], 1)
+    assert torch.equal(t.pull(ids, dtype=dtype), want.to(dtype))
+    grads = _rand(batch, fields * dim, dtype=dtype)
+    t.push(ids, grads, grad_scale=0.25)
+    assert t.check() > 0
+    for f in range(fields):
+        s = torch.zeros(rows, dim, dtype=torch.float64, device=DEV)
+        s.index_add_(0, ids[:, f], grads[:, f * dim:(f + 1) * dim].double())
+        ref = before[f].double() - 0.5 * 0.25 * s
+        # fp32 sums of a few duplicates, the product and the difference: well within 16 units in the last place of the terms
+        assert torch.allclose(t.local_shard(f).double(), ref, rtol=2.0 ** -20, atol=2.0 ** -20)
+    ids[0, 0], ids[batch - 1, fields - 1] = -1, rows  # rows that do not exist read as zeros and are reported
+    got = t.pull(ids, dtype=dtype)
+    assert not bool(got[0, :dim].any()) and not bool(got[batch - 1, -dim:].any())
+    assert torch.equal(got[:, :dim][1:batch - 1], t.local_shard(0)[ids[1:batch - 1, 0]].to(dtype))
+    with pytest.raises(Exception):
+        t.check()

@@ -51,6 +51,8 @@
 // step needs two fences: the one inside the push and the one in front of the
 // next pull (every owner has applied its updates); the push only fences first
 // when no fenced pull has run since the previous push.
+#include <algorithm>
+
 #include "kernels/comm.cuh"
 #include "kernels/common.cuh"
 #include "kernels/ps_placement.h"
@@ -176,15 +178,45 @@ constexpr int kRowsInFlight = 8;  // rows that a lane group loads before it stor
 
 // Pull and scatter are bound by latency: a row is 64 to 256 bytes somewhere in memory, found through a chain of dependent
 // loads and 64-bit divisions.  So every lane of a warp resolves one item of its own (the ids of a warp in one load), and
-// then the warp moves the rows of all of them, kRowsInFlight loads per lane before the first is consumed.  With one item
-// per lane group at a time (8192 x 26 x 64): pull 35 us, scatter 36; like this 14 and 29.  The same form of the apply pass,
-// which has three loads per row, needs 128 registers and was slower (32 against 27 us).  Large batches take 32 items per
-// warp; small ones 8, so that they still spread over the SMs.
-__device__ __forceinline__ int WarpChunk(int64_t total) { return total >= 65536 ? 32 : 8; }
+// then the warp moves the rows of all of them, kFlight loads per lane before the first is consumed.  With one item per lane
+// group at a time (8192 x 26 x 64): pull 32.5 us, scatter 36; like this 12.3 and 29.  The same form of the apply pass, which
+// has three loads per row, needs 128 registers and was slower (32 against 27 us).  The fewer items, the fewer a warp takes,
+// so that they still spread over the SMs (push of 2048 x 26 x 64 with 8, 16 and 32 items per warp 34, 29 and 32 us,
+// 256 x 26 x 64 16, 17 and 19).
+struct WarpItems {
+  int chunk;   // items per warp, a multiple of the rows that its lane groups move at once
+  int flight;  // 1, 4 or 8 loads of a lane group before the first store; a constant of the kernel, or the loads would not overlap
+  WarpItems(int64_t total, int dim) {
+    int lpi = 1;  // as in RowLanes
+    while (lpi < dim / 4 && lpi < 32) lpi <<= 1;
+    const int ipw = 32 / lpi;
+    chunk  = std::max(ipw, total >= 65536 ? 32 : total >= 32768 ? 16 : 8);
+    flight = chunk / ipw >= 8 ? 8 : chunk / ipw >= 2 ? 4 : 1;
+  }
+};
+
+// Whether the pull resolves an item per lane or (kFlight 0) per lane group.  Short rows keep most lanes of a warp busy as it is,
+// and few bytes are over before the longer kernel has begun.  Measured, per lane : per group in us: 512 x 26 x 64 3.4 : 4.0,
+// 1500 x 26 x 32 4.6 : 5.2, 2600 x 26 x 16 4.6 : 4.8, 256 x 26 x 256 4.3 : 4.3, but 256 x 26 x 64 3.1 : 2.8, 256 x 13 x 256
+// 4.2 : 3.0, 1500 x 26 x 16 4.1 : 3.7, 8192 x 26 x 8 7.6 : 7.1.
+bool PullPerLane(int64_t items, int dim) {
+  return dim > 16 ? items >= 6400 && items * dim >= 800000 : dim > 8 && items >= 65536;
+}
 
 template <typename OutT>
+__device__ __forceinline__ void StoreRow4(OutT* to, const U4& q) {
+  if (sizeof(OutT) == 4) {
+    *reinterpret_cast<U4*>(to) = q;
+  } else {
+    OutT o[4] = {FromFloat<OutT>(__uint_as_float(q.x)), FromFloat<OutT>(__uint_as_float(q.y)),
+                 FromFloat<OutT>(__uint_as_float(q.z)), FromFloat<OutT>(__uint_as_float(q.w))};
+    *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(o);
+  }
+}
+
+template <typename OutT, int kFlight>
 __global__ void __launch_bounds__(256)
-PsPullKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t out_ld, int64_t out_col0) {
+PsPullKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t out_ld, int64_t out_col0, int chunk) {
   const PsRank& pr = args.r[blockIdx.y];
   const int n      = pr.nservers;
   const int dim    = meta.dim;
@@ -193,8 +225,28 @@ PsPullKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t out_ld, int64_t 
   const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps      = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const int64_t total       = batch * meta.nfields;
-  const int chunk           = WarpChunk(total);
   OutT* out = static_cast<OutT*>(pr.out);
+  if constexpr (kFlight == 0) {  // an item per lane group
+    for (int64_t base = warp_global * L.ipw; base < total; base += nwarps * L.ipw) {
+      const int64_t item = base + L.sub;
+      if (item >= total) continue;
+      const int64_t b  = item / meta.nfields;
+      const int f      = static_cast<int>(item - b * meta.nfields);
+      const int64_t id = pr.ids[item];
+      OutT* dst        = out + b * out_ld + out_col0 + static_cast<int64_t>(f) * dim;
+      int owner;
+      int64_t lrow;
+      PsPlace(f, id < 0 ? 0 : id, n, &owner, &lrow);
+      const bool bad = id < 0 || lrow >= meta.rows_per_shard[f];
+      if (bad && L.sublane == 0) atomicExch(pr.error, 2);
+      const char* row = pr.slab[owner] + meta.field_off[f] + static_cast<uint64_t>(lrow) * dim * 4;
+      for (int v = L.sublane; v < vecs; v += L.lpi)
+        StoreRow4(dst + v * 4, bad                        ? U4{0, 0, 0, 0}
+                               : owner == pr.my_server ? *reinterpret_cast<const U4*>(row + v * 16)
+                                                       : LdSysFree(row + v * 16));
+    }
+    return;
+  }
   for (int64_t base = warp_global * chunk; base < total; base += nwarps * chunk) {
     const int64_t item = base + L.lane;
     const char* src = nullptr;  // null: a bad id, whose row reads as zeros
@@ -215,12 +267,12 @@ PsPullKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t out_ld, int64_t 
         own = owner == pr.my_server;
       }
     }
-    for (int j = 0; j < chunk; j += L.ipw * kRowsInFlight) {
+    for (int j = 0; j < chunk; j += L.ipw * kFlight) {
       for (int v0 = 0; v0 < vecs; v0 += L.lpi) {
         const int v = v0 + L.sublane;
-        U4 q[kRowsInFlight];
+        U4 q[kFlight > 0 ? kFlight : 1];
 #pragma unroll
-        for (int u = 0; u < kRowsInFlight; ++u) {
+        for (int u = 0; u < kFlight; ++u) {
           const int from   = j + u * L.ipw + L.sub;
           const char* row  = reinterpret_cast<const char*>(
               __shfl_sync(kFullMask, reinterpret_cast<unsigned long long>(src), from & 31));
@@ -230,18 +282,11 @@ PsPullKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t out_ld, int64_t 
             q[u] = local ? *reinterpret_cast<const U4*>(row + v * 16) : LdSysFree(row + v * 16);
         }
 #pragma unroll
-        for (int u = 0; u < kRowsInFlight; ++u) {
+        for (int u = 0; u < kFlight; ++u) {
           const int from   = j + u * L.ipw + L.sub;
           const int64_t at = __shfl_sync(kFullMask, dst, from & 31);
           if (from >= chunk || v >= vecs || at < 0) continue;
-          OutT* to = out + at + v * 4;
-          if (sizeof(OutT) == 4) {
-            *reinterpret_cast<U4*>(to) = q[u];
-          } else {
-            OutT o[4] = {FromFloat<OutT>(__uint_as_float(q[u].x)), FromFloat<OutT>(__uint_as_float(q[u].y)),
-                         FromFloat<OutT>(__uint_as_float(q[u].z)), FromFloat<OutT>(__uint_as_float(q[u].w))};
-            *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(o);
-          }
+          StoreRow4(out + at + v * 4, q[u]);
         }
       }
     }
@@ -465,10 +510,10 @@ PsClearIndexKernel(PsLaunch args, uint64_t slots);
 // Local segment-reduce of the batch.  kIndexed: the slot of every item comes from the index of the pull.
 // Otherwise phase 1 resolves one item per lane (32 probes in flight per warp) and extends the list of distinct
 // rows; phase 2 adds the gradient rows with `lpi` lanes per row.
-template <typename GradT, bool kVec, bool kIndexed>
+template <typename GradT, bool kVec, bool kIndexed, int kFlight>
 __global__ void __launch_bounds__(256)
 PsScatterKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t grad_ld, int64_t grad_col0, uint64_t slots,
-                float grad_scale) {
+                float grad_scale, int chunk) {
   const PsRank& pr = args.r[blockIdx.y];
   const int n      = pr.nservers;  // placement is among the servers
   const int dim    = meta.dim;
@@ -480,7 +525,6 @@ PsScatterKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t grad_ld, int6
   const GradT* grads        = static_cast<const GradT*>(pr.grads);
   unsigned long long* keys  = reinterpret_cast<unsigned long long*>(pr.acc);
   float* sums_base          = reinterpret_cast<float*>(pr.acc + slots * 8);
-  const int chunk           = WarpChunk(total);
   for (int64_t base = warp_global * chunk; base < total; base += nwarps * chunk) {
     const int64_t mine = base + L.lane;
     const bool have    = L.lane < chunk && mine < total;
@@ -503,13 +547,13 @@ PsScatterKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t grad_ld, int6
       }
       AppendSlots(pr.ulist, &pr.ctl->ucount, claimed, slot, L.lane);
     }
-    for (int j = 0; j < chunk; j += L.ipw * kRowsInFlight) {
+    for (int j = 0; j < chunk; j += L.ipw * kFlight) {
       for (int v0 = 0; v0 < vecs; v0 += L.lpi) {
         const int v = v0 + L.sublane;
-        float gv[kRowsInFlight][4];
-        uint32_t to[kRowsInFlight];
+        float gv[kFlight][4];
+        uint32_t to[kFlight];
 #pragma unroll
-        for (int u = 0; u < kRowsInFlight; ++u) {
+        for (int u = 0; u < kFlight; ++u) {
           const int from    = j + u * L.ipw + L.sub;
           const int64_t row = __shfl_sync(kFullMask, at, from & 31);
           to[u]             = __shfl_sync(kFullMask, slot, from & 31);
@@ -517,7 +561,7 @@ PsScatterKernel(PsLaunch args, PsMeta meta, int64_t batch, int64_t grad_ld, int6
           if (to[u] != kNoSlot) LoadGrad4<GradT, kVec>(grads + row + v * 4, gv[u]);
         }
 #pragma unroll
-        for (int u = 0; u < kRowsInFlight; ++u)
+        for (int u = 0; u < kFlight; ++u)
           if (to[u] != kNoSlot)
             RedAdd4(sums_base + static_cast<uint64_t>(to[u]) * dim + v * 4, gv[u][0] * grad_scale, gv[u][1] * grad_scale,
                     gv[u][2] * grad_scale, gv[u][3] * grad_scale);
@@ -1178,23 +1222,40 @@ int DropIndex(PsLaunch& l, int local, cudaStream_t s) {
   return 0;
 }
 
+template <typename OutT>
+int LaunchPull(const PsLaunch& l, dim3 grid, cudaStream_t s, int64_t batch, int64_t out_ld, int64_t out_col0) {
+  PsState& st = g_ps;
+  const int64_t items = batch * st.meta.nfields;
+  const WarpItems w(items, st.meta.dim);
+  auto* kernel = !PullPerLane(items, st.meta.dim) ? PsPullKernel<OutT, 0>
+                 : w.flight == 8                  ? PsPullKernel<OutT, 8>
+                                                  : PsPullKernel<OutT, 4>;
+  kernel<<<grid, 256, 0, s>>>(l, st.meta, batch, out_ld, out_col0, w.chunk);
+  TIPSK_LAUNCH_CHECK();
+  return 0;
+}
+
+template <typename GradT, bool kVec, bool kIndexed>
+int LaunchScatterOf(const PsLaunch& l, dim3 grid, cudaStream_t s, int64_t batch, int64_t grad_ld, int64_t grad_col0,
+                    float grad_scale) {
+  PsState& st = g_ps;
+  const WarpItems w(batch * st.meta.nfields, st.meta.dim);
+  auto* kernel = w.flight == 8   ? PsScatterKernel<GradT, kVec, kIndexed, 8>
+                 : w.flight == 4 ? PsScatterKernel<GradT, kVec, kIndexed, 4>
+                                 : PsScatterKernel<GradT, kVec, kIndexed, 1>;
+  kernel<<<grid, 256, 0, s>>>(l, st.meta, batch, grad_ld, grad_col0, st.slots, grad_scale, w.chunk);
+  TIPSK_LAUNCH_CHECK();
+  return 0;
+}
+
 template <typename GradT>
 int LaunchScatter(const PsLaunch& l, dim3 grid, cudaStream_t s, bool vec, bool indexed, int64_t batch,
                          int64_t grad_ld, int64_t grad_col0, float grad_scale) {
-  PsState& st = g_ps;
-  if (indexed) {
-    if (vec)
-      PsScatterKernel<GradT, true, true><<<grid, 256, 0, s>>>(l, st.meta, batch, grad_ld, grad_col0, st.slots, grad_scale);
-    else
-      PsScatterKernel<GradT, false, true><<<grid, 256, 0, s>>>(l, st.meta, batch, grad_ld, grad_col0, st.slots, grad_scale);
-  } else {
-    if (vec)
-      PsScatterKernel<GradT, true, false><<<grid, 256, 0, s>>>(l, st.meta, batch, grad_ld, grad_col0, st.slots, grad_scale);
-    else
-      PsScatterKernel<GradT, false, false><<<grid, 256, 0, s>>>(l, st.meta, batch, grad_ld, grad_col0, st.slots, grad_scale);
-  }
-  TIPSK_LAUNCH_CHECK();
-  return 0;
+  if (indexed)
+    return vec ? LaunchScatterOf<GradT, true, true>(l, grid, s, batch, grad_ld, grad_col0, grad_scale)
+               : LaunchScatterOf<GradT, false, true>(l, grid, s, batch, grad_ld, grad_col0, grad_scale);
+  return vec ? LaunchScatterOf<GradT, true, false>(l, grid, s, batch, grad_ld, grad_col0, grad_scale)
+             : LaunchScatterOf<GradT, false, false>(l, grid, s, batch, grad_ld, grad_col0, grad_scale);
 }
 
 }  // namespace
@@ -1441,12 +1502,8 @@ int tipsk_ps_pull(const int64_t* const* ids, void* const* outs, int64_t batch, i
     st.lead_fence = false;
   }
   if (!index) {
-    if (out_dtype == kF32)
-      PsPullKernel<float><<<grid, 256, 0, s>>>(l, st.meta, batch, out_ld, out_col0);
-    else
-      PsPullKernel<__nv_bfloat16><<<grid, 256, 0, s>>>(l, st.meta, batch, out_ld, out_col0);
-    TIPSK_LAUNCH_CHECK();
-    return 0;
+    return out_dtype == kF32 ? LaunchPull<float>(l, grid, s, batch, out_ld, out_col0)
+                             : LaunchPull<__nv_bfloat16>(l, grid, s, batch, out_ld, out_col0);
   }
   MarkPull(s);
   dim3 lgrid(ListGrid(items), local);
