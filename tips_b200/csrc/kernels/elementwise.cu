@@ -147,6 +147,7 @@ struct ListArgs {
 template <typename S, typename D, int kMode>
 __global__ void __launch_bounds__(kThreads) PackKernel(const __grid_constant__ ListArgs args, void* flat_v, float scale) {
   int lo = 0, hi = args.count - 1;  // last tensor whose first block is not behind this one
+  if (args.count == static_cast<int>(gridDim.x)) lo = hi = blockIdx.x;  // one block each: the search costs 0.4 us of 2.4
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (args.first[mid] <= static_cast<int>(blockIdx.x)) lo = mid;
