@@ -326,7 +326,7 @@ def test_softmax_cross_entropy_without_counted_rows():
 
 
 @pytest.mark.parametrize("dtype", [BF16, torch.float16, torch.float32])
-@pytest.mark.parametrize("rows,cols", [(1, 8), (31, 264), (33, 1000), (4097, 72)])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (31, 264), (33, 1000), (4097, 72), (1217, 4096)])  # the last: more than four blocks per SM in fp32
 @pytest.mark.parametrize("act", [None, "relu", "gelu"])
 def test_bias_act_backward_rows(dtype, rows, cols, act):
     from tips_b200.ops.pointwise import bias_act

@@ -59,10 +59,10 @@ BiasActFwdKernel(const T* __restrict__ x, const T* __restrict__ bias, T* __restr
 }
 
 // block (32, 8): tx -> vector column, ty -> row lane; grid (col tiles, row partitions).  Bound by HBM, and with GELU by the
-// instructions of its derivative, hence two values per instruction there; three or four rows in flight per thread.
+// instructions of its derivative, hence two values per instruction there; U rows in flight per thread.
 // 16384 x 4096 bf16: GELU (400 MB) 135 -> 85 us; bias gradient alone, 1232 x 30528 (75 MB) 39 -> 19 us.
-template <typename T, int kAct>
-__global__ void __launch_bounds__(256, kAct == 0 ? 3 : 2)
+template <typename T, int kAct, int U>
+__global__ void __launch_bounds__(256, kAct == 0 ? 3 : kAct == 2 && sizeof(T) == 4 ? 4 : 2)
 BiasActBwdKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ bias, T* __restrict__ dx,
                  float* __restrict__ dbias, int64_t rows, int cols) {
   constexpr int N = 16 / sizeof(T);
@@ -83,7 +83,6 @@ BiasActBwdKernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __r
       for (int k = 0; k < N; ++k) bv[k] = 0.f;
     }
     const int64_t step = static_cast<int64_t>(gridDim.y) * 8;
-    constexpr int U = kAct == 2 ? 3 : 4;  // rows in flight per thread
     for (int64_t r = static_cast<int64_t>(blockIdx.y) * 8 + threadIdx.y; r < rows; r += U * step) {
       Vec16<T> d[U], q[U];
 #pragma unroll
@@ -609,7 +608,14 @@ int tipsk_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx
   if (parts < 1) parts = 1;
   dim3 grid(col_tiles, parts), block(32, 8);
   EPI_DISPATCH(dtype, {
-    auto* kernel = act == 0 ? BiasActBwdKernel<T, 0> : act == 1 ? BiasActBwdKernel<T, 1> : BiasActBwdKernel<T, 2>;
+    // GELU of fp32 values is bound by its instructions and wants all blocks resident at once: four per SM with two rows in
+    // flight, six with one (65536 x 256 45 and 50 us, 4096 x 4096, whose grid is larger than four per SM, 48 and 39; three
+    // rows in flight, of which three blocks fit, 52 and 43).
+    constexpr int kGeluRows = sizeof(T) == 4 ? 2 : 3;
+    auto* kernel = act == 0   ? BiasActBwdKernel<T, 0, 4>
+                   : act == 1 ? BiasActBwdKernel<T, 1, 4>
+                   : sizeof(T) == 4 && col_tiles * parts > 4 * NumSMs() ? BiasActBwdKernel<T, 2, sizeof(T) == 4 ? 1 : 3>
+                                                                        : BiasActBwdKernel<T, 2, kGeluRows>;
     kernel<<<grid, block, 0, s>>>(static_cast<const T*>(dy), static_cast<const T*>(x), static_cast<const T*>(bias),
                                   static_cast<T*>(dx), dbias, rows, cols);
   });
