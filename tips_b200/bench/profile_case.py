@@ -1,7 +1,8 @@
 """Small single-kernel cases for profiler captures: each runs ONE kernel a handful of times on inputs a
 little larger than L2, holds well under a GB on the device and exits by itself in seconds.
 
-    python -m tips_b200.bench.profile_case {bn_fwd,bn_bwd,gemm,gemm_persistent,ln,sgd,ps_pull,ps_push,conv1x1,conv3x3,conv_dgrad,conv_wgrad,adam,ln_bwd,bias_act_bwd,softmax_xent}
+    python -m tips_b200.bench.profile_case {bn_fwd,bn_bwd,gemm,gemm_gelu,gemm_wgrad,ln,sgd,ps_pull,ps_push,conv1x1,conv3x3,conv_dgrad,conv_wgrad,
+                                           adam,ln_bwd,ln_bwd_groups,bias_act_bwd,softmax_xent,maxpool}
 """
 from __future__ import annotations
 
@@ -28,14 +29,20 @@ def main(argv=None):
             dy = torch.randn_like(y)
             for _ in range(reps):
                 torch.autograd.grad(y, xg, dy, retain_graph=True)
-    elif case in ("gemm", "gemm_persistent"):
+    elif case == "gemm_wgrad":
+        from tips_b200.ops.linear import _weight_grad
+        dz = torch.randn(16384, 4096, device=dev).to(torch.bfloat16)
+        x = torch.randn(16384, 1024, device=dev).to(torch.bfloat16)
+        for _ in range(reps):
+            _weight_grad(dz, x, torch.bfloat16)
+    elif case in ("gemm", "gemm_gelu"):
         from tips_b200.ops.linear import gemm_tn
-        k = 4096 if case == "gemm" else 1024  # the short-K shape takes the persistent double-buffered variant
+        k = 4096 if case == "gemm" else 1024  # the encoder's feed-forward layer keeps its pre-activation
         a = torch.randn(16384, k, device=dev).to(torch.bfloat16)
         b = torch.randn(4096, k, device=dev).to(torch.bfloat16)
         bias = torch.randn(4096, device=dev).to(torch.bfloat16)
         for _ in range(reps):
-            gemm_tn(a, b, bias, "relu")
+            gemm_tn(a, b, bias, "relu") if case == "gemm" else gemm_tn(a, b, bias, "gelu", want_pre=True)
     elif case in ("conv1x1", "conv3x3", "conv_dgrad", "conv_wgrad"):
         from tips_b200.ops import conv as C
         k, cin, cout = (1, 64, 256) if case == "conv1x1" else (3, 64, 64)
@@ -71,9 +78,17 @@ def main(argv=None):
         for _ in range(reps + 1):
             p.grad = torch.randn_like(p)
             opt.step()
-    elif case == "ln_bwd":
+    elif case == "maxpool":
+        from tips_b200.ops.pool import max_pool_3x3_s2
+        x = torch.randn(128, 64, 112, 112, device=dev).to(torch.bfloat16)
+        x = x.contiguous(memory_format=torch.channels_last).requires_grad_()
+        y = max_pool_3x3_s2(x)
+        dy = torch.randn_like(y)
+        for _ in range(reps):
+            torch.autograd.grad(max_pool_3x3_s2(x), x, dy)
+    elif case in ("ln_bwd", "ln_bwd_groups"):
         from tips_b200.ops.norm import LayerNorm
-        x = torch.randn(131072, 1024, device=dev).to(torch.bfloat16).requires_grad_()
+        x = torch.randn(131072 if case == "ln_bwd" else 16383, 1024, device=dev).to(torch.bfloat16).requires_grad_()
         ln = LayerNorm(1024).to(dev)
         y = ln(x)
         dy = torch.randn_like(y)

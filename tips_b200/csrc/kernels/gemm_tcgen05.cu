@@ -306,7 +306,7 @@ GemmTnKernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 // tiles than SMs and the output qualifies for the TMA store path.
 template <int BN>
 struct PersistCfg {
-  static constexpr int kStages     = BN >= 256 ? 3 : 5;
+  static constexpr int kStages     = 5;
   static constexpr int kABytes     = kBM * kBK * 2;
   static constexpr int kBBytes     = BN * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
