@@ -99,7 +99,7 @@ def test_split_contraction(m, n, k):
 # lines of the rule and with several channel blocks and output tiles.
 CONV3X3 = [(43, 56, 56, 64, 64, 1), (50, 55, 56, 64, 64, 1), (74, 8, 62, 64, 64, 1), (149, 31, 33, 64, 64, 1), (150, 9, 28, 64, 64, 1),
            (75, 28, 28, 64, 64, 1), (300, 2, 62, 64, 64, 1), (300, 12, 3, 64, 64, 0), (150, 9, 9, 64, 64, 0), (149, 5, 63, 64, 64, 0),
-           (36, 8, 62, 64, 64, 0), (149, 28, 28, 128, 128, 0), (75, 17, 28, 64, 192, 0), (43, 56, 56, 192, 64, 0),
+           (150, 100, 5, 64, 64, 1), (200, 84, 1, 64, 64, 0), (36, 8, 62, 64, 64, 0), (149, 28, 28, 128, 128, 0), (75, 17, 28, 64, 192, 0), (43, 56, 56, 192, 64, 0),
            (297, 9, 9, 64, 128, 0), (601, 5, 24, 192, 64, 0)]
 
 

@@ -114,7 +114,9 @@ __device__ __forceinline__ F2 RcpFast(F2 a) {
 
 // erfc(z) / exp(-z^2) for z = |v| / sqrt(2) by the rational approximation a1 t + ... + a5 t^5, t = 1 / (1 + p z)
 // (Abramowitz and Stegun, 7.1.26: absolute error of erf < 1.5e-7), and exp(-z^2), of two values at once.  For results
-// that are rounded to 16 bits next: one exponential and one reciprocal where erff takes two divergent branches.
+// that are rounded to 16 bits next: one exponential and one reciprocal where erff takes two divergent branches.  Error of the
+// bf16 GELU against 64 bits (relative 2-norm, with 0.5 v (1 + erff) : like this): normally distributed v 1.6645e-3 : 1.6645e-3,
+// v in -3..0 1.7087e-3 : 1.7087e-3, -4..-3 1.5916e-3 : 1.5944e-3, and beyond, where 1 + erff cancels, -6..-4 2.22e-3 : 1.69e-3.
 __device__ __forceinline__ void ErfcParts2(F2 v, F2* poly, F2* gauss) {
   const float2 s = SplitF2(v);
   const F2 z = Mul2(MakeF2(fabsf(s.x), fabsf(s.y)), Both(0.70710678118654752f));

@@ -727,8 +727,9 @@ int tipsk_softmax_xent_mean(const void* logits, const int64_t* labels, float* lo
                             int64_t rows, int cols, int64_t ignore_index, int dtype, void* stream) {
   if (rows <= 0 || cols <= 0) return 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // The row kernel needs whole, aligned 16-byte vectors and at most eight of them per thread (it is the faster one
-  // wherever it applies: see the kernel).
+  // The row kernel needs whole, aligned 16-byte vectors and at most eight of them per thread: more of them than two blocks of
+  // 512 threads, or four of 256, can keep in registers would have to be read again in each sweep, which is the general form
+  // (it is the faster one wherever it applies: see the kernel).
   const int n        = 16 / static_cast<int>(DTypeSize(dtype));
   const bool aligned = cols % n == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0 &&
                        reinterpret_cast<uintptr_t>(dlogits) % 16 == 0;

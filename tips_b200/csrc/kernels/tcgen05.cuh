@@ -56,8 +56,8 @@ __device__ __forceinline__ bool MbarWaitWarp(uint64_t* bar, uint32_t parity) {
 // True in one lane of a converged warp, always the same one.  The instructions that a single thread issues (tcgen05.mma,
 // commits, TMA) take their operands from uniform registers: behind this predicate, in a loop that the whole warp walks,
 // the compiler knows that one lane is active and keeps descriptors and counters uniform.  Behind `lane == 0` the issue of
-// narrow MMAs was the bound: with nothing else changed, the 64-column kernels went from 139 to 111 us (3x3, 64 -> 64, 256
-// images of 56 x 56), 134 to 124 us (7x7 stem, 64 images of 224 x 224) and 140 to 117 us (its weight gradient).
+// narrow MMAs was the bound: with nothing else changed, the 64-column kernels went from 134 to 124 us (7x7 stem, 64 images
+// of 224 x 224) and from 140 to 117 us (its weight gradient, one tap per tile).
 __device__ __forceinline__ bool ElectOne() {
   uint32_t leader;
   asm volatile(
@@ -160,7 +160,7 @@ __device__ __forceinline__ void ClusterSync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Tile load into this CTA's shared memory whose bytes are counted on the leader's copy of the barrier: clearing bit 24
-// of a shared::cluster address selects the even CTA of the pair.
+// of a shared::cluster address selects the even CTA of the pair (as CUTLASS's cute/arch/copy_sm100_tma.hpp documents).
 __device__ __forceinline__ void TmaLoad2DPair(void* smem_dst, const CUtensorMap* tmap, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
