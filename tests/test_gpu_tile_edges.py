@@ -160,6 +160,17 @@ def test_weight_gradient_of_non_finite_pixels(n, h, w, value):
     assert base.K().tipsk_conv_status() == 0
 
 
+def test_weight_gradient_of_nothing_but_nan():
+    from tips_b200.ops.conv import conv2d_wgrad
+    from tips_b200.ops import base
+    x = _rand(43, 64, 56, 56).contiguous(memory_format=torch.channels_last)
+    dy = _rand(43, 64, 56, 56, seed=1).contiguous(memory_format=torch.channels_last)
+    x[:, 5:40] = float("nan")
+    got = conv2d_wgrad(x, dy, (64, 3, 3, 64), 1, 1).isnan()
+    assert bool(got[..., 5:40].all()) and not bool(got[..., :5].any()) and not bool(got[..., 40:].any())
+    assert base.K().tipsk_conv_status() == 0
+
+
 # the smallest pixel counts that take several taps per tile (24 steps of 64 per CTA) and one below, with one and two tiles of
 # output channels, ragged boxes and stride 2; few pixels: one tap per tile
 @pytest.mark.parametrize("n,h,w,cout,stride,path", [(2, 6, 7, 64, 1, 0), (3, 20, 20, 256, 1, 0), (9, 15, 13, 320, 2, 0), (379, 20, 20, 64, 1, 1),
